@@ -43,43 +43,42 @@ __device__ __forceinline__ CacheSmem cache_smem(unsigned char* raw, uint32_t nwa
 
 // One world per CTA: block b steps worlds[b].
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads, 512 / kThreads) k_step_block(WorldDev* worlds, ColliderSet cs) {
+__global__ void __launch_bounds__(kThreads, 512 / kThreads) k_step_block(const WorldDev* worlds, const __grid_constant__ ColliderSet cs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpManifold* wsm = reinterpret_cast<WarpManifold*>(smem_raw);
-    WorldDev w = worlds[blockIdx.x];
+    const WorldDev w = worlds[blockIdx.x];
     const CacheSmem csm = cache_smem(smem_raw, blockDim.x / 32u, w.cache_cap);
     BlockGroup g;
     world_step(g, w, cs, wsm, csm, reinterpret_cast<float*>(smem_raw));
 }
-template __global__ void k_step_block<256>(WorldDev*, ColliderSet);
-template __global__ void k_step_block<512>(WorldDev*, ColliderSet);
+template __global__ void k_step_block<256>(const WorldDev*, const __grid_constant__ ColliderSet);
+template __global__ void k_step_block<512>(const WorldDev*, const __grid_constant__ ColliderSet);
 
 // One world over a cooperative grid, in two kernels: the narrow part of the
 // step, then its solve part (barrier words bar[0] and bar[1]).
-__global__ void __launch_bounds__(512, 1) k_step_grid(const WorldDev* world, ColliderSet cs, GridBar* bar,
+__global__ void __launch_bounds__(512, 1) k_step_grid(const __grid_constant__ WorldDev w,
+                                                      const __grid_constant__ ColliderSet cs, GridBar* bar,
                                                       unsigned long long timeout_ns) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpManifold* wsm = reinterpret_cast<WarpManifold*>(smem_raw);
-    WorldDev w = *world;
     const CacheSmem csm = cache_smem(smem_raw, blockDim.x / 32u, w.cache_cap);
     GridGroup g{bar, &w.ctr[C_ERROR], timeout_ns, gridDim.x};
     world_step_narrow(g, w, cs, wsm, csm);
 }
-__global__ void __launch_bounds__(256, 1) k_solve_grid(const WorldDev* world, GridBar* bar,
+__global__ void __launch_bounds__(256, 1) k_solve_grid(const __grid_constant__ WorldDev w, GridBar* bar,
                                                        unsigned long long timeout_ns, uint32_t part) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    WorldDev w = *world;
     GridGroup g{bar, &w.ctr[C_ERROR], timeout_ns, gridDim.x};
     world_step_solve(g, w, reinterpret_cast<float*>(smem_raw), true, part);
 }
 // The solve part on one thread-block cluster (the whole grid): all of it
 // (whole) or the sweeps and the store after k_solve_grid(...,
 // SOLVE_CONSTRAINTS).
-__global__ void __launch_bounds__(256, 1) k_solve_cluster(const WorldDev* world, uint32_t smem_bytes, uint32_t whole) {
+__global__ void __launch_bounds__(256, 1) k_solve_cluster(const __grid_constant__ WorldDev w, uint32_t smem_bytes,
+                                                          uint32_t whole) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint32_t ncta;
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
-    WorldDev w = *world;
     if (ncta != gridDim.x) {  // launch constants: the same verdict in every block
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&w.ctr[C_ERROR], ERR_BOUNDS);
         return;
@@ -1517,22 +1516,21 @@ int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, floa
         w.cfg.record_substeps = 1u;
         w.subrec = ctx->subrec.p;
     }
-    CK(cudaMemcpyAsync(ctx->d_world.p, &w, sizeof(w), cudaMemcpyHostToDevice, ctx->stream));
+    if (!grid) CK(cudaMemcpyAsync(ctx->d_world.p, &w, sizeof(w), cudaMemcpyHostToDevice, ctx->stream));
     const ColliderSet cs = ctx->cols.set();
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     if (grid) {
         CK(cudaMemsetAsync(ctx->bar.p, 0, 3 * sizeof(GridBar), ctx->stream));
-        const WorldDev* wp = ctx->d_world.p;
         GridBar* bp = ctx->bar.p;
         const unsigned long long timeout = ctx->wait_limit_ns ? ctx->wait_limit_ns : kGridWaitNs;
-        void* args[] = {(void*)&wp, (void*)&cs, (void*)&bp, (void*)&timeout};
+        void* args[] = {(void*)&w, (void*)&cs, (void*)&bp, (void*)&timeout};
         CK(cudaLaunchCooperativeKernel((const void*)k_step_grid, dim3(ctx->grid_blocks), dim3(kGridThreads), args,
                                        smem, ctx->stream));
         CK(cudaEventRecord(ctx->ev_mid, ctx->stream));
         const uint32_t whole = cluster && ctx->cluster_whole ? 1u : 0u;
         if (!whole) {
             uint32_t part = cluster ? SOLVE_CONSTRAINTS : SOLVE_ALL;
-            void* sargs[] = {(void*)&wp, (void*)&bp, (void*)&timeout, (void*)&part};
+            void* sargs[] = {(void*)&w, (void*)&bp, (void*)&timeout, (void*)&part};
             CK(cudaLaunchCooperativeKernel((const void*)k_solve_grid, dim3(ctx->grid_blocks), dim3(kSolveThreads),
                                            sargs, solve_smem(), ctx->stream));
         }
@@ -1541,7 +1539,7 @@ int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, floa
             cudaLaunchConfig_t lc = {};
             cudaLaunchAttribute at[1];
             cluster_config(&lc, at, ctx->cluster_size, ctx->cluster_smem, ctx->stream);
-            CK(cudaLaunchKernelEx(&lc, k_solve_cluster, wp, std::min(ctx->cluster_smem, ctx->cluster_state_cap),
+            CK(cudaLaunchKernelEx(&lc, k_solve_cluster, w, std::min(ctx->cluster_smem, ctx->cluster_state_cap),
                                   whole));
         }
     } else {

@@ -40,6 +40,7 @@ struct BlockGroup {
     // batch (the event-ordered sweeps are not compiled for this group).
     static constexpr bool kEventSweeps = false;
     static constexpr bool kDistributed = false;  // shared memory is the CTA's own
+    uint32_t n_pairs = 0;  // pairs of this step
     __device__ uint32_t rank() const { return threadIdx.x; }
     __device__ uint32_t size() const { return blockDim.x; }
     __device__ uint32_t block() const { return 0; }
@@ -66,6 +67,7 @@ struct GridGroup {
     unsigned long long timeout_ns;
     uint32_t nb;        // participating blocks: base .. base + nb - 1
     uint32_t base = 0;
+    uint32_t n_pairs = 0;  // pairs of this step
     __device__ uint32_t rank() const { return (blockIdx.x - base) * blockDim.x + threadIdx.x; }
     __device__ uint32_t size() const { return nb * blockDim.x; }
     __device__ uint32_t block() const { return blockIdx.x - base; }
@@ -75,9 +77,9 @@ struct GridGroup {
     // colour batches are small, and a barrier over a few blocks costs far less
     // than one over the whole grid.  The other blocks leave the kernel, or
     // run as tail(k).
-    __device__ GridGroup subgroup(uint32_t k) const { return GridGroup{bar + 1, err, timeout_ns, k, base}; }
+    __device__ GridGroup subgroup(uint32_t k) const { return GridGroup{bar + 1, err, timeout_ns, k, base, n_pairs}; }
     // The blocks after the first k, with the third barrier word (bar + 2).
-    __device__ GridGroup tail(uint32_t k) const { return GridGroup{bar + 2, err, timeout_ns, nb - k, base + k}; }
+    __device__ GridGroup tail(uint32_t k) const { return GridGroup{bar + 2, err, timeout_ns, nb - k, base + k, n_pairs}; }
     // Bounded grid barrier: a waiting block gives up after timeout_ns, sets
     // ERR_TIMEOUT and every later sync() of every block returns false.  The
     // block's threads meet at __syncthreads, then thread 0 arrives with an
@@ -133,6 +135,7 @@ struct GridGroup {
 struct ClusterGroup {
     static constexpr bool kEventSweeps = false;
     static constexpr bool kDistributed = true;  // other CTAs' shared memory through mapa
+    uint32_t n_pairs = 0;                       // pairs of this step
     __device__ uint32_t rank() const { return blockIdx.x * blockDim.x + threadIdx.x; }
     __device__ uint32_t size() const { return gridDim.x * blockDim.x; }
     __device__ uint32_t block() const { return blockIdx.x; }
@@ -507,7 +510,7 @@ __device__ __forceinline__ uint32_t find_body(const uint2* ids, uint32_t n, uint
 // Phase: begin (sleep skip test, per-body step-start state)
 // ---------------------------------------------------------------------------
 template <class G>
-__device__ bool phase_begin(G& g, WorldDev& w, bool skip_test, bool* skipped) {
+__device__ bool phase_begin(G& g, const WorldDev& w, bool skip_test, bool* skipped) {
     // counters (not the sticky error word) are zeroed by the host/graph memset.
     for (uint32_t i = g.rank(); i < w.n_bodies; i += g.size()) {
         const DBodyProp& pr = w.prop[i];
@@ -559,7 +562,7 @@ __device__ bool phase_begin(G& g, WorldDev& w, bool skip_test, bool* skipped) {
 // the list does not fit pair_cap (nothing is written; the host grows the
 // buffers).
 template <class G>
-__device__ bool phase_broadphase(G& g, WorldDev& w, const ColliderSet& cs, bool* overflow, unsigned char* smem) {
+__device__ bool phase_broadphase(G& g, const WorldDev& w, const ColliderSet& cs, bool* overflow, unsigned char* smem) {
     const uint32_t N = w.n_bodies;
     const float m = w.cfg.margin;
     // inflated world AABBs in id order (position s holds body ids[s]), w = 1
@@ -674,7 +677,7 @@ __device__ bool phase_broadphase(G& g, WorldDev& w, const ColliderSet& cs, bool*
                 return false;
             if (g.rank() == 0 && w.ts) w.ts[TS_BP_SCAN] = global_ns();
             *overflow = total > w.pair_cap;
-            w.n_pairs = total;
+            g.n_pairs = total;
             if (g.rank() == 0) *w.n_pairs_dev = total;
             if (*overflow) return true;
         }
@@ -744,8 +747,8 @@ __device__ bool phase_broadphase(G& g, WorldDev& w, const ColliderSet& cs, bool*
 // Phase: pairs (system.narrowPhase filter + processPair head)
 // ---------------------------------------------------------------------------
 template <class G>
-__device__ bool phase_pairs(G& g, WorldDev& w, const ColliderSet& cs, uint32_t cur) {
-    const uint32_t P = w.n_pairs;
+__device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint32_t cur) {
+    const uint32_t P = g.n_pairs;
     if (g.rank() == 0) {
         w.ctr[C_PAIRS_IN] = P;
         w.cframe[0] += 1ull;  // BrickPairCache.beginFrame
@@ -909,7 +912,7 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {
     return r;
 }
 
-__device__ void cache_replay(WorldDev& w, const CacheSmem& t) {
+__device__ void cache_replay(const WorldDev& w, const CacheSmem& t) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t cap = w.cache_cap;
     const uint32_t maxp = cap < 16u ? cap : 16u;
@@ -1084,7 +1087,7 @@ __host__ __device__ constexpr size_t cta_replay_scratch_bytes() {
            32u * sizeof(unsigned long long) + 32u * sizeof(uint32_t) + 4u * sizeof(uint32_t);
 }
 
-__device__ void cache_replay_cta(WorldDev& w, const CacheSmem& t, unsigned char* scratch) {
+__device__ void cache_replay_cta(const WorldDev& w, const CacheSmem& t, unsigned char* scratch) {
     const uint32_t tid = threadIdx.x, T = blockDim.x, lane = tid & 31u, wid = tid >> 5;
     const uint32_t cap = w.cache_cap;
     const uint32_t frame = (uint32_t)w.cframe[0];
@@ -1353,7 +1356,7 @@ __device__ __forceinline__ int32_t clip_hi(int32_t bound_excl, int32_t centre) {
     const long long d = (long long)bound_excl - 1ll - (long long)centre;
     return d < 1 ? (d < -2 ? -2 : (int32_t)d) : 1;
 }
-__device__ __forceinline__ void probe_neighbourhood(WorldDev& w, const ColliderSet& cs, const ProbeCtx& c, uint32_t p,
+__device__ __forceinline__ void probe_neighbourhood(const WorldDev& w, const ColliderSet& cs, const ProbeCtx& c, uint32_t p,
                                                     uint32_t ta, int32_t x, int32_t y, int32_t z, F3 wa, I3 cbv,
                                                     uint32_t* mask, Top4* t, uint32_t* checked) {
     const DCollider& cb = *c.cb;
@@ -1530,7 +1533,7 @@ __device__ void build_contact(const ColliderSet& cs, const ProbeCtx& c, const in
 // always the top four of the prefix).  A warp scan of top-4 multisets gives
 // every lane that prefix, seeded with the manifold's state; only the entering
 // candidates are replayed, in order, through addContact.
-__device__ void probe_pair(WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p, WarpManifold& sm) {
+__device__ void probe_pair(const WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p, WarpManifold& sm) {
     const uint32_t lane = threadIdx.x & 31;
     PairInfo& pi = w.pinfo[p];
     const uint32_t ia = pi.ia, ib = pi.ib;
@@ -1690,7 +1693,7 @@ __device__ void probe_pair(WorldDev& w, const ColliderSet& cs, uint32_t cur, uin
 // threads' top-4 multisets in voxel order; the threads build the contacts
 // that enter, and one thread adds them to the manifold in that order.
 constexpr uint32_t kBlockReplay = 64;
-__device__ void probe_pair_block(WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p, WarpManifold& sm) {
+__device__ void probe_pair_block(const WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p, WarpManifold& sm) {
     __shared__ Top4 s_top[32];
     __shared__ CandRec s_rec[kBlockReplay];
     const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = blockDim.x >> 5;
@@ -1858,7 +1861,7 @@ __device__ void probe_pair_block(WorldDev& w, const ColliderSet& cs, uint32_t cu
 }
 
 template <class G>
-__device__ bool phase_probe(G& g, WorldDev& w, const ColliderSet& cs, uint32_t cur, WarpManifold* warp_sm,
+__device__ bool phase_probe(G& g, const WorldDev& w, const ColliderSet& cs, uint32_t cur, WarpManifold* warp_sm,
                             const CacheSmem& csm) {
     const uint32_t lane = threadIdx.x & 31;
     WarpManifold& sm = warp_sm[threadIdx.x >> 5];
@@ -1891,7 +1894,7 @@ __device__ bool phase_probe(G& g, WorldDev& w, const ColliderSet& cs, uint32_t c
         uint32_t p = 0;
         if (lane == 0) p = atomicAdd(&w.ctr[C_WORK], 1u);
         p = __shfl_sync(0xffffffffu, p, 0);
-        if (p >= w.n_pairs) break;
+        if (p >= g.n_pairs) break;
         const uint32_t fl = w.pinfo[p].flags;
         if ((fl & (PF_DETECT | PF_CACHE)) && (fl & PF_REGION) && !(fl & PF_HEAVY)) probe_pair(w, cs, cur, p, sm);
     }
@@ -1916,9 +1919,9 @@ __device__ __forceinline__ void warm_from_prev(const WorldDev& w, uint32_t prev,
 }
 
 template <class G>
-__device__ bool phase_finalize(G& g, WorldDev& w, uint32_t cur, uint32_t prev) {
+__device__ bool phase_finalize(G& g, const WorldDev& w, uint32_t cur, uint32_t prev) {
     uint32_t skipped = 0, colliding = 0, contacts = 0, voxels = 0, manifolds = 0, cands = 0;
-    for (uint32_t p = g.rank(); p < w.n_pairs; p += g.size()) {
+    for (uint32_t p = g.rank(); p < g.n_pairs; p += g.size()) {
         const PairInfo& pi = w.pinfo[p];
         const uint32_t fl = pi.flags;
         ManifoldRec& m = w.man[cur][p];
@@ -2006,7 +2009,7 @@ __device__ bool phase_finalize(G& g, WorldDev& w, uint32_t cur, uint32_t prev) {
     if (!g.sync()) return false;
     // BrickPairCache.put values of this frame's misses (last writer wins)
     if (w.cfg.use_cache) {
-        for (uint32_t p = g.rank(); p < w.n_pairs; p += g.size()) {
+        for (uint32_t p = g.rank(); p < g.n_pairs; p += g.size()) {
             const PairInfo& pi = w.pinfo[p];
             if (!(pi.flags & PF_CACHE) || pi.hit != 2u) continue;
             if (pi.flags & (PF_NOCOLL | PF_SEPARATED)) continue;
@@ -2112,9 +2115,9 @@ __device__ __forceinline__ bool isl_unite(uint32_t* parent, uint32_t a, uint32_t
 }
 
 template <class G>
-__device__ bool phase_islands(G& g, WorldDev& w, uint32_t cur, uint32_t* scratch) {
+__device__ bool phase_islands(G& g, const WorldDev& w, uint32_t cur, uint32_t* scratch) {
     if (!w.cfg.islands_on || !w.isl_state) return true;
-    const uint32_t P = w.n_pairs, N = w.n_bodies;
+    const uint32_t P = g.n_pairs, N = w.n_bodies;
     uint32_t* st = w.isl_state;
     const uint32_t buf = *(volatile uint32_t*)&st[IS_BUF] & 1u, nprev = *(volatile uint32_t*)&st[IS_NKEYS];
     const unsigned long long* kp = w.isl_keys[buf];
@@ -2223,10 +2226,10 @@ __device__ bool phase_islands(G& g, WorldDev& w, uint32_t cur, uint32_t* scratch
 }
 
 template <class G>
-__device__ bool phase_constraints(G& g, WorldDev& w, uint32_t cur, uint32_t* M_out, uint32_t* ncol_out,
+__device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_t* M_out, uint32_t* ncol_out,
                                   bool islands = true) {
     if (islands && !phase_islands(g, w, cur, w.scan)) return false;
-    const uint32_t P = w.n_pairs, N = w.n_bodies;
+    const uint32_t P = g.n_pairs, N = w.n_bodies;
     // 1. solver constraint list: manifolds that are not both-sleeping, pair order
     for (uint32_t p = g.rank(); p < P; p += g.size()) {
         const ManifoldRec& m = w.man[cur][p];
@@ -2647,7 +2650,7 @@ __device__ __forceinline__ void apply_impulse(BV& b, F3 imp, F3 r) {  // BodySta
     b.v = F3{b.wr ? v2.x : b.v.x, b.wr ? v2.y : b.v.y, b.wr ? v2.z : b.v.z};
     b.w = F3{b.wr ? w2.x : b.w.x, b.wr ? w2.y : b.w.y, b.wr ? w2.z : b.w.z};
 }
-__device__ __forceinline__ void store_bv(WorldDev& w, uint32_t i, const BV& b) {
+__device__ __forceinline__ void store_bv(const WorldDev& w, uint32_t i, const BV& b) {
     if (!b.wr) return;
     w.body[i].v = make_float4(b.v.x, b.v.y, b.v.z, 0.f);
     w.body[i].w = make_float4(b.w.x, b.w.y, b.w.z, 0.f);
@@ -2735,7 +2738,7 @@ __device__ void prepare_point_s(const SolveFlags sf, const CPV vin, const CPV v,
         cpr(v, CP_TM1, i) = k2 > kEpsilon ? 1.0f / k2 : 0.0f;
     }
 }
-__device__ void prepare_point(WorldDev& w, uint32_t pos, uint32_t i, const Soft& soft, float hinv) {
+__device__ void prepare_point(const WorldDev& w, uint32_t pos, uint32_t i, const Soft& soft, float hinv) {
     const uint4 cmv = w.cm[pos];
     const BV a = load_bv(w, cmv.x), b = load_bv(w, cmv.y);
     const Qt qa = qof(w.body[cmv.x].q), qb = qof(w.body[cmv.y].q);
@@ -2759,7 +2762,7 @@ __device__ void warm_points(const CPV& v, uint32_t n, float scale, BV& a, BV& b)
         cpr(v, CP_TI1, i) = s2;
     }
 }
-__device__ void warm_manifold(WorldDev& w, uint32_t pos, float scale) {
+__device__ void warm_manifold(const WorldDev& w, uint32_t pos, float scale) {
     const uint4 cmv = w.cm[pos];
     BV a = load_bv(w, cmv.x), b = load_bv(w, cmv.y);
     warm_points(cpv_global(w, pos), cmv.z, scale, a, b);
@@ -2997,7 +3000,7 @@ __device__ __forceinline__ void velocity_points_rows(bool friction, float* rows,
         *reinterpret_cast<float2*>(r + CP_TI0) = make_float2(ti0, ti1);
     }
 }
-__device__ void velocity_manifold(WorldDev& w, uint32_t pos, const Soft& soft, bool use_bias) {
+__device__ void velocity_manifold(const WorldDev& w, uint32_t pos, const Soft& soft, bool use_bias) {
     const uint4 cmv = w.cm[pos];
     if (cmv.z == 0u) return;
     const float fr = w.cfr[pos].x;
@@ -3123,7 +3126,7 @@ __device__ void position_points_rows(const SolveFlags sf, const float* rows, uin
 }
 static_assert(CP_NX == 0 && CP_PX == 3 && CP_RAX == 6 && CP_RBX == 9 && CP_NM > CP_RBX,
               "position rows: normal, anchor a, anchor b, base separation in the first ten floats");
-__device__ void position_manifold(WorldDev& w, uint32_t pos, float* min_sep, float* max_pen) {
+__device__ void position_manifold(const WorldDev& w, uint32_t pos, float* min_sep, float* max_pen) {
     const uint4 cmv = w.cm[pos];
     const DBodyProp& pa = w.prop[cmv.x];
     const DBodyProp& pb = w.prop[cmv.y];
@@ -3140,7 +3143,7 @@ __device__ void position_manifold(WorldDev& w, uint32_t pos, float* min_sep, flo
 // End of one position sweep: reduce its min separation and max penetration
 // over the group and decide the early break (solver.zig:917-921).
 template <class G>
-__device__ bool pos_sweep_end(G& g, WorldDev& w, uint32_t it, float mn, float mx, bool* brk) {
+__device__ bool pos_sweep_end(G& g, const WorldDev& w, uint32_t it, float mn, float mx, bool* brk) {
     int32_t kmn = fkey(mn), kmx = fkey(mx);
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -3163,7 +3166,7 @@ __device__ bool pos_sweep_end(G& g, WorldDev& w, uint32_t it, float mn, float mx
 // Phase: solve (ContactSolver.solve, solver.zig:494-561)
 // ---------------------------------------------------------------------------
 template <class G>
-__device__ bool phase_solve(G& g, WorldDev& w, uint32_t M, uint32_t ncol) {
+__device__ bool phase_solve(G& g, const WorldDev& w, uint32_t M, uint32_t ncol) {
     const StepCfg& cf = w.cfg;
     const float dt = cf.dt;
     const bool has = M > 0u;
@@ -3469,7 +3472,7 @@ __device__ __noinline__ void flow_item(const FlowCtx fc, uint32_t k, uint32_t po
 // Waits until every lane of the warp sees its bodies' event counters at the
 // values given (at_least: at or past them).  Bounded: gives up after
 // kFlowTimeoutNs or when another warp gave up, returning false.
-__device__ __forceinline__ bool flow_wait(WorldDev& w, bool need_a, uint32_t a, uint32_t ea, bool need_b, uint32_t b,
+__device__ __forceinline__ bool flow_wait(const WorldDev& w, bool need_a, uint32_t a, uint32_t ea, bool need_b, uint32_t b,
                                           uint32_t eb, bool at_least) {
     bool ready = !need_a && !need_b;
     uint32_t spins = 0;
@@ -3503,7 +3506,7 @@ __device__ __forceinline__ bool flow_wait(WorldDev& w, bool need_a, uint32_t a, 
 // is chunk L * nblocks + b; the first fc.smem_chunks of them keep their
 // constraint-point fields in shared memory (fsm) for the whole solve.
 template <class G>
-__device__ bool flow_run(G& g, WorldDev& w, const FlowCtx& fc, float* fsm, uint32_t T, uint32_t k0, uint32_t k1,
+__device__ bool flow_run(G& g, const WorldDev& w, const FlowCtx& fc, float* fsm, uint32_t T, uint32_t k0, uint32_t k1,
                          float* mn, float* mx) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nwb = blockDim.x >> 5;
@@ -3555,7 +3558,7 @@ __device__ bool flow_run(G& g, WorldDev& w, const FlowCtx& fc, float* fsm, uint3
 }
 
 template <class G>
-__device__ bool phase_solve_flow(G& g, WorldDev& w, float* fsm, uint32_t M, uint32_t ncol) {
+__device__ bool phase_solve_flow(G& g, const WorldDev& w, float* fsm, uint32_t M, uint32_t ncol) {
     const StepCfg& cf = w.cfg;
     FlowCtx fc;
     fc.S = cf.substeps;
@@ -3727,7 +3730,7 @@ __device__ __forceinline__ size_t cluster_smem_bytes(uint32_t bcap, uint32_t nre
 }
 
 template <class G>
-__device__ bool phase_solve_cluster(G& g, WorldDev& w, uint32_t M, uint32_t ncol, unsigned char* smem,
+__device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_t ncol, unsigned char* smem,
                                     uint32_t smem_bytes) {
     const StepCfg& cf = w.cfg;
     const uint32_t C = g.nblocks(), k = g.block(), t = threadIdx.x, T = blockDim.x;
@@ -4175,7 +4178,7 @@ __device__ bool phase_solve_cluster(G& g, WorldDev& w, uint32_t M, uint32_t ncol
 // Phase: store (writeBack, storeImpulses, updateSleepStates)
 // ---------------------------------------------------------------------------
 template <class G>
-__device__ bool phase_store(G& g, WorldDev& w, uint32_t cur, uint32_t M, bool solved) {
+__device__ bool phase_store(G& g, const WorldDev& w, uint32_t cur, uint32_t M, bool solved) {
     const StepCfg& cf = w.cfg;
     for (uint32_t i = g.rank(); i < w.n_bodies; i += g.size()) {
         DBodyProp& pr = w.prop[i];
@@ -4244,7 +4247,7 @@ __device__ bool phase_store(G& g, WorldDev& w, uint32_t cur, uint32_t M, bool so
 // One whole step (VoxelPhysicsSystem.step with the pairs given)
 // ---------------------------------------------------------------------------
 template <class G>
-__device__ __forceinline__ void stamp(G& g, WorldDev& w, uint32_t slot) {
+__device__ __forceinline__ void stamp(G& g, const WorldDev& w, uint32_t slot) {
     if (g.rank() == 0 && w.ts) w.ts[slot] = global_ns();
 }
 
@@ -4252,7 +4255,7 @@ __device__ __forceinline__ void stamp(G& g, WorldDev& w, uint32_t slot) {
 // inverse inertia), the pair list, the narrow phase.  Returns true, and
 // leaves C_SOLVE_GO set, when the solve part of the step is to run.
 template <class G>
-__device__ bool world_step_narrow(G& g, WorldDev& w, const ColliderSet& cs, WarpManifold* warp_sm,
+__device__ bool world_step_narrow(G& g, const WorldDev& w, const ColliderSet& cs, WarpManifold* warp_sm,
                                   const CacheSmem& csm) {
     const uint32_t ph = w.cfg.phases;
     const uint32_t f0 = *(volatile uint32_t*)&w.frame[0];
@@ -4274,8 +4277,8 @@ __device__ bool world_step_narrow(G& g, WorldDev& w, const ColliderSet& cs, Warp
             return false;
         }
     } else {
-        w.n_pairs = *w.n_pairs_dev;
-        if ((ph & PH_NARROW) && w.n_pairs > w.pair_cap) {
+        g.n_pairs = *w.n_pairs_dev;
+        if ((ph & PH_NARROW) && g.n_pairs > w.pair_cap) {
             // the pair list did not fit: leave every state untouched, the
             // host grows the buffers and runs the step again
             if (g.rank() == 0) atomicOr(&w.ctr[C_ERROR], ERR_CAP);
@@ -4288,7 +4291,7 @@ __device__ bool world_step_narrow(G& g, WorldDev& w, const ColliderSet& cs, Warp
         const uint32_t cur = (f0 + 1u) & 1u, prev = cur ^ 1u;
         if (g.rank() == 0) {
             w.frame[0] = f0 + 1u;
-            w.frame[1] = w.n_pairs;
+            w.frame[1] = g.n_pairs;
         }
         if (!phase_pairs(g, w, cs, cur)) return false;
         stamp(g, w, TS_PAIRS);
@@ -4313,16 +4316,16 @@ enum : uint32_t {
 // (the parts run as two kernels).  part SOLVE_CONSTRAINTS stops after the
 // colouring and leaves M, ncol and C_SOLVE_GO = 2 for world_step_sweeps.
 template <class G>
-__device__ void world_step_solve(G& g, WorldDev& w, float* fsm, bool check_go, uint32_t part = SOLVE_ALL) {
+__device__ void world_step_solve(G& g, const WorldDev& w, float* fsm, bool check_go, uint32_t part = SOLVE_ALL) {
     const uint32_t ph = w.cfg.phases;
     if (!(ph & PH_SOLVE) || w.n_bodies == 0u) return;
     if (check_go && *(volatile uint32_t*)&w.ctr[C_SOLVE_GO] == 0u) return;
-    w.n_pairs = *(volatile uint32_t*)w.n_pairs_dev;
+    g.n_pairs = *(volatile uint32_t*)w.n_pairs_dev;
     const uint32_t cur = *(volatile uint32_t*)&w.frame[0] & 1u;  // the latest manifolds
     // The solver's work per colour batch is a few hundred manifolds: run it
     // on k blocks (one per solver_div manifolds, at least 2) with a cheaper
     // barrier.
-    const uint32_t nman = (ph & PH_NARROW) ? *(volatile uint32_t*)&w.ctr[C_MANIFOLDS] : w.n_pairs;
+    const uint32_t nman = (ph & PH_NARROW) ? *(volatile uint32_t*)&w.ctr[C_MANIFOLDS] : g.n_pairs;
     uint32_t want = max(2u, (nman + w.cfg.solver_div - 1u) / w.cfg.solver_div);
     // event-ordered sweeps: enough blocks to hold every chunk (at most
     // nman / 32 + one partial chunk per colour) in shared memory
@@ -4392,12 +4395,12 @@ __device__ void world_step_solve(G& g, WorldDev& w, float* fsm, bool check_go, u
 // configuration, the colouring's round count and the position sweeps' early
 // break, which every block reads from a slot that no block writes again
 // before the next barrier.
-__device__ __forceinline__ void world_step_sweeps(ClusterGroup& g, WorldDev& w, unsigned char* smem,
+__device__ __forceinline__ void world_step_sweeps(ClusterGroup& g, const WorldDev& w, unsigned char* smem,
                                                   uint32_t smem_bytes, bool whole) {
     const uint32_t ph = w.cfg.phases;
     if (!(ph & PH_SOLVE) || w.n_bodies == 0u) return;
     if (*(volatile uint32_t*)&w.ctr[C_SOLVE_GO] != (whole ? 1u : 2u)) return;
-    w.n_pairs = *(volatile uint32_t*)w.n_pairs_dev;
+    g.n_pairs = *(volatile uint32_t*)w.n_pairs_dev;
     const uint32_t cur = *(volatile uint32_t*)&w.frame[0] & 1u;
     uint32_t M, ncol;
     if (whole) {
@@ -4424,7 +4427,7 @@ __device__ __forceinline__ void world_step_sweeps(ClusterGroup& g, WorldDev& w, 
 // One whole step (VoxelPhysicsSystem.step with the pairs given) in one
 // kernel: the narrow part, then the solve part.
 template <class G>
-__device__ void world_step(G& g, WorldDev& w, const ColliderSet& cs, WarpManifold* warp_sm, const CacheSmem& csm,
+__device__ void world_step(G& g, const WorldDev& w, const ColliderSet& cs, WarpManifold* warp_sm, const CacheSmem& csm,
                            float* fsm) {
     if (world_step_narrow(g, w, cs, warp_sm, csm)) world_step_solve(g, w, fsm, false);
 }

@@ -234,10 +234,17 @@ struct CacheLook {
     unsigned long long th;
 };
 
+// A world as the kernels see it: the buffers and settings of one step, read
+// only.  The grid and cluster kernels take it as a kernel parameter, so a
+// field is an operand in the constant bank and no copy precedes the launch: a
+// copy per thread, 0.7 KB of stack, is 0.4 MB a CTA, more than the L1 it lives
+// in (kernels of the 4096-body pile's step 1421 -> 1304 us, of 523 boxes 667
+// -> 633).  The one-CTA kernel steps one of many worlds and keeps a copy per
+// thread, whose fields the compiler can hold in registers over the loops' stores; read
+// from shared memory, 256 worlds took 268 ms instead of 260.
 struct WorldDev {
     StepCfg cfg;
     uint32_t n_bodies;
-    uint32_t n_pairs;             // set from *n_pairs_dev at kernel start
     uint32_t* n_pairs_dev;        // pair count of this step (device)
     uint32_t pair_cap;
     uint32_t ht_cap;              // power of two >= 2 * pair_cap
