@@ -393,9 +393,9 @@ int vxp_set_launch_mode(vxp_ctx* ctx, int mode);
 int vxp_set_solver_blocks_divisor(vxp_ctx* ctx, uint32_t div);
 
 /* Narrow-phase work split: a pair whose overlap region holds at least n
- * voxels is probed by a whole CTA before the other pairs, which are probed one
- * warp each (default 2048; 0: every pair by one warp; the worlds of a batch,
- * one CTA each, use 1024).  Results do not depend on it. */
+ * voxels is cut into parts of about n / 4 voxels, probed by one warp each
+ * before the other pairs, which are probed one warp each (default 1024; 0:
+ * every pair by one warp).  Results do not depend on it. */
 int vxp_set_heavy_pair_voxels(vxp_ctx* ctx, uint32_t n);
 
 /* Narrow-phase probe tables: with enable (the default) every collider of at

@@ -382,3 +382,42 @@ def test_small_brick_pair_cache(vxp, mode, cache):
     sixty-fourths)."""
     sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=6, seed=2)
     lockstep(vxp, sc, 60, mode=mode, brick_pair_cache_size=cache, substeps=8).close()
+
+
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("tables", [True, False])
+@pytest.mark.parametrize("heavy", [1, 130])
+def test_cut_pairs_merge(vxp, mode, tables, heavy):
+    """Pairs cut into parts of 32 voxels whose candidates are merged (every
+    pair at heavy=1; candidates are not dumped, which would keep pairs whole),
+    far from the world origin, where the distance test's error bound is wide,
+    with and without probe tables: equal to the oracle bit for bit."""
+    sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=4, seed=9)
+    sc.bodies["position"] += np.array([700.0, 0.0, -300.0], dtype=np.float32)
+    g = vxp.VoxelPhysicsSystem(substeps=8)
+    g.load_scene(sc)
+    g.set_launch_mode(mode)
+    g.set_heavy_pair_voxels(heavy)
+    g.set_probe_tables(tables)
+    r = O.OracleWorld(substeps=8)
+    r.load_scene(sc)
+    dt = np.float32(sc.dt)
+    for s in range(90):
+        pairs = r.pairs()
+        g.step(dt, pairs)
+        r.step(dt, pairs)
+        assert g.manifolds().tobytes() == r.manifolds().tobytes(), f"step {s}: manifolds differ"
+        gs, rs = g.stats(), r.stats()
+        for k in STAT_KEYS:
+            assert gs[k] == rs[k], f"step {s}: stats[{k}] gpu {gs[k]} oracle {rs[k]}"
+    assert g.get_bodies().tobytes() == r.get_bodies().tobytes()
+    g.close()
+    r.close()
+
+
+@pytest.mark.parametrize("cache", [48, 63, 1000, 1039])
+def test_cache_replay_bins(vxp, cache):
+    """Brick-pair cache sizes at the edges of the replay's 16-slot bins: the
+    fewest bins, a last bin with a remainder, windows that wrap."""
+    sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=7, seed=3)
+    lockstep(vxp, sc, 50, mode=1, brick_pair_cache_size=cache, substeps=8).close()

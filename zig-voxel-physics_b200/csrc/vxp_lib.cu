@@ -327,6 +327,14 @@ std::string fmt(const char* f, ...) {
 }
 
 constexpr uint32_t kBlockThreads = 512;
+// Regions of at least this many voxels are cut into parts of a quarter of it.
+// A part costs some 4 us beyond its voxels (its pair's data, the log, the
+// merge), a group of 32 voxels about 1.3 us: probe phase of 523 boxes on the
+// grid 116 / 92 / 72 / 75 / 90 / 116 us at 128 / 256 / 512 / 1024 / 2048 /
+// 4096 voxels, of 4096 boxes 632 / 439 / 291 / 225 / 221 / 226, of 125 bodies
+// of 64^3 voxels 675 / 655 / 644 / 605 / 571 / 593 (3951 uncut), of 64 cubes
+// on one CTA 584 / 267 / 159 / 143 / 146 / 148.
+constexpr uint32_t kHeavyVoxels = 1024;
 // CTA sizes of the two cooperative grid kernels of a large world's step (one
 // CTA per SM each): the narrow part wants many warps to hide its memory
 // latency, the solve part wants registers for its long dependent chains.
@@ -978,7 +986,7 @@ StepCfg step_cfg(const vxp_config& c, float dt, uint32_t dump, uint32_t phases) 
     s.device_pairs = 0;
     s.margin = 0.1f;
     s.solver_flow = 1;
-    s.heavy_voxels = 1024;  // batches of small worlds: one CTA per world
+    s.heavy_voxels = kHeavyVoxels;
     s.count_bricks = 0;
     s.owner_groups = 1;
     s.islands_on = c.enable_islands;
@@ -1011,6 +1019,7 @@ struct WorldBuffers {
     DBuf<uint32_t> frame;
     DBuf<uint32_t> cons, colour, pos_of, packed_pair, adj, flag;
     DBuf<CacheLook> clist;
+    DBuf<uint2> part, part_log, plog;
     DBuf<float> cp, crow;
     // islands: per body, per pair slot (two builds' keys), kept state words
     DBuf<uint32_t> isl_parent, isl_flag, isl_size, isl_state;
@@ -1078,6 +1087,13 @@ struct WorldBuffers {
         ok &= flag.reserve(cap) == cudaSuccess;
         ok &= clist.reserve(cap) == cudaSuccess;
         ok &= cp.reserve((size_t)CP_NFIELDS * 4 * cap) == cudaSuccess;
+        // parts of cut pairs: a context's world (few pairs can be very large)
+        // gets room for 64 Ki and their candidates, a batch slot four a pair
+        // (its candidates go to cp)
+        const size_t parts = std::max<size_t>((size_t)4 * cap, spill_rows ? 65536 : 0);
+        ok &= part.reserve(parts) == cudaSuccess;
+        ok &= part_log.reserve(parts) == cudaSuccess;
+        if (spill_rows) ok &= plog.reserve(32 * parts) == cudaSuccess;
         if (spill_rows) ok &= crow.reserve((size_t)CP_NVEL * 4 * cap) == cudaSuccess;
         ok &= isl_keys0.reserve(cap, true) == cudaSuccess;
         ok &= isl_keys1.reserve(cap, true) == cudaSuccess;
@@ -1280,6 +1296,11 @@ struct WorldBuffers {
         w.cval = cval.p;
         w.cwriter = cwriter.p;
         w.clist = clist.p;
+        w.part = part.p;
+        w.part_log = part_log.p;
+        w.part_cap = (uint32_t)part.n;
+        w.plog = plog.p ? plog.p : reinterpret_cast<uint2*>(cp.p);
+        w.plog_cap = (uint32_t)(plog.p ? plog.n : cp.bytes() / sizeof(uint2));
         w.cframe = cframe.p;
         w.cons = cons.p;
         w.colour = colour.p;
@@ -1338,7 +1359,7 @@ struct WorldBuffers {
                ids.bytes() + pcount.bytes() + poff.bytes() + adj_off.bytes() + adj_cur.bytes() + bmask.bytes() +
                pairs.bytes() + pinfo.bytes() + man0.bytes() + man1.bytes() + ht0.bytes() + ht1.bytes() +
                cons.bytes() + colour.bytes() + pos_of.bytes() + packed_pair.bytes() + adj.bytes() + flag.bytes() +
-               clist.bytes() + cp.bytes() + cm.bytes() + rk.bytes() + ev.bytes() + snap.bytes() + chunk.bytes() + cfr.bytes() +
+               clist.bytes() + part.bytes() + part_log.bytes() + plog.bytes() + cp.bytes() + cm.bytes() + rk.bytes() + ev.bytes() + snap.bytes() + chunk.bytes() + cfr.bytes() +
                ckey.bytes() + cval.bytes() +
                cwriter.bytes() + scan.bytes() + ctr.bytes() + ts.bytes() + dump.bytes() + ocnt.bytes() + ocur.bytes() +
                stat.bytes() + bpmask.bytes() + crow.bytes() + isl_parent.bytes() + isl_flag.bytes() +
@@ -1451,7 +1472,7 @@ struct vxp_ctx {
     int use_grid = -1;  // -1 auto, 0 block, 1 grid
     uint32_t solver_div = 128;
     uint32_t solver_flow = 1;
-    uint32_t heavy_voxels = 2048;
+    uint32_t heavy_voxels = kHeavyVoxels;
     unsigned long long wait_limit_ns = 0;  // grid-barrier wait limit; 0: kGridWaitNs
     bool count_bricks = false;  // traffic accounting (C_BRICKS)
     bool record_substeps = false;

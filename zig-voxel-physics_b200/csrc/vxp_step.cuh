@@ -378,33 +378,32 @@ __device__ __forceinline__ void project8(const F3 v[8], F3 axis, float* mn, floa
     *mn = lo;
     *mx = hi;
 }
-__device__ bool sat_separated(const Obb& a, const Obb& b) {
+// The fifteen axes one after another in one rolled loop: a warp runs this
+// once or twice a step, so much of its time is the fetch of instructions seen
+// for the first time (pair filter of 523 boxes 35 us unrolled, 31 us so).
+__device__ __noinline__ bool sat_separated(const Obb& a, const Obb& b) {
     F3 aa[3], ab[3], va[8], vb[8];
     obb_axes(a, aa);
     obb_axes(b, ab);
     obb_verts(a, va);
     obb_verts(b, vb);
-    float p0, p1, q0, q1;
-    for (int i = 0; i < 3; ++i) {
-        project8(va, aa[i], &p0, &p1);
-        project8(vb, aa[i], &q0, &q1);
-        if (p1 < q0 || q1 < p0) return true;
-    }
-    for (int i = 0; i < 3; ++i) {
-        project8(va, ab[i], &p0, &p1);
-        project8(vb, ab[i], &q0, &q1);
-        if (p1 < q0 || q1 < p0) return true;
-    }
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) {
+#pragma unroll 1
+    for (int t = 0; t < 15; ++t) {
+        F3 ax;
+        if (t < 6) {
+            ax = t < 3 ? aa[t] : ab[t - 3];
+        } else {
+            const int i = (t - 6) / 3, j = (t - 6) % 3;
             const F3 cr = cross3(aa[i], ab[j]);
             const float l = len3(cr);
             if (l < 0.001f) continue;
-            const F3 ax = cr * (1.0f / l);
-            project8(va, ax, &p0, &p1);
-            project8(vb, ax, &q0, &q1);
-            if (p1 < q0 || q1 < p0) return true;
+            ax = cr * (1.0f / l);
         }
+        float p0, p1, q0, q1;
+        project8(va, ax, &p0, &p1);
+        project8(vb, ax, &q0, &q1);
+        if (p1 < q0 || q1 < p0) return true;
+    }
     return false;
 }
 
@@ -746,6 +745,7 @@ __device__ bool phase_broadphase(G& g, const WorldDev& w, const ColliderSet& cs,
 // ---------------------------------------------------------------------------
 // Phase: pairs (system.narrowPhase filter + processPair head)
 // ---------------------------------------------------------------------------
+constexpr uint32_t kMaxParts = 32, kMaxPartVoxels = 1024;
 template <class G>
 __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint32_t cur) {
     const uint32_t P = g.n_pairs;
@@ -771,6 +771,7 @@ __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint
         pi.flags = fl;
         pi.voxels_checked = 0;
         pi.candidates = 0;
+        pi.parts_done = 0;
         pi.hit = 0u;
         pi.cache_slot = 0xFFFFFFFFu;
         w.flag[p] = (fl & PF_CARRY) ? 0u : 1u;
@@ -788,10 +789,11 @@ __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint
             return false;
     }
     uint32_t tested = 0;
-    for (uint32_t p = g.rank(); p < P; p += g.size()) {
+    // one pair: returns whether it is to be probed by one warp
+    auto test = [&](uint32_t p) -> bool {
         PairInfo& pi = w.pinfo[p];
         uint32_t fl = pi.flags;
-        if (fl & (PF_CARRY | PF_DROPPED | PF_INVALID)) continue;
+        if (fl & (PF_CARRY | PF_DROPPED | PF_INVALID)) return false;
         fl |= PF_TESTED;
         ++tested;
         const DBody& A = w.body[pi.ia];
@@ -800,8 +802,10 @@ __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint
         const DBodyProp& pb = w.prop[pi.ib];
         if (pa.collider >= cs.n || pb.collider >= cs.n) {
             pi.flags = fl | PF_NOCOLL;
-            continue;
+            return false;
         }
+        pi.ca = pa.collider;
+        pi.cb = pb.collider;
         const DCollider& ca = cs.c[pa.collider];
         const DCollider& cb = cs.c[pb.collider];
         const F3 xa = f3of(A.p), xb = f3of(B.p);
@@ -809,7 +813,7 @@ __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint
         if (w.cfg.use_sat) {
             if (sat_separated(obb_from(ca, xa, qa), obb_from(cb, xb, qb))) {
                 pi.flags = fl | PF_SEPARATED;
-                continue;
+                return false;
             }
         }
         const bool use_cache =
@@ -825,24 +829,50 @@ __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint
         } else {
             fl |= PF_DETECT;
         }
+        bool light = false;
         I3 rmin, rmax;
         if (overlap_region(ca, xa, qa, cb, xb, qb, &rmin, &rmax)) {
             if (rmin.x <= rmax.x && rmin.y <= rmax.y && rmin.z <= rmax.z) {
                 fl |= PF_REGION;
-                // a large region is probed by a whole CTA (listed in w.cons,
-                // which is free until phase_constraints)
+                // a large region is cut into parts of a quarter of the limit
+                // (at most kMaxParts, which then are larger); the other pairs
+                // are listed in w.colour, which is free until
+                // phase_constraints, and so is a pair the part list has no
+                // room for, and every pair while candidates are dumped (a
+                // part may be probed twice)
                 const unsigned long long V = (unsigned long long)(rmax.x - rmin.x + 1) *
                                              (unsigned long long)(rmax.y - rmin.y + 1) *
                                              (unsigned long long)(rmax.z - rmin.z + 1);
-                if (w.cfg.heavy_voxels && V >= w.cfg.heavy_voxels) {
-                    fl |= PF_HEAVY;
-                    w.cons[atomicAdd(&w.ctr[C_NHEAVY], 1u)] = p;
+                uint32_t parts = 0;
+                if (w.cfg.heavy_voxels && V >= w.cfg.heavy_voxels && V < (1ull << 27) && !w.cfg.dump_candidates) {
+                    const uint32_t len = max(32u, min(kMaxPartVoxels, w.cfg.heavy_voxels / 4u));
+                    parts = (uint32_t)min((unsigned long long)kMaxParts, (V + len - 1u) / len);
+                    pi.parts = parts;
+                    const uint32_t at = atomicAdd(&w.ctr[C_NHEAVY], parts);
+                    const bool fits = at < w.part_cap && parts <= w.part_cap - at;
+                    for (uint32_t j = 0; j < parts && at + j < w.part_cap; ++j)
+                        w.part[at + j] = make_uint2(fits ? p : 0xFFFFFFFFu, j);
+                    if (!fits) parts = 0u;
                 }
+                if (parts) fl |= PF_HEAVY;
+                else light = true;
             }
             pi.rmin[0] = rmin.x; pi.rmin[1] = rmin.y; pi.rmin[2] = rmin.z;
             pi.rmax[0] = rmax.x; pi.rmax[1] = rmax.y; pi.rmax[2] = rmax.z;
         }
         pi.flags = fl;
+        return light;
+    };
+    // (whole warps, for the list's places: one add a warp)
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t p0 = g.rank() - lane; p0 < P; p0 += g.size()) {
+        const bool light = p0 + lane < P && test(p0 + lane);
+        const uint32_t who = __ballot_sync(0xffffffffu, light);
+        if (who == 0u) continue;
+        uint32_t at = 0;
+        if (lane == 0u) at = atomicAdd(&w.ctr[C_NLIGHT], (uint32_t)__popc(who));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (light) w.colour[at + (uint32_t)__popc(who & ((1u << lane) - 1u))] = p0 + lane;
     }
     tested = warp_sum(tested);
     if ((threadIdx.x & 31) == 0 && tested) atomicAdd(&w.ctr[C_PAIRS_TESTED], tested);
@@ -1071,33 +1101,37 @@ __device__ void cache_replay(const WorldDev& w, const CacheSmem& t) {
     }
 }
 
-// The same replay on a whole CTA (the grid step's CTA 0, which detects
-// nothing), for tables of at least 64 x 16 slots.  Up to kCtaReplayPending
-// lookups are pending, in order, one per thread; each round every pending
-// lookup whose window overlaps no earlier pending one is ready (the
-// sixty-fourths prefix OR of cache_replay, over the block), the ready ones run
-// at once, each scanned by sixteen lanes (a ballot finds the first empty slot
-// and the key, a min-reduction the least recently used slot), and the rest
-// move up in order.  The windows of a round are disjoint, so every lookup
-// sees the state the sequential replay gives it.  scratch: at least
-// cta_replay_scratch_bytes() bytes (the block's unused warp scratch).
-constexpr uint32_t kCtaReplayPending = 256;
-__host__ __device__ constexpr size_t cta_replay_scratch_bytes() {
-    return 2u * kCtaReplayPending * sizeof(CacheLook) + kCtaReplayPending * sizeof(uint16_t) +
-           32u * sizeof(unsigned long long) + 32u * sizeof(uint32_t) + 4u * sizeof(uint32_t);
+// The same replay on a whole CTA (CTA 0 of a step on several, which detects
+// nothing), for tables of at least 48 slots.  The table is cut into bins of
+// 16 slots (the last one takes the remainder), so a window touches its
+// start's bin and the next at most; a lookup is taken after every earlier one
+// that touches either bin.  One warp numbers each bin's lookups in order
+// (tickets), a batch of kReplayBatch at a time; then the half-warps take the
+// lookups in turn, each waiting until both its bins have come to its tickets
+// and advancing them when it is through.  Half-warp h takes lookups h, h +
+// halves, ... in order, so the earliest lookup not yet taken is always some
+// half-warp's current one and its bins are free: the replay ends.  The wait
+// is bounded all the same (kReplayTimeoutNs, ERR_TIMEOUT).
+// The time is the longest chain of lookups with overlapping windows, about a
+// hundred of 1.9k on the pile, of some 200 cycles each; rounds of 256 pending
+// lookups with five block barriers a round took 205 us there.
+constexpr uint32_t kReplayBatch = 2048;
+constexpr unsigned long long kReplayTimeoutNs = 2000000000ull;
+__host__ __device__ constexpr size_t cta_replay_scratch_bytes(uint32_t cap) {
+    return kReplayBatch * sizeof(ushort2) + 3u * (cap / 16u) * sizeof(uint32_t);
 }
 
 __device__ void cache_replay_cta(const WorldDev& w, const CacheSmem& t, unsigned char* scratch) {
-    const uint32_t tid = threadIdx.x, T = blockDim.x, lane = tid & 31u, wid = tid >> 5;
-    const uint32_t cap = w.cache_cap;
+    const uint32_t tid = threadIdx.x, T = blockDim.x, lane = tid & 31u;
+    const uint32_t cap = w.cache_cap, nb = cap / 16u;
     const uint32_t frame = (uint32_t)w.cframe[0];
     const uint32_t n = w.ctr[C_NCACHE];
-    CacheLook* bufA = reinterpret_cast<CacheLook*>(scratch);
-    CacheLook* bufB = bufA + kCtaReplayPending;
-    uint16_t* rdy = reinterpret_cast<uint16_t*>(bufB + kCtaReplayPending);
-    unsigned long long* s_or = reinterpret_cast<unsigned long long*>(rdy + kCtaReplayPending);
-    uint32_t* s_cnt = reinterpret_cast<uint32_t*>(s_or + 32);
-    uint32_t* s_tot = s_cnt + 32;
+    const CacheLook* list = w.clist;
+    ushort2* ticket = reinterpret_cast<ushort2*>(scratch);
+    volatile uint32_t* turn = reinterpret_cast<uint32_t*>(ticket + kReplayBatch);
+    uint32_t* cnt = const_cast<uint32_t*>(turn) + nb;
+    uint32_t* touch = cnt + nb;
+    auto bin_of = [&](uint32_t start) { return min(start / 16u, nb - 1u); };
     for (uint32_t i = tid; i < cap; i += T) {
         const CacheKeyRec k = w.ckey[i];
         t.ab[i] = make_uint2(k.a, k.b);
@@ -1105,122 +1139,129 @@ __device__ void cache_replay_cta(const WorldDev& w, const CacheSmem& t, unsigned
         t.lu[i] = k.valid ? (uint32_t)k.last_used : 0u;
     }
     uint32_t hits = 0, misses = 0, evictions = 0;
-    CacheLook* P = bufA;
-    CacheLook* Q = bufB;
-    uint32_t np = 0, taken = 0;
-    const uint32_t nw = (kCtaReplayPending + 31u) / 32u;  // warps holding pending entries
-    for (;;) {
-        // fill the pending list up to its capacity, in order
-        const uint32_t take = min(kCtaReplayPending - np, n - taken);
-        for (uint32_t i = tid; i < take; i += T) P[np + i] = w.clist[taken + i];
-        taken += take;
-        np += take;
-        __syncthreads();
-        if (np == 0u) break;
-        // ready: no earlier pending window in the same or an adjacent sixty-fourth
-        const bool pending = tid < np;
-        uint32_t bk = 0;
-        unsigned long long m = 0ull;
-        if (pending) {
-            bk = (uint32_t)(((unsigned long long)P[tid].start * 64ull) / cap);
-            m = 1ull << bk;
+    const uint32_t l16 = lane & 15u, halves = T >> 4, half = tid >> 4, sh = lane & 16u;
+    for (uint32_t b0 = 0; b0 < n; b0 += kReplayBatch) {
+        const uint32_t m = min(kReplayBatch, n - b0);
+        for (uint32_t i = tid; i < nb; i += T) {
+            turn[i] = 0u;
+            cnt[i] = 0u;
+            touch[i] = 0u;
         }
-        unsigned long long inc = m;
-#pragma unroll
-        for (uint32_t d = 1; d < 32u; d <<= 1) {
-            const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, d);
-            if (lane >= d) inc |= o;
-        }
-        if (lane == 31u && wid < nw) s_or[wid] = inc;
         __syncthreads();
-        unsigned long long ex = __shfl_up_sync(0xffffffffu, inc, 1);
-        if (lane == 0u) ex = 0ull;
-        for (uint32_t k = 0; k < wid && k < nw; ++k) ex |= s_or[k];
-        const unsigned long long near =
-            m | (m << 1) | (m >> 1) | (bk == 0u ? 1ull << 63 : 0ull) | (bk == 63u ? 1ull : 0ull);
-        const bool ready = pending && !(ex & near);
-        // positions: ready ones in a list, the others moved up into Q in order
-        const uint32_t c = ready ? 1u : (pending ? 0x10000u : 0u);
-        uint32_t ci = c;
-#pragma unroll
-        for (uint32_t d = 1; d < 32u; d <<= 1) {
-            const uint32_t o = __shfl_up_sync(0xffffffffu, ci, d);
-            if (lane >= d) ci += o;
-        }
-        if (lane == 31u && wid < nw) s_cnt[wid] = ci;
-        __syncthreads();
-        if (tid == 0) {
-            uint32_t run = 0;
-            for (uint32_t k = 0; k < nw; ++k) {
-                const uint32_t v = s_cnt[k];
-                s_cnt[k] = run;
-                run += v;
+        if (tid < 32u) {
+            const uint32_t lt = (1u << lane) - 1u;
+            uint32_t ns = lane < m ? list[b0 + lane].start : 0u;
+            for (uint32_t i0 = 0; i0 < m; i0 += 32u) {
+                const bool act = i0 + lane < m;
+                const uint32_t b = bin_of(ns), bn = b + 1u < nb ? b + 1u : 0u, bp = b ? b - 1u : nb - 1u;
+                if (i0 + 32u + lane < m) ns = list[b0 + i0 + 32u + lane].start;
+                if (act) atomicOr(&touch[b], 1u << lane);
+                __syncwarp();
+                uint32_t q0 = 0, q1 = 0;
+                if (act) {
+                    const uint32_t mb = touch[b];
+                    // the lookups touching bin b start in b or the bin before it
+                    q0 = mb | touch[bp];
+                    q1 = mb | touch[bn];
+                    ticket[i0 + lane] = make_ushort2((unsigned short)(cnt[b] + (uint32_t)__popc(q0 & lt)),
+                                                     (unsigned short)(cnt[bn] + (uint32_t)__popc(q1 & lt)));
+                }
+                __syncwarp();
+                if (act) {
+                    atomicAdd(&cnt[b], 1u);
+                    atomicAdd(&cnt[bn], 1u);
+                    touch[b] = 0u;
+                }
+                __syncwarp();
             }
-            *s_tot = run;
         }
         __syncthreads();
-        const uint32_t off = (wid < nw ? s_cnt[wid] : 0u) + ci - c;
-        if (ready) rdy[off & 0xFFFFu] = (uint16_t)tid;
-        else if (pending) Q[off >> 16] = P[tid];
-        __syncthreads();
-        const uint32_t tot = *s_tot, nready = tot & 0xFFFFu;
-        // the ready lookups, sixteen lanes each (the windows are disjoint)
-        const uint32_t l16 = tid & 15u, grp = tid >> 4, ngrp = T >> 4;
-        const uint32_t half = (lane >> 4) << 4;
-        for (uint32_t j0 = 0; j0 < nready; j0 += ngrp) {
-            const uint32_t j = j0 + grp;
-            const bool act = j < nready;
-            CacheLook L{0u, 0u, 0u, 0u, 0ull};
-            if (act) L = P[rdy[j]];
+        uint32_t i = half;
+        CacheLook L{0u, 0u, 0u, 0u, 0ull}, N{0u, 0u, 0u, 0u, 0ull};
+        uint32_t k0 = 0, k1 = 0, t0 = 0, t1 = 0;
+        if (i < m) L = list[b0 + i];
+        if (i + halves < m) N = list[b0 + i + halves];
+        auto take = [&]() {
+            k0 = bin_of(L.start);
+            k1 = k0 + 1u < nb ? k0 + 1u : 0u;
+            if (i < m) {
+                t0 = ticket[i].x;
+                t1 = ticket[i].y;
+            }
+        };
+        take();
+        unsigned long long since = 0;
+        uint32_t spins = 0;
+        while (__any_sync(0xffffffffu, i < m)) {
+            bool act = i < m && turn[k0] == t0 && turn[k1] == t1;
+            act = __shfl_sync(0xffffffffu, (int)act, (int)sh) != 0;  // one verdict for the half-warp
+            if (!__any_sync(0xffffffffu, act)) {
+                if ((++spins & 1023u) == 0u) {
+                    if (since == 0u) since = global_ns();
+                    const bool late = global_ns() - since > kReplayTimeoutNs;
+                    if (__any_sync(0xffffffffu, late)) {
+                        if (lane == 0u) atomicOr(&w.ctr[C_ERROR], ERR_TIMEOUT);
+                        break;
+                    }
+                }
+                continue;
+            }
+            spins = 0;
+            since = 0;
+            __threadfence_block();
+            // get: the first empty slot (miss) or the key (hit), whichever
+            // comes first; put after a miss: that empty slot, else the first
+            // least recently used one
             uint32_t x = L.start + l16;
             if (x >= cap) x -= cap;
+            uint32_t lu = 0xFFFFFFFFu;
             bool empty = false, match = false;
-            unsigned long long key = ~0ull;
             if (act) {
-                const uint32_t lu = t.lu[x];
+                lu = *(volatile uint32_t*)&t.lu[x];
                 const uint2 ab = t.ab[x];
                 const unsigned long long th = t.th[x];
                 empty = lu == 0u;
                 match = !empty && ab.x == L.a && ab.y == L.b && th == L.th;
-                if (!empty) key = ((unsigned long long)lu << 32) | l16;
             }
-            const uint32_t be = (__ballot_sync(0xffffffffu, empty) >> half) & 0xFFFFu;
-            const uint32_t bm = (__ballot_sync(0xffffffffu, match) >> half) & 0xFFFFu;
+            const uint32_t be = (__ballot_sync(0xffffffffu, empty) >> sh) & 0xFFFFu;
+            const uint32_t bm = (__ballot_sync(0xffffffffu, match) >> sh) & 0xFFFFu;
+            uint32_t least = lu;
 #pragma unroll
-            for (uint32_t d = 8; d > 0; d >>= 1) {
-                const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, d, 16);
-                key = o < key ? o : key;
-            }
-            if (act && l16 == 0u) {
-                const uint32_t fi = be ? (uint32_t)(__ffs(be) - 1) : 16u;
-                const uint32_t fm = bm ? (uint32_t)(__ffs(bm) - 1) : 16u;
-                const uint32_t mi = (uint32_t)(key & 0xFFFFu);
-                const bool hit = fm < fi;
-                const bool evict = !hit && fi == 16u;
-                uint32_t target = L.start + (hit ? fm : (evict ? mi : fi));
+            for (uint32_t d = 8; d > 0; d >>= 1) least = min(least, __shfl_xor_sync(0xffffffffu, least, d, 16));
+            const uint32_t bl = (__ballot_sync(0xffffffffu, lu == least) >> sh) & 0xFFFFu;
+            if (act) {
+                const uint32_t fi = be ? (uint32_t)(__ffs(be) - 1) : 16u, fm = bm ? (uint32_t)(__ffs(bm) - 1) : 16u;
+                const bool hit = fm < fi, evict = !hit && fi == 16u;
+                uint32_t target = L.start + (hit ? fm : (evict ? (uint32_t)(__ffs(bl) - 1) : fi));
                 if (target >= cap) target -= cap;
-                PairInfo& pi = w.pinfo[L.p];
-                t.lu[target] = frame;
-                if (hit) {
-                    pi.hit = 1u;
-                    ++hits;
-                } else {
-                    t.ab[target] = make_uint2(L.a, L.b);
-                    t.th[target] = L.th;
-                    w.cwriter[target] = L.p;
-                    pi.hit = 2u;
-                    ++misses;
-                    if (evict) ++evictions;
+                if (l16 == 0u) {
+                    t.lu[target] = frame;
+                    if (hit) {
+                        ++hits;
+                    } else {
+                        t.ab[target] = make_uint2(L.a, L.b);
+                        t.th[target] = L.th;
+                        w.cwriter[target] = L.p;
+                        ++misses;
+                        if (evict) ++evictions;
+                    }
+                    __threadfence_block();
+                    turn[k0] = t0 + 1u;
+                    turn[k1] = t1 + 1u;
+                    PairInfo& pi = w.pinfo[L.p];
+                    pi.hit = hit ? 1u : 2u;
+                    pi.cache_slot = target;
                 }
-                pi.cache_slot = target;
+                i += halves;
+                L = N;
+                if (i + halves < m) N = list[b0 + i + halves];
+                take();
             }
+            __syncwarp();
         }
         __syncthreads();
-        CacheLook* tmp = P;
-        P = Q;
-        Q = tmp;
-        np = tot >> 16;
     }
+    __syncthreads();
     for (uint32_t i = tid; i < cap; i += T) {
         CacheKeyRec k;
         k.a = t.ab[i].x;
@@ -1245,48 +1286,12 @@ __device__ void cache_replay_cta(const WorldDev& w, const CacheSmem& t, unsigned
 // ---------------------------------------------------------------------------
 // Phase: probe (detectVoxelCollisions + checkNeighborhood + addContact)
 // ---------------------------------------------------------------------------
-// Top-4 multiset of penetrations, sorted descending, -inf padded.
-struct Top4 {
-    float v[4];
-};
-__device__ __forceinline__ Top4 top4_empty() {
-    const float ni = -__int_as_float(0x7f800000);
-    return Top4{{ni, ni, ni, ni}};
-}
-__device__ __forceinline__ void cswap_desc(float& a, float& b) {
-    const float hi = fmaxf(a, b), lo = fminf(a, b);
-    a = hi;
-    b = lo;
-}
-// Top four of the union of two descending multisets.
-__device__ __forceinline__ Top4 top4_merge(const Top4& a, const Top4& b) {
-    Top4 c{{fmaxf(a.v[0], b.v[3]), fmaxf(a.v[1], b.v[2]), fmaxf(a.v[2], b.v[1]), fmaxf(a.v[3], b.v[0])}};
-    cswap_desc(c.v[0], c.v[2]);
-    cswap_desc(c.v[1], c.v[3]);
-    cswap_desc(c.v[0], c.v[1]);
-    cswap_desc(c.v[2], c.v[3]);
-    return c;
-}
-__device__ __forceinline__ void top4_insert(Top4& t, float x) {
-    if (!(x > t.v[3])) return;
-    t.v[3] = x;
-    cswap_desc(t.v[2], t.v[3]);
-    cswap_desc(t.v[1], t.v[2]);
-    cswap_desc(t.v[0], t.v[1]);
-}
-__device__ __forceinline__ Top4 top4_shfl_up(const Top4& t, int d) {
-    Top4 r;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) r.v[i] = __shfl_up_sync(0xffffffffu, t.v[i], d);
-    return r;
-}
-
 struct ProbeCtx {
     const DCollider* ca;
     const DCollider* cb;
     F3 pa, pb;
     Qt qa, qb, qna, qnb;
-    float vs_a, vs_b, spec;
+    float vs_a, vs_b;
 };
 
 // The 27 neighbour offsets in checkNeighborhood order: dz, dy, dx in {-1,0,1}.
@@ -1342,522 +1347,638 @@ __device__ void generate_contact(const ProbeCtx& c, uint32_t va, I3 ia, F3 wa, u
     out->feature_id = feature_id(ia, ib);
 }
 
-// checkNeighborhood (narrow_phase.zig:796-857) for one A voxel: its 27
-// probes in dz, dy, dx order, clipped to B's voxel bounds first (a probe
-// outside them is skipped, isValidCoord); for each non-empty B voxel the
-// type filter, the distance test and, for a pass, the candidate's penetration
-// into the lane's top-4 and its bit (dz*9 + dy*3 + dx, offsets from -1) into
-// the mask.
-__device__ __forceinline__ int32_t clip_lo(int32_t bound, int32_t centre) {
-    const long long d = (long long)bound - (long long)centre;
-    return d > -1 ? (d > 2 ? 2 : (int32_t)d) : -1;
-}
-__device__ __forceinline__ int32_t clip_hi(int32_t bound_excl, int32_t centre) {
-    const long long d = (long long)bound_excl - 1ll - (long long)centre;
-    return d < 1 ? (d < -2 ? -2 : (int32_t)d) : 1;
-}
-__device__ __forceinline__ void probe_neighbourhood(const WorldDev& w, const ColliderSet& cs, const ProbeCtx& c, uint32_t p,
-                                                    uint32_t ta, int32_t x, int32_t y, int32_t z, F3 wa, I3 cbv,
-                                                    uint32_t* mask, Top4* t, uint32_t* checked) {
-    const DCollider& cb = *c.cb;
-    if (cb.nb_off != kNoTable) {
-        // one lookup gives the non-empty probes (counted as checked) and those
-        // passing type_filter(ta, tb) (ta is never empty here); only the
-        // latter are transformed and distance-tested, in probe order.  A
-        // centre outside [min_bound - 1, max_bound] has no neighbour in bounds.
-        const uint32_t ex = (uint32_t)(cb.max_bound[0] - cb.min_bound[0]) + 2u,
-                       ey = (uint32_t)(cb.max_bound[1] - cb.min_bound[1]) + 2u,
-                       ez = (uint32_t)(cb.max_bound[2] - cb.min_bound[2]) + 2u;
-        const uint32_t tx = (uint32_t)cbv.x - ((uint32_t)cb.min_bound[0] - 1u),
-                       ty = (uint32_t)cbv.y - ((uint32_t)cb.min_bound[1] - 1u),
-                       tz = (uint32_t)cbv.z - ((uint32_t)cb.min_bound[2] - 1u);
-        if (tx >= ex || ty >= ey || tz >= ez) return;
-        const uint4 nm = __ldg(cs.nb + cb.nb_off + (tx + ex * (ty + ey * tz)));
-        *checked += (uint32_t)__popc(nm.x);
-        const uint32_t ps = ta == kCorner ? nm.x : (ta == kEdge ? nm.z : nm.y);
-        for (uint32_t m = ps; m; m &= m - 1u) {
-            const uint32_t k = __ffs(m) - 1;
-            const I3 o = probe_offset(k);
-            const int32_t bx = cbv.x + o.x, by = cbv.y + o.y, bz = cbv.z + o.z;
-            const F3 wb = transform_point_n(c.pb, c.qnb, voxel_to_local(c.vs_b, bx, by, bz));
-            const F3 diff = wb - wa;
-            const float d2 = lensq3(diff);
-            const bool pass = d2 < c.spec;
-            if (w.cfg.dump_candidates) {
-                const uint32_t slot = atomicAdd(&w.ctr[C_DUMP_N], 1u);
-                if (slot < w.dump_cap) {
-                    WorldDev::Cand& r = w.dump[slot];
-                    r.pair_index = p;
-                    r.a[0] = x; r.a[1] = y; r.a[2] = z;
-                    r.b[0] = bx; r.b[1] = by; r.b[2] = bz;
-                    r.passed = pass ? 1u : 0u;
-                    r.dist_sq = d2;
-                }
+// The masks of the 27 probes of checkNeighborhood (narrow_phase.zig:796-857)
+// around B's voxel cbv, bit dz*9 + dy*3 + dx (offsets from -1), clipped to B's
+// voxel bounds (a probe outside them is skipped, isValidCoord): non-empty,
+// corner, corner or edge, inside.  From B's table; without one, by the same
+// 27 lookups that build a table entry.
+__device__ __noinline__ uint4 probe_masks_lookup(const ColliderSet& cs, const DCollider& cb, I3 cbv) {
+    uint32_t ne = 0u, co = 0u, ec = 0u, in = 0u;
+    for (int32_t dz = -1; dz <= 1; ++dz)
+        for (int32_t dy = -1; dy <= 1; ++dy)
+            for (int32_t dx = -1; dx <= 1; ++dx) {
+                // 64-bit: a centre saturated by the float conversion must not wrap
+                const long long bx = (long long)cbv.x + dx, by = (long long)cbv.y + dy, bz = (long long)cbv.z + dz;
+                if (bx < cb.min_bound[0] || bx >= cb.max_bound[0] || by < cb.min_bound[1] || by >= cb.max_bound[1] ||
+                    bz < cb.min_bound[2] || bz >= cb.max_bound[2])
+                    continue;
+                const uint32_t tb = vtype(voxel_at(cs, cb, (int32_t)bx, (int32_t)by, (int32_t)bz));
+                const uint32_t bit = 1u << ((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1));
+                if (tb != kEmpty) ne |= bit;
+                if (tb == kCorner) co |= bit;
+                if (tb == kCorner || tb == kEdge) ec |= bit;
+                if (tb == kInside) in |= bit;
             }
-            if (pass) {
-                *mask |= 1u << k;
-                top4_insert(*t, cand_pen(c.vs_a, ta, ((nm.w >> k) & 1u) ? (uint32_t)kInside : (uint32_t)kCorner, d2));
-            }
-        }
-        return;
-    }
-    const int32_t lx = clip_lo(cb.min_bound[0], cbv.x), hx = clip_hi(cb.max_bound[0], cbv.x);
-    const int32_t ly = clip_lo(cb.min_bound[1], cbv.y), hy = clip_hi(cb.max_bound[1], cbv.y);
-    const int32_t lz = clip_lo(cb.min_bound[2], cbv.z), hz = clip_hi(cb.max_bound[2], cbv.z);
-    if (lx > hx || ly > hy || lz > hz) return;
-    // the brick holding the centre voxel (every probe is inside B's voxel
-    // bounds, so inside its brick grid): probes in the same brick read their
-    // byte at a fixed offset from the centre's, the others look their brick up
-    const int32_t cx = cbv.x & 7, cy = cbv.y & 7, cz = cbv.z & 7;
-    const int32_t cslot = brick_slot(cs, cb, cbv.x >> 3, cbv.y >> 3, cbv.z >> 3);
-    const uint8_t* cvox = cs.vox + (size_t)(cb.brick_off + (uint32_t)max(cslot, 0)) * 512u +
-                          (uint32_t)(cx + 8 * cy + 64 * cz);
-    for (int32_t dz = lz; dz <= hz; ++dz)
-        for (int32_t dy = ly; dy <= hy; ++dy)
-            for (int32_t dx = lx; dx <= hx; ++dx) {
-                const uint32_t k = (uint32_t)((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1));
-                const int32_t bx = cbv.x + dx, by = cbv.y + dy, bz = cbv.z + dz;
-                const bool same = (uint32_t)(cx + dx) < 8u && (uint32_t)(cy + dy) < 8u && (uint32_t)(cz + dz) < 8u;
-                const uint32_t vb = same ? (cslot >= 0 ? (uint32_t)__ldg(cvox + (dx + 8 * dy + 64 * dz)) : 0u)
-                                         : voxel_at(cs, cb, bx, by, bz);
-                const uint32_t tb = vtype(vb);
-                if (tb == kEmpty) continue;
-                ++*checked;
-                if (!type_filter(ta, tb)) continue;
-                const F3 wb = transform_point_n(c.pb, c.qnb, voxel_to_local(c.vs_b, bx, by, bz));
-                const F3 diff = wb - wa;
-                const float d2 = lensq3(diff);
-                const bool pass = d2 < c.spec;
-                if (w.cfg.dump_candidates) {
-                    const uint32_t slot = atomicAdd(&w.ctr[C_DUMP_N], 1u);
-                    if (slot < w.dump_cap) {
-                        WorldDev::Cand& r = w.dump[slot];
-                        r.pair_index = p;
-                        r.a[0] = x; r.a[1] = y; r.a[2] = z;
-                        r.b[0] = bx; r.b[1] = by; r.b[2] = bz;
-                        r.passed = pass ? 1u : 0u;
-                        r.dist_sq = d2;
-                    }
-                }
-                if (pass) {
-                    *mask |= 1u << k;
-                    top4_insert(*t, cand_pen(c.vs_a, ta, tb, d2));
-                }
-            }
+    return make_uint4(ne, co, ec, in);
 }
 
-// A candidate entering the manifold during detection: penetration, feature
-// id, and where it came from (A voxel li of the region in loop order, probe
-// k).  Its contact is built only if it is still in the manifold when the pair
-// ends: a contact's fields are a function of (li, k), and the impulses of
-// every contact added during detection are zero.
-struct CandRec {
-    unsigned long long fid;
-    float pen;
-    uint32_t li, k, _pad;
+// floor(p / vs) with the quotient rounded as an IEEE division, through the
+// reciprocal: p * rvs is within 2^-22 of the quotient, relatively, so away
+// from the integers both have the same floor; near one (or for a value the
+// bound says nothing about) the division decides.
+__device__ __forceinline__ int32_t floor_div(float p, float vs, float rvs) {
+    const float q = p * rvs;
+    const float d = fabsf(q - rintf(q));
+    if (!(d > fabsf(q) * 0x1p-20f + 1e-30f)) return (int32_t)floorf(p / vs);
+    return (int32_t)floorf(q);
+}
+// The quaternion Quat.rotate really uses: renormalised when |q|^2 is outside
+// [0.99, 1.01].  qrotate(q, v) == qrotate_unit(rotation_of(q), v).
+__device__ __forceinline__ Qt rotation_of(Qt q) {
+    const float l2 = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+    return (l2 < 0.99f || l2 > 1.01f) ? qnormalize(q) : q;
+}
+// l / d and l % d: below 2^24 by a float reciprocal (off by at most one, put
+// right by the remainder), a quarter of the instructions of the division.
+__device__ __forceinline__ uint32_t div_mod(uint32_t l, uint32_t d, uint32_t* rem) {
+    if ((l | d) >> 24) {
+        const uint32_t q = l / d;
+        *rem = l - q * d;
+        return q;
+    }
+    uint32_t q = (uint32_t)__fdividef((float)l, (float)d);
+    int32_t r = (int32_t)(l - q * d);
+    if (r < 0) {
+        --q;
+        r += (int32_t)d;
+    } else if (r >= (int32_t)d) {
+        ++q;
+        r -= (int32_t)d;
+    }
+    *rem = (uint32_t)r;
+    return q;
+}
+
+// What the detection loop of one pair reads, as values.
+struct ProbeGeo {
+    const DCollider* ca;
+    const DCollider* cb;
+    F3 pa, pb;
+    Qt fa, fb, ib;  // rotations: A to world, B to world, world to B
+    float vs_a, vs_b, rvs_b, half_b, spec;
+    // A probe's distance in the world, as the reference computes it, and its
+    // distance in B's frame from the already transformed A voxel differ by at
+    // most err; below lo2 (squared distance in B's frame) a probe surely
+    // passes the distance test, above hi2 it surely fails, between them the
+    // reference's expression decides.
+    float err, lo2, hi2;
+    int32_t x0, y0, z0;
+    uint32_t nx, ny;
+    bool wide;  // the region is wider than a feature id's 16 bits an axis
 };
 
-// Entering candidates a warp lists at once before lane 0 applies them.
-constexpr uint32_t kWarpReplay = 16;
+__device__ __forceinline__ void probe_setup(const WorldDev& w, const ColliderSet& cs, const PairInfo& pi, ProbeCtx& c,
+                                            ProbeGeo& g) {
+    const uint32_t ia = pi.ia, ib = pi.ib;
+    const DBody& A = w.body[ia];
+    const DBody& B = w.body[ib];
+    c.ca = &cs.c[pi.ca];
+    c.cb = &cs.c[pi.cb];
+    c.pa = f3of(A.p);
+    c.pb = f3of(B.p);
+    c.qa = qof(A.q);
+    c.qb = qof(B.q);
+    c.qna = qof(w.qn[ia]);
+    c.qnb = qof(w.qn[ib]);
+    c.vs_a = c.ca->vs;
+    c.vs_b = c.cb->vs;
+    g.ca = c.ca;
+    g.cb = c.cb;
+    g.pa = c.pa;
+    g.pb = c.pb;
+    g.fa = rotation_of(c.qna);
+    g.fb = rotation_of(c.qnb);
+    g.ib = rotation_of(qconj(c.qb));
+    g.vs_a = c.vs_a;
+    g.vs_b = c.vs_b;
+    g.rvs_b = 1.0f / c.vs_b;
+    g.half_b = c.vs_b * 0.5f;
+    const float cds = c.vs_a * c.vs_a * 1.0f * 1.0f;
+    g.spec = cds + 0.02f * 0.02f + 2.0f * sqrtf(cds) * 0.02f;
+    // The bound: world to B is a rotation up to sigma = ||ib|^2 - 1| (twice
+    // that, relatively: v + 2w(q x v) + 2 q x (q x v)) and rounding, over
+    // lengths of at most R (B's bounds, two voxels wider); the world side
+    // rounds at the size of B's position.  The factors are several times the
+    // worst case of the operations' roundings (2^-24 each).
+    float R = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        R += (fmaxf(fabsf((float)c.cb->min_bound[k]), fabsf((float)c.cb->max_bound[k])) + 2.0f) * c.vs_b;
+    const Qt q = g.ib;
+    const float sigma = fabsf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w - 1.0f) + 0x1p-20f;
+    g.err = (3.0f * sigma + 0x1p-16f) * R + 0x1p-20f * (fabsf(c.pb.x) + fabsf(c.pb.y) + fabsf(c.pb.z));
+    const float sr = sqrtf(g.spec);
+    const float lo = fmaxf(sr - g.err, 0.0f), hi = sr + g.err;
+    g.lo2 = lo * lo * (1.0f - 0x1p-18f);
+    g.hi2 = hi * hi * (1.0f + 0x1p-18f);
+    if (w.cfg.dump_candidates) {  // every probe through the reference's expression
+        g.lo2 = 0.0f;
+        g.hi2 = __int_as_float(0x7f800000);
+    }
+    g.x0 = pi.rmin[0];
+    g.y0 = pi.rmin[1];
+    g.z0 = pi.rmin[2];
+    g.nx = (uint32_t)(pi.rmax[0] - pi.rmin[0] + 1);
+    g.ny = (uint32_t)(pi.rmax[1] - pi.rmin[1] + 1);
+    g.wide = g.nx > 0x10000u || g.ny > 0x10000u || pi.rmax[2] - pi.rmin[2] >= 0x10000;
+}
+__device__ __forceinline__ I3 region_voxel(const ProbeGeo& g, uint32_t li) {
+    uint32_t x, y;
+    const uint32_t t = div_mod(li, g.nx, &x);
+    const uint32_t z = div_mod(t, g.ny, &y);
+    return I3{g.x0 + (int32_t)x, g.y0 + (int32_t)y, g.z0 + (int32_t)z};
+}
+// A probe's squared distance, in the reference's expression.
+__device__ __forceinline__ float probe_d2(const ProbeGeo& g, I3 b, F3 wa) {
+    const F3 wb = qrotate_unit(g.fb, voxel_to_local(g.vs_b, b.x, b.y, b.z)) + g.pb;
+    return lensq3(wb - wa);
+}
+
+// Candidates one part of a cut pair hands to the merge; one with more is
+// probed again there.
+constexpr uint32_t kPartLog = 64;
+// Penetrations a lane keeps at hand for its voxel's candidates (later ones
+// are computed again when their turn comes).
+constexpr uint32_t kLanePens = 8;
 
 // Per-warp shared state of phase_probe.
 struct WarpManifold {
     ContactRec c[4];              // the pair's contacts, built when it ends
-    CandRec k[4];                 // the manifold during detection
-    CandRec list[kWarpReplay];
-    float pens[4];
-    uint32_t n;
-    uint32_t pad[3];
+    uint2 log[kPartLog];          // (penetration, A voxel | probe << 27) of a part's entering candidates
+    float pens[kLanePens][32];
+    unsigned long long fid[4];    // feature ids of the manifold's slots (regions wider than their 16 bits)
 };
 
-// ContactManifold.addContact (narrow_phase.zig:451-481) on candidate
-// records, executed by one lane: a contact with the same feature id is
-// replaced (keeping its impulses, all zero here), else appended while fewer
-// than four, else the first contact of least penetration below the new one
-// is replaced.
-__device__ __forceinline__ void add_cand(WarpManifold& m, const CandRec& r) {
-    for (uint32_t i = 0; i < m.n; ++i) {
-        if (m.k[i].fid == r.fid) {
-            m.k[i] = r;
-            return;
-        }
+// The manifold during detection, the same in every lane of the warp: per
+// slot the penetration and where the candidate came from (A voxel li of the
+// region in loop order, probe k).  A contact is built only if it is still
+// there when the pair ends: its fields are a function of (li, k), and the
+// impulses of every contact added during detection are zero.
+struct Manifold4 {
+    float p[4];
+    uint32_t li[4], k[4];
+    uint32_t n;
+    float least;  // a candidate enters only above this
+};
+__device__ __forceinline__ void manifold_clear(Manifold4& m) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m.p[i] = 0.0f;
+        m.li[i] = m.k[i] = 0u;
     }
+    m.n = 0u;
+    m.least = -__int_as_float(0x7f800000);
+}
+// ContactManifold.addContact (narrow_phase.zig:451-481) for a candidate whose
+// feature id is new: appended while fewer than four, else the first contact
+// of least penetration below the new one is replaced.  Returns the slot.
+__device__ __forceinline__ uint32_t manifold_add(Manifold4& m, float pen, uint32_t li, uint32_t k) {
+    uint32_t at = 4u;
     if (m.n < 4u) {
-        m.k[m.n] = r;
+        at = m.n;
         m.n += 1u;
-        return;
+    } else {
+        float mp = pen;
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i)
+            if (m.p[i] < mp) {
+                mp = m.p[i];
+                at = i;
+            }
     }
-    float mp = r.pen;
-    int mi = -1;
-    for (uint32_t i = 0; i < m.n; ++i) {
-        if (m.k[i].pen < mp) {
-            mp = m.k[i].pen;
-            mi = (int)i;
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; ++i)
+        if (i == at) {
+            m.p[i] = pen;
+            m.li[i] = li;
+            m.k[i] = k;
         }
-    }
-    if (mi >= 0) m.k[mi] = r;
+    if (m.n == 4u) m.least = fminf(fminf(m.p[0], m.p[1]), fminf(m.p[2], m.p[3]));
+    return at;
 }
-// The manifold's penetration multiset (at most four finite values, so every
-// insert lands), by one lane, into m.pens.
-__device__ __forceinline__ void cand_pens(WarpManifold& m) {
-    Top4 s = top4_empty();
-    for (uint32_t i = 0; i < m.n; ++i) top4_insert(s, m.k[i].pen);
-    m.pens[0] = s.v[0];
-    m.pens[1] = s.v[1];
-    m.pens[2] = s.v[2];
-    m.pens[3] = s.v[3];
-}
-// generateContact for candidate r of the pair probed with c over the region
+// generateContact for candidate (li, k) of the pair probed with c over the region
 // starting at rmin, nx x ny voxels per z layer: the same lookups and
 // transforms as the detection loop.
 __device__ void build_contact(const ColliderSet& cs, const ProbeCtx& c, const int32_t* rmin, uint32_t nx,
-                              uint32_t ny, const CandRec& r, ContactRec* out) {
-    const int32_t x = rmin[0] + (int32_t)(r.li % nx), y = rmin[1] + (int32_t)((r.li / nx) % ny),
-                  z = rmin[2] + (int32_t)(r.li / (nx * ny));
+                              uint32_t ny, uint32_t li, uint32_t k, ContactRec* out) {
+    const int32_t x = rmin[0] + (int32_t)(li % nx), y = rmin[1] + (int32_t)((li / nx) % ny),
+                  z = rmin[2] + (int32_t)(li / (nx * ny));
     const uint32_t va = voxel_at(cs, *c.ca, x, y, z);
     const F3 wa = transform_point_n(c.pa, c.qna, voxel_to_local(c.vs_a, x, y, z));
     const I3 cbv = local_to_voxel(c.vs_b, inverse_transform_point(c.pb, c.qb, wa));
-    const I3 o = probe_offset(r.k);
+    const I3 o = probe_offset(k);
     const I3 ibv{cbv.x + o.x, cbv.y + o.y, cbv.z + o.z};
     const uint32_t vb = voxel_at(cs, *c.cb, ibv.x, ibv.y, ibv.z);
     const F3 wb = transform_point_n(c.pb, c.qnb, voxel_to_local(c.vs_b, ibv.x, ibv.y, ibv.z));
     generate_contact(c, va, I3{x, y, z}, wa, vb, ibv, wb, out);
 }
 
-// One warp runs detectVoxelCollisions for pair p.  The inclusive z, y, x loop
-// over the overlap region is cut into groups of 32 consecutive voxels, one per
-// lane; each lane runs the 27 probes of its voxel.  The manifold reduction is
-// order dependent, so it is reproduced exactly: a candidate can only enter the
-// 4-slot manifold if its penetration beats the 4th largest penetration of all
-// candidates before it (the multiset of penetrations held by the manifold is
-// always the top four of the prefix).  A warp scan of top-4 multisets gives
-// every lane that prefix, seeded with the manifold's state; only the entering
-// candidates are replayed, in order, through addContact.
-__device__ void probe_pair(const WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p, WarpManifold& sm) {
-    const uint32_t lane = threadIdx.x & 31;
-    PairInfo& pi = w.pinfo[p];
-    const uint32_t ia = pi.ia, ib = pi.ib;
-    const DBody& A = w.body[ia];
-    const DBody& B = w.body[ib];
-    const DBodyProp& prA = w.prop[ia];
-    const DBodyProp& prB = w.prop[ib];
-    ProbeCtx c;
-    c.ca = &cs.c[prA.collider];
-    c.cb = &cs.c[prB.collider];
-    c.pa = f3of(A.p);
-    c.pb = f3of(B.p);
-    c.qa = qof(A.q);
-    c.qb = qof(B.q);
-    c.qna = qof(w.qn[ia]);
-    c.qnb = qof(w.qn[ib]);
-    c.vs_a = c.ca->vs;
-    c.vs_b = c.cb->vs;
-    {
-        const float cds = c.vs_a * c.vs_a * 1.0f * 1.0f;
-        c.spec = cds + 0.02f * 0.02f + 2.0f * sqrtf(cds) * 0.02f;
+__device__ __noinline__ void dump_candidate(uint32_t* ctr, WorldDev::Cand* dump, uint32_t cap, uint32_t p, I3 a, I3 b,
+                                            bool pass, float d2) {
+    const uint32_t slot = atomicAdd(&ctr[C_DUMP_N], 1u);
+    if (slot >= cap) return;
+    WorldDev::Cand& r = dump[slot];
+    r.pair_index = p;
+    r.a[0] = a.x; r.a[1] = a.y; r.a[2] = a.z;
+    r.b[0] = b.x; r.b[1] = b.y; r.b[2] = b.z;
+    r.passed = pass ? 1u : 0u;
+    r.dist_sq = d2;
+}
+
+// The feature id of candidate (li, k).
+__device__ __noinline__ unsigned long long candidate_fid(const ProbeGeo g, uint32_t li, uint32_t k) {
+    const I3 at = region_voxel(g, li);
+    const F3 wa = qrotate_unit(g.fa, voxel_to_local(g.vs_a, at.x, at.y, at.z)) + g.pa;
+    const F3 pl = qrotate_unit(g.ib, wa - g.pb);
+    const I3 o = probe_offset(k);
+    return feature_id(at, I3{floor_div(pl.x, g.vs_b, g.rvs_b) + o.x, floor_div(pl.y, g.vs_b, g.rvs_b) + o.y,
+                             floor_div(pl.z, g.vs_b, g.rvs_b) + o.z});
+}
+// addContact for a candidate, by the whole warp.  Two candidates of a pair
+// share a feature id only in a region wider than its 16 bits an axis (one A
+// voxel's B voxels lie within three of each other): then the old contact is
+// replaced in its slot.
+__device__ __forceinline__ void candidate_add(const ProbeGeo& g, WarpManifold& sm, Manifold4& m, float pen, uint32_t li,
+                                              uint32_t k) {
+    if (!g.wide) {
+        manifold_add(m, pen, li, k);
+        return;
     }
-    const DCollider& ca = *c.ca;
-    const DCollider& cb = *c.cb;
-    const int32_t nx = pi.rmax[0] - pi.rmin[0] + 1, ny = pi.rmax[1] - pi.rmin[1] + 1,
-                  nz = pi.rmax[2] - pi.rmin[2] + 1;
-    const unsigned long long V = (unsigned long long)nx * (unsigned long long)ny * (unsigned long long)nz;
-    if (lane == 0) sm.n = 0u;
-    Top4 state = top4_empty();
-    uint32_t checked = 0, ncand = 0;
-    if (w.cfg.count_bricks) {
-        // traffic accounting: A bricks in the region, B bricks in B's region
-        uint32_t nb = warp_count_bricks(cs, ca, I3{pi.rmin[0], pi.rmin[1], pi.rmin[2]},
-                                        I3{pi.rmax[0], pi.rmax[1], pi.rmax[2]});
-        I3 blo, bhi;
-        if (overlap_region(cb, c.pb, c.qb, ca, c.pa, c.qa, &blo, &bhi)) nb += warp_count_bricks(cs, cb, blo, bhi);
-        if (lane == 0) atomicAdd(&w.ctr[C_BRICKS], nb);
+    const unsigned long long fid = candidate_fid(g, li, k);
+    for (uint32_t i = 0; i < m.n; ++i)
+        if (sm.fid[i] == fid) {
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; ++j)
+                if (j == i) {
+                    m.p[j] = pen;
+                    m.li[j] = li;
+                    m.k[j] = k;
+                }
+            if (m.n == 4u) m.least = fminf(fminf(m.p[0], m.p[1]), fminf(m.p[2], m.p[3]));
+            return;
+        }
+    const uint32_t at = manifold_add(m, pen, li, k);
+    __syncwarp();
+    if (at < 4u && (threadIdx.x & 31u) == 0u) sm.fid[at] = fid;
+    __syncwarp();
+}
+
+// Voxels [first, end) of the overlap region's inclusive z, y, x loop by one
+// warp, into its manifold.
+//
+// Groups of 32 consecutive voxels, one per lane; each lane runs the 27 probes
+// of its voxel.  The manifold reduction is order dependent, so it is
+// reproduced exactly: a candidate enters the 4-slot manifold only if its
+// penetration beats the least one held.  The lanes keep the candidates that
+// beat the least as it stood before the group; then, one after another in
+// canonical order (lane = voxel order, then probe order), the first lane
+// whose next candidate still beats it hands that candidate to the warp, which
+// adds it in registers.  The first kPartLog candidates added are also kept in
+// sm.log; logged: how many were added.
+//
+// The loop is bound by instructions and by the latency of its two loads (the
+// A voxel, B's table entry).  So the distance test runs in B's frame, where
+// the A voxel already is (five operations a probe against about sixty for the
+// world-space expression), and the world-space expression is left to the
+// probes near the threshold and to those that could enter the manifold; and
+// the groups are pipelined: while one is probed, the next one's table entries
+// and the A voxels of the one after are on their way.
+__device__ __forceinline__ void probe_range(const WorldDev& w, const ColliderSet& cs, const ProbeGeo& geo, uint32_t p,
+                                         unsigned long long first, unsigned long long end, WarpManifold& sm,
+                                         Manifold4& m, uint32_t& checked, uint32_t& ncand, uint32_t& logged) {
+    const uint32_t lane = threadIdx.x & 31;
+    // Everything the loop reads, in registers: the stores below would make
+    // the compiler read the structs again for every group.
+    const F3 pa = geo.pa, pb = geo.pb;
+    const Qt fa = geo.fa, ib = geo.ib;
+    const float vs_a = geo.vs_a, vs_b = geo.vs_b, rvs_b = geo.rvs_b, half_a = vs_a * 0.5f, half_b = vs_b * 0.5f;
+    const float err = geo.err, lo2 = geo.lo2, hi2 = geo.hi2;
+    const uint32_t nx = geo.nx, ny = geo.ny;
+    const DCollider& ca = *geo.ca;
+    const DCollider& cb = *geo.cb;
+    // A's bricks: the region lies in A's bounds, which the brick grid covers
+    // with a brick to spare, so a lookup needs no bounds test
+    const int32_t bdx = ca.bdim[0], bdxy = bdx * ca.bdim[1];
+    const int32_t* agrid = cs.grid + ca.grid_off - (ca.bmin[0] + bdx * ca.bmin[1] + bdxy * ca.bmin[2]);
+    const uint8_t* avox = cs.vox + (size_t)ca.brick_off * 512u;
+    const bool table = cb.nb_off != kNoTable;
+    const uint4* btab = cs.nb + cb.nb_off;
+    const uint32_t bx1 = (uint32_t)cb.min_bound[0] - 1u, by1 = (uint32_t)cb.min_bound[1] - 1u,
+                   bz1 = (uint32_t)cb.min_bound[2] - 1u;
+    const uint32_t ex = (uint32_t)cb.max_bound[0] - bx1 + 1u, ey = (uint32_t)cb.max_bound[1] - by1 + 1u,
+                   ez = (uint32_t)cb.max_bound[2] - bz1 + 1u;
+    checked = ncand = logged = 0u;
+    // squared distance in B's frame above which a candidate cannot enter
+    auto enter_limit = [&]() {
+        const float lim = (vs_a - m.least) * (1.0f + 0x1p-20f) + vs_a * 0x1p-20f + err;
+        return lim * lim * (1.0f + 0x1p-18f);
+    };
+    float tpen2 = enter_limit();
+    // the lane's voxel of the next group to fetch: 32 further each time
+    I3 nat;
+    {
+        uint32_t x, y;
+        const uint32_t t = div_mod((uint32_t)first + lane, nx, &x), z = div_mod(t, ny, &y);
+        nat = I3{geo.x0 + (int32_t)x, geo.y0 + (int32_t)y, geo.z0 + (int32_t)z};
+    }
+    uint32_t ux, uy;
+    const uint32_t ut = div_mod(32u, nx, &ux);
+    const int32_t sz = (int32_t)div_mod(ut, ny, &uy), sx = (int32_t)ux, sy = (int32_t)uy;
+    const int32_t xe = geo.x0 + (int32_t)nx, ye = geo.y0 + (int32_t)ny;
+    // A voxel of a lane, then (where it is not empty) its place in B's frame
+    // and the masks around it
+    struct Vox {
+        I3 at;
+        uint32_t v;
+    };
+    struct Probe {
+        I3 at, cbv;
+        F3 wa, pl;
+        uint32_t ta;
+        uint4 nm;
+    };
+    auto fetch = [&](unsigned long long l) {
+        Vox v{nat, kEmpty};
+        if (l < end) {
+            const int32_t slot = __ldg(agrid + (nat.x >> 3) + bdx * (nat.y >> 3) + bdxy * (nat.z >> 3));
+            if (slot >= 0)
+                v.v = __ldg(avox + (size_t)(uint32_t)slot * 512u +
+                            (uint32_t)((nat.x & 7) + 8 * (nat.y & 7) + 64 * (nat.z & 7)));
+        }
+        nat.x += sx;
+        nat.y += sy;
+        nat.z += sz;
+        if (nat.x >= xe) {
+            nat.x -= (int32_t)nx;
+            ++nat.y;
+        }
+        if (nat.y >= ye) {
+            nat.y -= (int32_t)ny;
+            ++nat.z;
+        }
+        return v;
+    };
+    auto place = [&](const Vox& v) {
+        Probe r;
+        r.at = v.at;
+        r.ta = vtype(v.v);
+        r.nm = make_uint4(0u, 0u, 0u, 0u);
+        r.cbv = I3{0, 0, 0};
+        r.wa = r.pl = F3{0.f, 0.f, 0.f};
+        if (r.ta != kEmpty) {
+            r.wa = qrotate_unit(fa, F3{(float)r.at.x * vs_a + half_a, (float)r.at.y * vs_a + half_a,
+                                       (float)r.at.z * vs_a + half_a}) + pa;
+            r.pl = qrotate_unit(ib, r.wa - pb);
+            r.cbv = I3{floor_div(r.pl.x, vs_b, rvs_b), floor_div(r.pl.y, vs_b, rvs_b),
+                       floor_div(r.pl.z, vs_b, rvs_b)};
+            if (table) {
+                // a centre outside [min_bound - 1, max_bound] has no neighbour in bounds
+                const uint32_t tx = (uint32_t)r.cbv.x - bx1, ty = (uint32_t)r.cbv.y - by1, tz = (uint32_t)r.cbv.z - bz1;
+                if (tx < ex && ty < ey && tz < ez) r.nm = __ldg(btab + (tx + ex * (ty + ey * tz)));
+            } else {
+                r.nm = probe_masks_lookup(cs, cb, r.cbv);
+            }
+        }
+        return r;
+    };
+    Vox vn = fetch(first + lane);
+    Probe pn = place(vn);
+    vn = fetch(first + 32ull + lane);
+    for (unsigned long long base = first; base < end; base += 32ull) {
+        const Probe c = pn;
+        pn = place(vn);
+        vn = fetch(base + 64ull + lane);
+        checked += (uint32_t)__popc(c.nm.x);
+        // the probes passing type_filter(ta, tb), and those of them whose
+        // penetration is at least the voxel size
+        const uint32_t ps = c.ta == kCorner ? c.nm.x : (c.ta == kEdge ? c.nm.z : c.nm.y);
+        const uint32_t in = c.ta == kInside ? c.nm.x : c.nm.w;
+        if (__ballot_sync(0xffffffffu, ps != 0u) == 0u) continue;
+        uint32_t mask = 0u, keep = 0u, kept = 0u;
+        const I3 at = c.at, cbv = c.cbv;
+        const F3 wa = c.wa;
+        // squared distances along the axes to the three voxels of each
+        float X[3], Y[3], Z[3];
+        {
+            const float dx = c.pl.x - ((float)cbv.x * vs_b + half_b), dy = c.pl.y - ((float)cbv.y * vs_b + half_b),
+                        dz = c.pl.z - ((float)cbv.z * vs_b + half_b);
+            X[0] = (dx + vs_b) * (dx + vs_b); X[1] = dx * dx; X[2] = (dx - vs_b) * (dx - vs_b);
+            Y[0] = (dy + vs_b) * (dy + vs_b); Y[1] = dy * dy; Y[2] = (dy - vs_b) * (dy - vs_b);
+            Z[0] = (dz + vs_b) * (dz + vs_b); Z[1] = dz * dz; Z[2] = (dz - vs_b) * (dz - vs_b);
+        }
+        // the probes that surely fail the distance test leave at once, all 27
+        // side by side (a corner voxel has a dozen probes, of which few are
+        // near enough; one by one, the warp would wait for its fullest lane)
+        uint32_t nearby = 0u;
+#pragma unroll
+        for (int k = 0; k < 27; ++k)
+            if (!(X[k % 3] + Y[(k / 3) % 3] + Z[k / 9] > hi2)) nearby |= 1u << k;
+        const bool deep = vs_a > m.least;
+        for (uint32_t mm = ps & nearby; mm; mm &= mm - 1u) {
+            const uint32_t k = __ffs(mm) - 1, bit = mm & (0u - mm);
+            // bits of each axis' -1 and +1 neighbours
+            const float dx2 = (bit & 0x1249249u) ? X[0] : ((bit & 0x4924924u) ? X[2] : X[1]);
+            const float dy2 = (bit & 0x01C0E07u) ? Y[0] : ((bit & 0x70381C0u) ? Y[2] : Y[1]);
+            const float dz2 = k < 9u ? Z[0] : (k >= 18u ? Z[2] : Z[1]);
+            const float da = dx2 + dy2 + dz2;
+            const bool ins = ((in >> k) & 1u) != 0u;
+            const bool may = ins ? deep : !(da > tpen2);
+            float d2 = 0.0f;
+            bool pass = da < lo2;
+            if (!pass || may) {
+                const I3 o = probe_offset(k);
+                const I3 b{cbv.x + o.x, cbv.y + o.y, cbv.z + o.z};
+                d2 = probe_d2(geo, b, wa);
+                pass = d2 < geo.spec;
+                if (w.cfg.dump_candidates) dump_candidate(w.ctr, w.dump, w.dump_cap, p, at, b, pass, d2);
+            }
+            if (pass) mask |= bit;
+            if (pass && may) {
+                const float pen = cand_pen(vs_a, ins ? (uint32_t)kInside : (uint32_t)kCorner, kCorner, d2);
+                if (pen > m.least) {
+                    keep |= bit;
+                    if (kept < kLanePens) sm.pens[kept][lane] = pen;
+                    ++kept;
+                }
+            }
+        }
+        ncand += (uint32_t)__popc(mask);
+        if (__ballot_sync(0xffffffffu, keep != 0u) == 0u) continue;
+        // the lane's next candidate (its penetration; -inf: none left)
+        uint32_t j = 0;
+        const float none = -__int_as_float(0x7f800000);
+        auto next_pen = [&]() {
+            if (keep == 0u) return none;
+            if (j < kLanePens) return sm.pens[j][lane];
+            const uint32_t k = __ffs(keep) - 1;
+            const I3 o = probe_offset(k);
+            return cand_pen(vs_a, ((in >> k) & 1u) ? (uint32_t)kInside : (uint32_t)kCorner, kCorner,
+                            probe_d2(geo, I3{cbv.x + o.x, cbv.y + o.y, cbv.z + o.z}, wa));
+        };
+        float pen = next_pen();
+        for (;;) {
+            while (keep && !(pen > m.least)) {
+                keep &= keep - 1u;
+                ++j;
+                pen = next_pen();
+            }
+            const uint32_t who = __ballot_sync(0xffffffffu, keep != 0u);
+            if (who == 0u) break;
+            const uint32_t src = __ffs(who) - 1;
+            const float cpen = __shfl_sync(0xffffffffu, pen, src);
+            const uint32_t ck = (uint32_t)(__ffs(__shfl_sync(0xffffffffu, keep, src)) - 1);
+            const uint32_t cli = (uint32_t)base + src;
+            candidate_add(geo, sm, m, cpen, cli, ck);
+            if (lane == src) {
+                if (logged < kPartLog) sm.log[logged] = make_uint2(__float_as_uint(cpen), cli | (ck << 27));
+                keep &= keep - 1u;
+                ++j;
+                pen = next_pen();
+            }
+            ++logged;
+        }
+        tpen2 = enter_limit();
     }
     __syncwarp();
-    for (unsigned long long base = 0; base < V; base += 32ull) {
-        const unsigned long long l = base + lane;
-        uint32_t va = 0u;
-        int32_t x = 0, y = 0, z = 0;
-        if (l < V) {
-            const uint32_t li = (uint32_t)l;
-            x = pi.rmin[0] + (int32_t)(li % (uint32_t)nx);
-            y = pi.rmin[1] + (int32_t)((li / (uint32_t)nx) % (uint32_t)ny);
-            z = pi.rmin[2] + (int32_t)(li / ((uint32_t)nx * (uint32_t)ny));
-            va = voxel_at(cs, ca, x, y, z);
-        }
-        uint32_t mask = 0u;
-        Top4 t = top4_empty();
-        F3 wa{0.f, 0.f, 0.f};
-        I3 cbv{0, 0, 0};
-        const uint32_t ta = vtype(va);
-        if (ta != kEmpty) {
-            wa = transform_point_n(c.pa, c.qna, voxel_to_local(c.vs_a, x, y, z));
-            cbv = local_to_voxel(c.vs_b, inverse_transform_point(c.pb, c.qb, wa));
-            probe_neighbourhood(w, cs, c, p, ta, x, y, z, wa, cbv, &mask, &t, &checked);
-        }
-        if (__ballot_sync(0xffffffffu, mask != 0u) == 0u) continue;
-        ncand += __popc(mask);
-        // a candidate enters only above the running 4th penetration, which is
-        // at least the manifold's: when no lane's best beats that, none does
-        if (__ballot_sync(0xffffffffu, t.v[0] > state.v[3]) == 0u) continue;
-        // exclusive warp scan of the lanes' top-4 multisets
-        Top4 inc = t;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const Top4 o = top4_shfl_up(inc, d);
-            if ((int)lane >= d) inc = top4_merge(o, inc);
-        }
-        Top4 ex = top4_shfl_up(inc, 1);
-        if (lane == 0) ex = top4_empty();
-        Top4 run = top4_merge(state, ex);
-        // candidates of this lane that enter the manifold
-        uint32_t enter = 0u;
-        for (uint32_t mm = mask; mm; mm &= mm - 1u) {
-            const uint32_t k = __ffs(mm) - 1;
-            const I3 o = probe_offset(k);
-            const int32_t bx = cbv.x + o.x, by = cbv.y + o.y, bz = cbv.z + o.z;
-            const uint32_t vb = voxel_at(cs, cb, bx, by, bz);
-            const F3 wb = transform_point_n(c.pb, c.qnb, voxel_to_local(c.vs_b, bx, by, bz));
-            const float d2 = lensq3(wb - wa);
-            const float pen = cand_pen(c.vs_a, ta, vtype(vb), d2);
-            if (pen > run.v[3]) {
-                enter |= 1u << k;
-                top4_insert(run, pen);
-            }
-        }
-        // entering candidates in canonical order (lane = voxel order, then
-        // probe order): the lanes list them at once, kWarpReplay at a time;
-        // lane 0 applies them in list order
-        const uint32_t ne = (uint32_t)__popc(enter);
-        const uint32_t ninc = warp_incl_scan(ne);
-        const uint32_t total = __shfl_sync(0xffffffffu, ninc, 31);
-        for (uint32_t lo = 0; lo < total; lo += kWarpReplay) {
-            uint32_t e = ninc - ne;
-            for (uint32_t mm = enter; mm; mm &= mm - 1u, ++e) {
-                if (e < lo || e >= lo + kWarpReplay) continue;
-                const uint32_t k = __ffs(mm) - 1;
-                const I3 o = probe_offset(k);
-                const I3 ibv{cbv.x + o.x, cbv.y + o.y, cbv.z + o.z};
-                const uint32_t vb = voxel_at(cs, cb, ibv.x, ibv.y, ibv.z);
-                const F3 wb = transform_point_n(c.pb, c.qnb, voxel_to_local(c.vs_b, ibv.x, ibv.y, ibv.z));
-                CandRec& r = sm.list[e - lo];
-                r.fid = feature_id(I3{x, y, z}, ibv);
-                r.pen = cand_pen(c.vs_a, ta, vtype(vb), lensq3(wb - wa));
-                r.li = (uint32_t)l;
-                r.k = k;
-                r._pad = 0u;
-            }
-            __syncwarp();
-            if (lane == 0) {
-                const uint32_t cnt = min(kWarpReplay, total - lo);
-                for (uint32_t i = 0; i < cnt; ++i) add_cand(sm, sm.list[i]);
-            }
-            __syncwarp();
-        }
-        // manifold penetration multiset -> state
-        if (lane == 0) cand_pens(sm);
-        __syncwarp();
-        state.v[0] = sm.pens[0];
-        state.v[1] = sm.pens[1];
-        state.v[2] = sm.pens[2];
-        state.v[3] = sm.pens[3];
-    }
-    checked = warp_sum(checked);
-    ncand = warp_sum(ncand);
+}
+
+// The pair's manifold record from the warp's manifold.
+__device__ __forceinline__ void probe_store(const WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p, const PairInfo& pi,
+                            const ProbeCtx& c, const ProbeGeo& g, const Manifold4& m, WarpManifold& sm) {
+    const uint32_t lane = threadIdx.x & 31;
     // the contacts left in the manifold
-    if (lane < sm.n) build_contact(cs, c, pi.rmin, (uint32_t)nx, (uint32_t)ny, sm.k[lane], &sm.c[lane]);
+    uint32_t li = m.li[0], k = m.k[0];
+#pragma unroll
+    for (uint32_t i = 1; i < 4u; ++i)
+        if (lane == i) {
+            li = m.li[i];
+            k = m.k[i];
+        }
+    if (lane < m.n) build_contact(cs, c, pi.rmin, g.nx, g.ny, li, k, &sm.c[lane]);
     __syncwarp();
     ManifoldRec& out = w.man[cur][p];
     if (lane == 0) {
-        pi.voxels_checked = checked;
-        pi.candidates = ncand;
+        const DBodyProp& prA = w.prop[pi.ia];
+        const DBodyProp& prB = w.prop[pi.ib];
         out.a = prA.id;
         out.b = prB.id;
-        out.n = sm.n;
+        out.n = m.n;
         out.friction = sqrtf(prA.friction * prB.friction);
         out.restitution = fmaxf(prA.restitution, prB.restitution);
         out._pad = 0u;
     }
-    __syncwarp();
     // copy the contacts (one lane per 4-byte word)
-    const uint32_t words = sm.n * (uint32_t)(sizeof(ContactRec) / 4);
+    const uint32_t words = m.n * (uint32_t)(sizeof(ContactRec) / 4);
     const uint32_t* src = reinterpret_cast<const uint32_t*>(sm.c);
     uint32_t* dst = reinterpret_cast<uint32_t*>(out.c);
     for (uint32_t i = lane; i < words; i += 32u) dst[i] = src[i];
     __syncwarp();
 }
+// Traffic accounting: A bricks in the region, B bricks in B's region.
+__device__ __noinline__ void probe_count_bricks(uint32_t* ctr, const ColliderSet& cs, const PairInfo& pi,
+                                                const ProbeCtx c) {
+    uint32_t nb = warp_count_bricks(cs, *c.ca, I3{pi.rmin[0], pi.rmin[1], pi.rmin[2]},
+                                    I3{pi.rmax[0], pi.rmax[1], pi.rmax[2]});
+    I3 blo, bhi;
+    if (overlap_region(*c.cb, c.pb, c.qb, *c.ca, c.pa, c.qa, &blo, &bhi)) nb += warp_count_bricks(cs, *c.cb, blo, bhi);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&ctr[C_BRICKS], nb);
+}
+__device__ __forceinline__ unsigned long long region_volume(const int32_t* rmin, const int32_t* rmax) {
+    return (unsigned long long)(rmax[0] - rmin[0] + 1) * (unsigned long long)(rmax[1] - rmin[1] + 1) *
+           (unsigned long long)(rmax[2] - rmin[2] + 1);
+}
 
-// The same narrow phase for one pair with a large overlap region, run by the
-// whole CTA: each pass covers blockDim.x consecutive voxels of the inclusive
-// z, y, x loop (one per thread).  The manifold's order-dependent reduction is
-// reproduced as in probe_pair, with a CTA-wide exclusive scan of the
-// threads' top-4 multisets in voxel order; the threads build the contacts
-// that enter, and one thread adds them to the manifold in that order.
-constexpr uint32_t kBlockReplay = 64;
-__device__ void probe_pair_block(const WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p, WarpManifold& sm) {
-    __shared__ Top4 s_top[32];
-    __shared__ CandRec s_rec[kBlockReplay];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = blockDim.x >> 5;
+// detectVoxelCollisions for pair p by one warp, or for one part of it where
+// its region is cut (part < ~0u, PF_HEAVY).
+// A part takes its voxels as probe_range does, from an empty manifold.  A
+// candidate that enters the pair's manifold beats the least penetration held
+// after all candidates before it, so also after those before it in its part:
+// the part's entering candidates, logged in order, contain the pair's.  The
+// warp that finishes a pair's last part applies the logs in part order, taking
+// the candidates that beat the manifold as it stands; a part whose log did not
+// fit is probed again there.  No warp waits for another, and the parts of all
+// large pairs share the machine evenly (a CTA a pair, with a barrier after
+// each 512 voxels, spent nine tenths of its time in those barriers).
+__device__ __forceinline__ void probe_item(const WorldDev& w, const ColliderSet& cs, uint32_t cur, uint32_t p,
+                                           uint32_t part, uint32_t item, WarpManifold& sm) {
+    const uint32_t lane = threadIdx.x & 31;
     PairInfo& pi = w.pinfo[p];
-    const uint32_t ia = pi.ia, ib = pi.ib;
-    const DBody& A = w.body[ia];
-    const DBody& B = w.body[ib];
-    const DBodyProp& prA = w.prop[ia];
-    const DBodyProp& prB = w.prop[ib];
+    const bool cut = part != 0xFFFFFFFFu;
+    const uint32_t parts = cut ? pi.parts : 1u;
     ProbeCtx c;
-    c.ca = &cs.c[prA.collider];
-    c.cb = &cs.c[prB.collider];
-    c.pa = f3of(A.p);
-    c.pb = f3of(B.p);
-    c.qa = qof(A.q);
-    c.qb = qof(B.q);
-    c.qna = qof(w.qn[ia]);
-    c.qnb = qof(w.qn[ib]);
-    c.vs_a = c.ca->vs;
-    c.vs_b = c.cb->vs;
-    {
-        const float cds = c.vs_a * c.vs_a * 1.0f * 1.0f;
-        c.spec = cds + 0.02f * 0.02f + 2.0f * sqrtf(cds) * 0.02f;
-    }
-    const DCollider& ca = *c.ca;
-    const DCollider& cb = *c.cb;
-    const int32_t nx = pi.rmax[0] - pi.rmin[0] + 1, ny = pi.rmax[1] - pi.rmin[1] + 1,
-                  nz = pi.rmax[2] - pi.rmin[2] + 1;
-    const unsigned long long V = (unsigned long long)nx * (unsigned long long)ny * (unsigned long long)nz;
-    if (tid == 0) sm.n = 0u;
-    if (wid == 0 && w.cfg.count_bricks) {
-        // traffic accounting: A bricks in the region, B bricks in B's region
-        uint32_t nb = warp_count_bricks(cs, ca, I3{pi.rmin[0], pi.rmin[1], pi.rmin[2]},
-                                        I3{pi.rmax[0], pi.rmax[1], pi.rmax[2]});
-        I3 blo, bhi;
-        if (overlap_region(cb, c.pb, c.qb, ca, c.pa, c.qa, &blo, &bhi)) nb += warp_count_bricks(cs, cb, blo, bhi);
-        if (lane == 0) atomicAdd(&w.ctr[C_BRICKS], nb);
-    }
-    __syncthreads();
-    Top4 state = top4_empty();
-    uint32_t checked = 0, ncand = 0;
-    for (unsigned long long base = 0; base < V; base += blockDim.x) {
-        const unsigned long long l = base + tid;
-        uint32_t va = 0u;
-        int32_t x = 0, y = 0, z = 0;
-        if (l < V) {
-            const uint32_t li = (uint32_t)l;
-            x = pi.rmin[0] + (int32_t)(li % (uint32_t)nx);
-            y = pi.rmin[1] + (int32_t)((li / (uint32_t)nx) % (uint32_t)ny);
-            z = pi.rmin[2] + (int32_t)(li / ((uint32_t)nx * (uint32_t)ny));
-            va = voxel_at(cs, ca, x, y, z);
-        }
-        uint32_t mask = 0u;
-        Top4 t = top4_empty();
-        F3 wa{0.f, 0.f, 0.f};
-        I3 cbv{0, 0, 0};
-        const uint32_t ta = vtype(va);
-        if (ta != kEmpty) {
-            wa = transform_point_n(c.pa, c.qna, voxel_to_local(c.vs_a, x, y, z));
-            cbv = local_to_voxel(c.vs_b, inverse_transform_point(c.pb, c.qb, wa));
-            probe_neighbourhood(w, cs, c, p, ta, x, y, z, wa, cbv, &mask, &t, &checked);
-        }
-        if (!__syncthreads_or(mask != 0u)) continue;
-        ncand += __popc(mask);
-        // a candidate enters only above the running 4th penetration, which is
-        // at least the manifold's: when no thread's best beats that, none does
-        if (!__syncthreads_or(t.v[0] > state.v[3])) continue;
-        // CTA-wide exclusive scan of the threads' top-4 multisets
-        Top4 inc = t;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const Top4 o = top4_shfl_up(inc, d);
-            if ((int)lane >= d) inc = top4_merge(o, inc);
-        }
-        if (lane == 31) s_top[wid] = inc;
-        __syncthreads();
-        if (wid == 0) {
-            Top4 wi = lane < nwarps ? s_top[lane] : top4_empty();
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const Top4 o = top4_shfl_up(wi, d);
-                if ((int)lane >= d) wi = top4_merge(o, wi);
+    ProbeGeo g;
+    probe_setup(w, cs, pi, c, g);
+    const unsigned long long V = region_volume(pi.rmin, pi.rmax);
+    const unsigned long long len = cut ? ((V + parts - 1u) / parts + 31ull) & ~31ull : V;
+    if (w.cfg.count_bricks && (!cut || part == 0u)) probe_count_bricks(w.ctr, cs, pi, c);
+    Manifold4 m;
+    manifold_clear(m);
+    bool merging = false;
+    uint32_t q = cut ? part : 0u;  // the part being probed
+    for (;;) {
+        uint32_t checked, ncand, logged;
+        const unsigned long long lo = min(V, len * q), hi = min(V, lo + len);
+        probe_range(w, cs, g, p, lo, hi, sm, m, checked, ncand, logged);
+        if (merging) {
+            ++q;
+        } else {
+            checked = warp_sum(checked);
+            ncand = warp_sum(ncand);
+            if (!cut) {
+                if (lane == 0) {
+                    pi.voxels_checked = checked;
+                    pi.candidates = ncand;
+                }
+                break;
             }
-            Top4 we = top4_shfl_up(wi, 1);
-            if (lane == 0) we = top4_empty();
-            if (lane < nwarps) s_top[lane] = we;
+            // the log to memory
+            uint32_t off = 0;
+            if (lane == 0) {
+                off = logged && logged <= kPartLog ? atomicAdd(&w.ctr[C_NLOG], logged) : 0u;
+                atomicAdd(&pi.voxels_checked, checked);
+                atomicAdd(&pi.candidates, ncand);
+            }
+            off = __shfl_sync(0xffffffffu, off, 0);
+            const bool kept = logged <= kPartLog && off + logged <= w.plog_cap;
+            if (kept)
+                for (uint32_t i = lane; i < logged; i += 32u) w.plog[off + i] = sm.log[i];
+            if (lane == 0) w.part_log[item] = make_uint2(off, kept ? logged : 0xFFFFFFFFu);
+            __threadfence();
+            __syncwarp();
+            uint32_t done = 0;
+            if (lane == 0) done = atomicAdd(&pi.parts_done, 1u);
+            done = __shfl_sync(0xffffffffu, done, 0);
+            if (done + 1u != parts) return;
+            __threadfence();
+            manifold_clear(m);
+            merging = true;
+            q = 0;
         }
-        __syncthreads();
-        Top4 ex = top4_shfl_up(inc, 1);
-        if (lane == 0) ex = top4_empty();
-        Top4 run = top4_merge(state, top4_merge(s_top[wid], ex));
-        // candidates of this thread that enter the manifold
-        uint32_t enter = 0u;
-        for (uint32_t mm = mask; mm; mm &= mm - 1u) {
-            const uint32_t k = __ffs(mm) - 1;
-            const I3 o = probe_offset(k);
-            const int32_t bx = cbv.x + o.x, by = cbv.y + o.y, bz = cbv.z + o.z;
-            const uint32_t vb = voxel_at(cs, cb, bx, by, bz);
-            const F3 wb = transform_point_n(c.pb, c.qnb, voxel_to_local(c.vs_b, bx, by, bz));
-            const float d2 = lensq3(wb - wa);
-            const float pen = cand_pen(c.vs_a, ta, vtype(vb), d2);
-            if (pen > run.v[3]) {
-                enter |= 1u << k;
-                top4_insert(run, pen);
+        // the merge, in part order
+        bool again = false;
+        for (; q < parts; ++q) {
+            const uint2 lg = __ldcg(w.part_log + (item - part) + q);
+            again = lg.y == 0xFFFFFFFFu;
+            if (again) break;
+            for (uint32_t b = 0; b < lg.y; b += 32u) {
+                uint2 r = make_uint2(0u, 0u);
+                float pen = -__int_as_float(0x7f800000);
+                if (b + lane < lg.y) {
+                    r = __ldcg(w.plog + lg.x + b + lane);
+                    pen = __uint_as_float(r.x);
+                }
+                for (uint32_t who; (who = __ballot_sync(0xffffffffu, pen > m.least)) != 0u;) {
+                    const uint32_t src = __ffs(who) - 1;
+                    const float cpen = __shfl_sync(0xffffffffu, pen, src);
+                    const uint32_t rec = __shfl_sync(0xffffffffu, r.y, src);
+                    candidate_add(g, sm, m, cpen, rec & 0x7FFFFFFu, rec >> 27);
+                    if (lane <= src) pen = -__int_as_float(0x7f800000);
+                }
             }
         }
-        // entering candidates in (voxel, probe) order: the threads list them
-        // at once, kBlockReplay at a time, into s_rec; thread 0 applies them
-        // in that order
-        uint32_t total = 0;
-        const uint32_t off = block_excl_scan((uint32_t)__popc(enter), &total);
-        for (uint32_t lo = 0; lo < total; lo += kBlockReplay) {
-            uint32_t e = off;
-            for (uint32_t mm = enter; mm; mm &= mm - 1u, ++e) {
-                if (e < lo || e >= lo + kBlockReplay) continue;
-                const uint32_t k = __ffs(mm) - 1;
-                const I3 o = probe_offset(k);
-                const I3 ibv{cbv.x + o.x, cbv.y + o.y, cbv.z + o.z};
-                const uint32_t vb = voxel_at(cs, cb, ibv.x, ibv.y, ibv.z);
-                const F3 wb = transform_point_n(c.pb, c.qnb, voxel_to_local(c.vs_b, ibv.x, ibv.y, ibv.z));
-                CandRec& r = s_rec[e - lo];
-                r.fid = feature_id(I3{x, y, z}, ibv);
-                r.pen = cand_pen(c.vs_a, ta, vtype(vb), lensq3(wb - wa));
-                r.li = (uint32_t)l;
-                r.k = k;
-                r._pad = 0u;
-            }
-            __syncthreads();
-            if (tid == 0) {
-                const uint32_t cnt = min(kBlockReplay, total - lo);
-                for (uint32_t i = 0; i < cnt; ++i) add_cand(sm, s_rec[i]);
-            }
-            __syncthreads();
-        }
-        // manifold penetration multiset -> state
-        if (tid == 0) cand_pens(sm);
-        __syncthreads();
-        state.v[0] = sm.pens[0];
-        state.v[1] = sm.pens[1];
-        state.v[2] = sm.pens[2];
-        state.v[3] = sm.pens[3];
+        if (!again) break;
     }
-    checked = block_sum(checked);
-    ncand = block_sum(ncand);
-    // the contacts left in the manifold
-    if (tid < sm.n) build_contact(cs, c, pi.rmin, (uint32_t)nx, (uint32_t)ny, sm.k[tid], &sm.c[tid]);
-    __syncthreads();
-    ManifoldRec& out = w.man[cur][p];
-    if (tid == 0) {
-        pi.voxels_checked = checked;
-        pi.candidates = ncand;
-        out.a = prA.id;
-        out.b = prB.id;
-        out.n = sm.n;
-        out.friction = sqrtf(prA.friction * prB.friction);
-        out.restitution = fmaxf(prA.restitution, prB.restitution);
-        out._pad = 0u;
-    }
-    __syncthreads();
-    const uint32_t words = sm.n * (uint32_t)(sizeof(ContactRec) / 4);
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(sm.c);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(out.c);
-    for (uint32_t i = tid; i < words; i += blockDim.x) dst[i] = src[i];
-    __syncthreads();
+    probe_store(w, cs, cur, p, pi, c, g, m, sm);
 }
 
 template <class G>
@@ -1870,33 +1991,32 @@ __device__ bool phase_probe(G& g, const WorldDev& w, const ColliderSet& cs, uint
     // its SM would slow it more than it is worth), or by one warp of a lone
     // CTA while its other warps start detecting at once
     const bool replay_cta = w.cfg.use_cache && g.nblocks() > 1u && g.block() == 0u;
-    if (replay_cta && w.cache_cap >= 64u * 16u &&
-        (size_t)(blockDim.x >> 5) * sizeof(WarpManifold) >= cta_replay_scratch_bytes()) {
+    if (replay_cta && w.cache_cap >= 48u &&
+        (size_t)(blockDim.x >> 5) * sizeof(WarpManifold) >= cta_replay_scratch_bytes(w.cache_cap)) {
         cache_replay_cta(w, csm, reinterpret_cast<unsigned char*>(warp_sm));
         return g.sync();
     }
     if (w.cfg.use_cache && g.rank() < 32u) cache_replay(w, csm);
-    // large regions first, one CTA each, then the rest one warp each
-    const uint32_t nh = *(volatile uint32_t*)&w.ctr[C_NHEAVY];
     if (replay_cta) return g.sync();
-    if (nh) {
-        __shared__ uint32_t s_h;
-        for (;;) {
-            __syncthreads();
-            if (threadIdx.x == 0) s_h = atomicAdd(&w.ctr[C_HWORK], 1u);
-            __syncthreads();
-            const uint32_t h = s_h;
-            if (h >= nh) break;
-            probe_pair_block(w, cs, cur, w.cons[h], warp_sm[0]);
-        }
-    }
+    // the parts of cut pairs first, then the other pairs, one warp each; a
+    // warp asks for its next item before it works on the one it has
+    const uint32_t nh = min(*(volatile uint32_t*)&w.ctr[C_NHEAVY], w.part_cap), nl = *(volatile uint32_t*)&w.ctr[C_NLIGHT];
+    uint32_t ask = 0;
+    if (lane == 0) ask = atomicAdd(&w.ctr[C_WORK], 1u);
     for (;;) {
-        uint32_t p = 0;
-        if (lane == 0) p = atomicAdd(&w.ctr[C_WORK], 1u);
-        p = __shfl_sync(0xffffffffu, p, 0);
-        if (p >= g.n_pairs) break;
-        const uint32_t fl = w.pinfo[p].flags;
-        if ((fl & (PF_DETECT | PF_CACHE)) && (fl & PF_REGION) && !(fl & PF_HEAVY)) probe_pair(w, cs, cur, p, sm);
+        const uint32_t i = __shfl_sync(0xffffffffu, ask, 0);
+        if (i >= nh + nl) break;
+        if (lane == 0) ask = atomicAdd(&w.ctr[C_WORK], 1u);
+        uint32_t p, part = 0xFFFFFFFFu;
+        if (i < nh) {
+            const uint2 it = w.part[i];
+            p = it.x;
+            part = it.y;
+            if (p == 0xFFFFFFFFu) continue;  // a place left by a pair that did not fit the list
+        } else {
+            p = w.colour[i - nh];
+        }
+        probe_item(w, cs, cur, p, part, i, sm);
     }
     return g.sync();
 }

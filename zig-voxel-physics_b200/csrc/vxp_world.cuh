@@ -85,17 +85,19 @@ enum : uint32_t {
     PF_DETECT = 1u << 7,    // detectVoxelCollisions runs
     PF_REGION = 1u << 8,    // overlap region non-empty
     PF_TESTED = 1u << 9,    // processPair was called
-    PF_HEAVY = 1u << 10,    // overlap region large enough to be probed by a whole CTA
+    PF_HEAVY = 1u << 10,    // overlap region cut into parts, probed by several warps
 };
 
 struct PairInfo {
     uint32_t ia, ib;
+    uint32_t ca, cb;        // their colliders (a tested pair)
     uint32_t flags;
     uint32_t hit;           // brick-pair cache: 0 not consulted, 1 hit, 2 miss
     uint32_t cache_slot;    // hit: entry read; miss: entry written
     int32_t rmin[3], rmax[3];
     uint32_t voxels_checked;
     uint32_t candidates;
+    uint32_t parts, parts_done;  // PF_HEAVY: parts, and how many of them are probed
     uint32_t key_a, key_b;
     unsigned long long th; // transform hash of the cache key
 };
@@ -162,7 +164,7 @@ struct StepCfg {
     uint32_t solver_flow;     // 1: sweeps ordered by per-body event counters, 0: colour barriers
     uint32_t flow_smem_chunks;  // constraint chunks per block the launch's shared memory holds
     uint32_t record_substeps;   // 1: write every body's state after each substep to subrec
-    uint32_t heavy_voxels;      // overlap regions of at least this many voxels are probed by a CTA (0: never)
+    uint32_t heavy_voxels;      // overlap regions of at least this many voxels are cut into parts (0: never)
     uint32_t count_bricks;      // count the bricks each probed pair touches (C_BRICKS; traffic accounting only)
     uint32_t owner_groups;      // > 1: pack each colour by owner group (home body mod this; the sweep cluster's size)
     uint32_t islands_on;        // IslandManager statistics each solve (PhysicsConfig.enable_islands)
@@ -190,7 +192,7 @@ enum : uint32_t {
     C_STEP_SKIPPED,
     C_MAX_PEN_KEY,   // ordered-int key of max penetration
     C_CANDIDATES,
-    C_WORK,          // work counter of phase_probe
+    C_WORK,          // work counter of phase_probe over both lists
     C_DUMP_N,        // candidates dumped
     C_AWAKE,         // dynamic awake bodies seen by the sleep check
     C_BRICKS,        // bricks of A in the overlap region + bricks of B in B's
@@ -198,8 +200,9 @@ enum : uint32_t {
     C_KIN_CONTACT,   // constraints touching an awake kinematic body
     C_SOLVE_GO,      // set by the narrow part of a step when its solve part may run
     C_SUBREC,        // substeps recorded in subrec by the last solve
-    C_NHEAVY,        // pairs in the CTA-probed list (w.cons during the probe)
-    C_HWORK,         // work counter over that list
+    C_NHEAVY,        // parts of cut pairs listed (w.part)
+    C_NLIGHT,        // other pairs to probe (w.colour during the probe)
+    C_NLOG,          // candidates in plog
     C_CONS_M,        // constraint manifolds of the step (solve part split in two kernels)
     C_CONS_NCOL,     // their colours
     C_SWEEP,         // how the cluster sweeps ran (SWEEP_*)
@@ -266,6 +269,12 @@ struct WorldDev {
     // pairs
     uint2* pairs;                 // (body_a id, body_b id)
     PairInfo* pinfo;
+    // the parts of pairs with a large region: (pair, part), and per part its
+    // candidates in plog (first, number; ~0u: not kept)
+    uint2* part;
+    uint2* part_log;
+    uint2* plog;                  // (a batch slot's is cp, which is free until the constraint table is built)
+    uint32_t part_cap, plog_cap;
     // contact manager: two manifold arrays / hash tables, flipped per frame
     ManifoldRec* man[2];
     HashSlot* ht[2];

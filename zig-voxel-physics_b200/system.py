@@ -226,7 +226,7 @@ class VoxelPhysicsSystem:
         return int(n.value)
 
     def set_heavy_pair_voxels(self, n: int) -> None:
-        """Pairs with at least n overlap-region voxels are probed by a whole CTA (0: never)."""
+        """Pairs with at least n overlap-region voxels are probed by several warps (0: never)."""
         self._check(self.lib.vxp_set_heavy_pair_voxels(self.ctx, int(n)))
 
     def set_wait_limit_ns(self, ns: int) -> None:
