@@ -1045,7 +1045,7 @@ struct WorldBuffers {
         scan_blocks = blocks;
         bool ok = true;
         ok &= n_pairs_dev.reserve(1) == cudaSuccess;
-        ok &= frame.reserve(2) == cudaSuccess;
+        ok &= frame.reserve(4) == cudaSuccess;
         ok &= colour_cnt.reserve(257) == cudaSuccess;
         ok &= colour_cur.reserve(256) == cudaSuccess;
         ok &= ocnt.reserve(kOwnerPoints + 2 * kMaxOwnerGroups) == cudaSuccess;
@@ -1121,6 +1121,11 @@ struct WorldBuffers {
                 }
                 const uint32_t latest_n = fr[1];
                 const uint32_t latest = fr[0] & 1u;  // the next step reads it as previous
+                if (cudaMemcpy(frame.p + 2u + latest, &new_ht, sizeof(new_ht), cudaMemcpyHostToDevice) !=
+                    cudaSuccess) {
+                    err = "frame write failed";
+                    return VXP_ERR_CUDA;
+                }
                 if (latest_n) {
                     ManifoldRec* m = latest ? man1.p : man0.p;
                     HashSlot* h = latest ? ht1.p : ht0.p;

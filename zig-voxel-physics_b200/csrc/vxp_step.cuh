@@ -463,7 +463,13 @@ __device__ __forceinline__ unsigned long long cache_key_hash(uint32_t a, uint32_
     return h;
 }
 
-// Hash table of pair keys (open addressing).
+// Hash table of pair keys (open addressing).  A frame's table is as large as
+// its pair list asks for (load at most one half), not as its buffer: the
+// clear is part of every step (a 4 MB buffer for the 4096-body pile).
+__device__ __forceinline__ uint32_t ht_size_of(const WorldDev& w, uint32_t n_pairs) {
+    const uint32_t want = max(64u, 2u * n_pairs);
+    return min(w.ht_cap, 1u << (32 - __clz((int)(want - 1u))));
+}
 __device__ __forceinline__ uint32_t ht_hash(unsigned long long k, uint32_t cap) {
     k ^= k >> 33;
     k *= 0xff51afd7ed558ccdull;
@@ -484,10 +490,12 @@ __device__ void ht_insert(HashSlot* t, uint32_t cap, unsigned long long key, uin
     }
 }
 __device__ uint32_t ht_find(const HashSlot* t, uint32_t cap, unsigned long long key) {
+    if (cap == 0u) return 0xFFFFFFFFu;
     uint32_t s = ht_hash(key, cap);
     for (uint32_t i = 0; i < cap; ++i) {
-        const unsigned long long k = t[s].key;
-        if (k == key) return t[s].idx;
+        const uint4 v = *reinterpret_cast<const uint4*>(t + s);  // key and index at once
+        const unsigned long long k = (unsigned long long)v.x | ((unsigned long long)v.y << 32);
+        if (k == key) return v.z;
         if (k == 0ull) return 0xFFFFFFFFu;
         s = (s + 1u) & (cap - 1u);
     }
@@ -753,10 +761,10 @@ __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint
         w.ctr[C_PAIRS_IN] = P;
         w.cframe[0] += 1ull;  // BrickPairCache.beginFrame
     }
-    for (uint32_t i = g.rank(); i < w.ht_cap; i += g.size()) {
-        w.ht[cur][i].key = 0ull;
-        w.ht[cur][i].idx = 0xFFFFFFFFu;
-    }
+    const uint32_t ht_cur = ht_size_of(w, P);
+    for (uint32_t i = g.rank(); i < ht_cur; i += g.size())
+        *reinterpret_cast<uint4*>(w.ht[cur] + i) = make_uint4(0u, 0u, 0xFFFFFFFFu, 0u);
+    if (g.rank() == 0) w.frame[2u + cur] = ht_cur;
     for (uint32_t p = g.rank(); p < P; p += g.size()) {
         const uint2 pr = w.pairs[p];
         const uint32_t ia = find_body(w.ids, w.n_bodies, pr.x), ib = find_body(w.ids, w.n_bodies, pr.y);
@@ -2024,22 +2032,60 @@ __device__ bool phase_probe(G& g, const WorldDev& w, const ColliderSet& cs, uint
 // ---------------------------------------------------------------------------
 // Phase: finalize (cache hits, carries, ContactManager.addManifold warm start)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void warm_from_prev(const WorldDev& w, uint32_t prev, ManifoldRec& m) {
-    const uint32_t idx = ht_find(w.ht[prev], w.ht_cap, pair_key(m.a, m.b));
+// N 8-byte words from src to dst, all loaded before any is stored: a struct
+// assignment's loads wait for the stores before them (they may alias), one
+// L2 round trip a word.
+template <int N>
+__device__ __forceinline__ void copy_words(void* dst, const void* src) {
+    unsigned long long r[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) r[i] = reinterpret_cast<const unsigned long long*>(src)[i];
+#pragma unroll
+    for (int i = 0; i < N; ++i) reinterpret_cast<unsigned long long*>(dst)[i] = r[i];
+}
+static_assert(sizeof(ContactRec) == 88 && sizeof(ManifoldRec) == 24 + 4 * 88, "copied in 8-byte words");
+
+// ContactManager.addManifold's warm start: the impulses of the previous
+// frame's contacts with the same feature ids.  Both manifolds' ids and the
+// old impulses are loaded at once.
+__device__ __forceinline__ void warm_from_prev(const WorldDev& w, uint32_t prev, uint32_t ht_size, ManifoldRec& m) {
+    const uint32_t idx = ht_find(w.ht[prev], ht_size, pair_key(m.a, m.b));
     if (idx == 0xFFFFFFFFu) return;
     const ManifoldRec& o = w.man[prev][idx];
-    for (uint32_t i = 0; i < m.n; ++i)
-        for (uint32_t j = 0; j < o.n; ++j)
-            if (m.c[i].feature_id == o.c[j].feature_id) {
-                m.c[i].normal_impulse = o.c[j].normal_impulse;
-                m.c[i].tangent_impulse[0] = o.c[j].tangent_impulse[0];
-                m.c[i].tangent_impulse[1] = o.c[j].tangent_impulse[1];
-                break;
+    const uint32_t n = m.n, on = o.n;
+    unsigned long long fo[4], fm[4];
+    float i0[4], i1[4], i2[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; ++j) {
+        fo[j] = o.c[j].feature_id;
+        fm[j] = m.c[j].feature_id;
+        i0[j] = o.c[j].normal_impulse;
+        i1[j] = o.c[j].tangent_impulse[0];
+        i2[j] = o.c[j].tangent_impulse[1];
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; ++i) {
+        bool found = false;
+        float a = 0.f, b = 0.f, c = 0.f;
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j)
+            if (!found && j < on && fm[i] == fo[j]) {
+                found = true;
+                a = i0[j];
+                b = i1[j];
+                c = i2[j];
             }
+        if (i < n && found) {
+            m.c[i].normal_impulse = a;
+            m.c[i].tangent_impulse[0] = b;
+            m.c[i].tangent_impulse[1] = c;
+        }
+    }
 }
 
 template <class G>
 __device__ bool phase_finalize(G& g, const WorldDev& w, uint32_t cur, uint32_t prev) {
+    const uint32_t ht_cur = ht_size_of(w, g.n_pairs), ht_prev = *(volatile uint32_t*)&w.frame[2u + prev];
     uint32_t skipped = 0, colliding = 0, contacts = 0, voxels = 0, manifolds = 0, cands = 0;
     for (uint32_t p = g.rank(); p < g.n_pairs; p += g.size()) {
         const PairInfo& pi = w.pinfo[p];
@@ -2048,9 +2094,15 @@ __device__ bool phase_finalize(G& g, const WorldDev& w, uint32_t cur, uint32_t p
         if (fl & PF_CARRY) {
             ++skipped;
             const uint2 pr = w.pairs[p];
-            const uint32_t idx = ht_find(w.ht[prev], w.ht_cap, pair_key(pr.x, pr.y));
-            if (idx != 0xFFFFFFFFu) m = w.man[prev][idx];
-            else m.n = 0u;
+            const uint32_t idx = ht_find(w.ht[prev], ht_prev, pair_key(pr.x, pr.y));
+            if (idx != 0xFFFFFFFFu) {
+                const ManifoldRec& o = w.man[prev][idx];
+                copy_words<24>(&m, &o);
+                copy_words<23>(reinterpret_cast<unsigned long long*>(&m) + 24,
+                               reinterpret_cast<const unsigned long long*>(&o) + 24);
+            } else {
+                m.n = 0u;
+            }
         } else if (!(fl & PF_TESTED) || (fl & (PF_NOCOLL | PF_SEPARATED))) {
             m.n = 0u;
         } else if ((fl & PF_CACHE) && pi.hit == 1u) {
@@ -2071,19 +2123,19 @@ __device__ bool phase_finalize(G& g, const WorldDev& w, uint32_t cur, uint32_t p
                         if (m.c[j].feature_id == v.c[i].feature_id) {
                             const float ni = m.c[j].normal_impulse, t0 = m.c[j].tangent_impulse[0],
                                         t1 = m.c[j].tangent_impulse[1];
-                            m.c[j] = v.c[i];
+                            copy_words<11>(&m.c[j], &v.c[i]);
                             m.c[j].normal_impulse = ni;
                             m.c[j].tangent_impulse[0] = t0;
                             m.c[j].tangent_impulse[1] = t1;
                             dup = true;
                             break;
                         }
-                    if (!dup && m.n < 4u) m.c[m.n++] = v.c[i];
+                    if (!dup && m.n < 4u) copy_words<11>(&m.c[m.n++], &v.c[i]);
                 }
                 ++colliding;
                 contacts += v.n;
                 voxels += v.voxels_checked;
-                warm_from_prev(w, prev, m);
+                warm_from_prev(w, prev, ht_prev, m);
             } else {
                 m.n = 0u;
             }
@@ -2102,14 +2154,14 @@ __device__ bool phase_finalize(G& g, const WorldDev& w, uint32_t cur, uint32_t p
             if (m.n > 0u) {
                 ++colliding;
                 contacts += m.n;
-                warm_from_prev(w, prev, m);
+                warm_from_prev(w, prev, ht_prev, m);
             }
         } else {
             m.n = 0u;
         }
         if (m.n > 0u) {
             ++manifolds;
-            ht_insert(w.ht[cur], w.ht_cap, pair_key(m.a, m.b), p);
+            ht_insert(w.ht[cur], ht_cur, pair_key(m.a, m.b), p);
         }
     }
     skipped = warp_sum(skipped);
@@ -2142,13 +2194,16 @@ __device__ bool phase_finalize(G& g, const WorldDev& w, uint32_t cur, uint32_t p
             v.has_collision = n > 0u ? 1u : 0u;
             v.voxels_checked = pi.voxels_checked;
             for (uint32_t i = 0; i < n; ++i) {
-                v.c[i] = m.c[i];
-                v.c[i].normal_impulse = 0.f;
-                v.c[i].tangent_impulse[0] = 0.f;
-                v.c[i].tangent_impulse[1] = 0.f;
-                v.c[i].normal_mass = 0.f;
-                v.c[i].tangent_mass[0] = 0.f;
-                v.c[i].tangent_mass[1] = 0.f;
+                // words 6 (its second half) to 9: the impulses and masses, zero in the cache
+                unsigned long long r[11];
+                const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&m.c[i]);
+                unsigned long long* dst = reinterpret_cast<unsigned long long*>(&v.c[i]);
+#pragma unroll
+                for (int k = 0; k < 11; ++k) r[k] = src[k];
+#pragma unroll
+                for (int k = 0; k < 11; ++k)
+                    dst[k] = k == 6 ? (r[k] & 0xFFFFFFFFull) : (k >= 7 && k <= 8) ? 0ull
+                                                             : k == 9 ? (r[k] & ~0xFFFFFFFFull) : r[k];
             }
         }
     }
@@ -2634,8 +2689,27 @@ __device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_
         const DBody& B = w.body[pi.ib];
         const F3 pa = f3of(A.p), pb = f3of(B.p);
         const Qt qa = qof(A.q), qb = qof(B.q);
-        for (uint32_t i = 0; i < m.n; ++i) {
-            const ContactRec& ct = m.c[i];
+        // a contact's first sixteen floats (point, normal, penetration, anchors,
+        // impulses), the next point's loaded before this one's are stored
+        struct Ct {
+            float point[3], normal[3], penetration, la[3], lb[3], normal_impulse, tangent_impulse[2];
+        };
+        static_assert(sizeof(Ct) == 64, "loaded in 8-byte words");
+        auto ct_load = [&](uint32_t i) {
+            union {
+                unsigned long long w[8];
+                Ct c;
+            } u;
+            const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&m.c[i]);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) u.w[k] = src[k];
+            return u.c;
+        };
+        const uint32_t mn = m.n;
+        Ct nxt = ct_load(0);
+        for (uint32_t i = 0; i < mn; ++i) {
+            const Ct ct = nxt;
+            if (i + 1u < mn) nxt = ct_load(i + 1u);
             const F3 la{ct.la[0], ct.la[1], ct.la[2]}, lb{ct.lb[0], ct.lb[1], ct.lb[2]};
             const F3 nn{ct.normal[0], ct.normal[1], ct.normal[2]};
             const F3 wa = qrotate(qa, la) + pa;
@@ -4349,15 +4423,29 @@ __device__ bool phase_store(G& g, const WorldDev& w, uint32_t cur, uint32_t M, b
         for (uint32_t pos = g.rank(); pos < M; pos += g.size()) {
             const uint4 cmv = w.cm[pos];
             ManifoldRec& m = w.man[cur][cmv.w];
+            // every field loaded before any is stored
+            float v[4][6];
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i)
+                if (i < cmv.z) {
+                    v[i][0] = w.cp[cpi(w, CP_NI, i, pos)];
+                    v[i][1] = w.cp[cpi(w, CP_TI0, i, pos)];
+                    v[i][2] = w.cp[cpi(w, CP_TI1, i, pos)];
+                    v[i][3] = w.cp[cpi(w, CP_NM, i, pos)];
+                    v[i][4] = w.cp[cpi(w, CP_TM0, i, pos)];
+                    v[i][5] = w.cp[cpi(w, CP_TM1, i, pos)];
+                }
             const uint32_t n = cmv.z < m.n ? cmv.z : m.n;
-            for (uint32_t i = 0; i < n; ++i) {
-                m.c[i].normal_impulse = w.cp[cpi(w, CP_NI, i, pos)];
-                m.c[i].tangent_impulse[0] = w.cp[cpi(w, CP_TI0, i, pos)];
-                m.c[i].tangent_impulse[1] = w.cp[cpi(w, CP_TI1, i, pos)];
-                m.c[i].normal_mass = w.cp[cpi(w, CP_NM, i, pos)];
-                m.c[i].tangent_mass[0] = w.cp[cpi(w, CP_TM0, i, pos)];
-                m.c[i].tangent_mass[1] = w.cp[cpi(w, CP_TM1, i, pos)];
-            }
+#pragma unroll
+            for (uint32_t i = 0; i < 4u; ++i)
+                if (i < n) {
+                    m.c[i].normal_impulse = v[i][0];
+                    m.c[i].tangent_impulse[0] = v[i][1];
+                    m.c[i].tangent_impulse[1] = v[i][2];
+                    m.c[i].normal_mass = v[i][3];
+                    m.c[i].tangent_mass[0] = v[i][4];
+                    m.c[i].tangent_mass[1] = v[i][5];
+                }
         }
     }
     return true;

@@ -127,7 +127,7 @@ struct CacheValRec {
     uint32_t n, has_collision, voxels_checked, _pad;
 };
 
-struct HashSlot {            // pairKey -> manifold index
+struct __align__(16) HashSlot {  // pairKey -> manifold index
     unsigned long long key;  // 0 = empty (pair keys are never 0: ids > 0)
     uint32_t idx, _pad;
 };
@@ -279,7 +279,8 @@ struct WorldDev {
     ManifoldRec* man[2];
     HashSlot* ht[2];
     uint32_t* frame;              // [0] = frame counter (man[frame & 1] is the latest),
-                                  // [1] = pair count of the latest manifold array
+                                  // [1] = pair count of the latest manifold array,
+                                  // [2], [3] = slots of ht[0], ht[1] in use (a power of two, or 0: empty)
     // brick-pair cache
     CacheKeyRec* ckey;
     CacheValRec* cval;
