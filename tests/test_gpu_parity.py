@@ -421,3 +421,12 @@ def test_cache_replay_bins(vxp, cache):
     fewest bins, a last bin with a remainder, windows that wrap."""
     sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=7, seed=3)
     lockstep(vxp, sc, 50, mode=1, brick_pair_cache_size=cache, substeps=8).close()
+
+
+@pytest.mark.parametrize("boxes", [2, 3, 5, 6])
+@pytest.mark.parametrize("colouring", [0, 1])
+def test_launch_chosen_by_size(vxp, boxes, colouring):
+    """The step as the library launches it by itself: worlds of 8, 27, 125 and
+    216 boxes lie on either side of the one-CTA / cluster / grid lines."""
+    sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=boxes, seed=6)
+    lockstep(vxp, sc, 80, mode=-1, colouring=colouring, substeps=8).close()

@@ -31,6 +31,7 @@ using namespace vxp;
 // Kernels
 // ===========================================================================
 
+constexpr uint32_t kClusterThreads = 256;
 // Dynamic shared memory: one WarpManifold per warp, then the cache table.
 __device__ __forceinline__ CacheSmem cache_smem(unsigned char* raw, uint32_t nwarps, uint32_t cap) {
     unsigned char* p = raw + sizeof(WarpManifold) * nwarps;
@@ -77,15 +78,25 @@ __global__ void __launch_bounds__(256, 1) k_solve_grid(const __grid_constant__ W
 __global__ void __launch_bounds__(256, 1) k_solve_cluster(const __grid_constant__ WorldDev w, uint32_t smem_bytes,
                                                           uint32_t whole) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint32_t ncta;
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
-    if (ncta != gridDim.x) {  // launch constants: the same verdict in every block
+    ClusterGroup g = cluster_group();
+    if (g.ncta != gridDim.x) {  // launch constants: the same verdict in every block
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&w.ctr[C_ERROR], ERR_BOUNDS);
         return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0 && w.ts) w.ts[TS_SW_START] = global_ns();
-    ClusterGroup g;
     world_step_sweeps(g, w, smem_raw, smem_bytes, whole != 0u);
+}
+// A whole step of a world too small to fill the GPU on one cluster: one launch
+// and hardware barriers (0.2 us) where the grid's three kernels pay 2 us a
+// barrier and 6 us a launch, and sixteen times the warps of one CTA for the
+// pairs and voxels.
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    k_step_cluster(const __grid_constant__ WorldDev w, const __grid_constant__ ColliderSet cs, uint32_t smem_bytes) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    WarpManifold* wsm = reinterpret_cast<WarpManifold*>(smem_raw);
+    const CacheSmem csm = cache_smem(smem_raw, blockDim.x / 32u, w.cache_cap);
+    ClusterGroup g = cluster_group();
+    if (world_step_narrow(g, w, cs, wsm, csm)) world_step_sweeps(g, w, smem_raw, smem_bytes, true);
 }
 
 // Pair source: world AABB of each body's collider (AABB.transform,
@@ -1002,6 +1013,7 @@ struct WorldBuffers {
     // constraint rows that do not fit in the cluster's shared memory
     bool spill_rows = false;
     std::vector<uint32_t> collider_public;
+    std::vector<uint32_t> moving_collider;  // per non-static body its collider's index
     DBuf<DBody> body;
     DBuf<DBodyProp> prop;
     DBuf<float4> p0, qn, aabb_mn, aabb_mx;
@@ -1019,7 +1031,7 @@ struct WorldBuffers {
     DBuf<uint32_t> frame;
     DBuf<uint32_t> cons, colour, pos_of, packed_pair, adj, flag;
     DBuf<CacheLook> clist;
-    DBuf<uint2> part, part_log, plog;
+    DBuf<uint2> part, plog;  // part: the parts, then as many log records; plog: see ensure_parts
     DBuf<float> cp, crow;
     // islands: per body, per pair slot (two builds' keys), kept state words
     DBuf<uint32_t> isl_parent, isl_flag, isl_size, isl_state;
@@ -1066,6 +1078,16 @@ struct WorldBuffers {
         return VXP_OK;
     }
 
+    // Room for n parts of cut pairs.  own_log: with a buffer of their own for
+    // their candidates (a world of few pairs with very large regions).
+    int ensure_parts(size_t n, bool own_log, std::string& err) {
+        if (part.reserve(2u * n) != cudaSuccess || (own_log && plog.reserve(32u * n) != cudaSuccess)) {
+            err = fmt("device allocation of %zu pair parts failed", n);
+            return VXP_ERR_OOM;
+        }
+        return VXP_OK;
+    }
+
     // Grows every pair-sized buffer to hold `need` pairs; keeps the latest
     // frame's manifolds and rebuilds their hash table.
     int ensure_pairs(uint32_t need, std::string& err) {
@@ -1087,13 +1109,8 @@ struct WorldBuffers {
         ok &= flag.reserve(cap) == cudaSuccess;
         ok &= clist.reserve(cap) == cudaSuccess;
         ok &= cp.reserve((size_t)CP_NFIELDS * 4 * cap) == cudaSuccess;
-        // parts of cut pairs: a context's world (few pairs can be very large)
-        // gets room for 64 Ki and their candidates, a batch slot four a pair
-        // (its candidates go to cp)
-        const size_t parts = std::max<size_t>((size_t)4 * cap, spill_rows ? 65536 : 0);
-        ok &= part.reserve(parts) == cudaSuccess;
-        ok &= part_log.reserve(parts) == cudaSuccess;
-        if (spill_rows) ok &= plog.reserve(32 * parts) == cudaSuccess;
+        // parts of cut pairs, four a pair; their candidates go to cp
+        if (int rc = ensure_parts(4u * cap, false, err)) return rc;
         if (spill_rows) ok &= crow.reserve((size_t)CP_NVEL * 4 * cap) == cudaSuccess;
         ok &= isl_keys0.reserve(cap, true) == cudaSuccess;
         ok &= isl_keys1.reserve(cap, true) == cudaSuccess;
@@ -1190,6 +1207,7 @@ struct WorldBuffers {
         std::vector<DBodyProp> dp(n);
         std::vector<uint2> id(n);
         collider_public.resize(n);
+        moving_collider.clear();
         for (uint32_t i = 0; i < n; ++i) {
             const vxp_body& s = b[i];
             if (s.body_type > 2u) {
@@ -1212,6 +1230,7 @@ struct WorldBuffers {
             p.id = s.id;
             p.type = s.body_type;
             p.collider = cols.index_of(s.collider_id);
+            if (s.body_type != 0u) moving_collider.push_back(p.collider);
             p.sleeping = s.is_sleeping ? 1u : 0u;
             collider_public[i] = s.collider_id;
             id[i] = make_uint2(s.id, i);
@@ -1302,8 +1321,8 @@ struct WorldBuffers {
         w.cwriter = cwriter.p;
         w.clist = clist.p;
         w.part = part.p;
-        w.part_log = part_log.p;
-        w.part_cap = (uint32_t)part.n;
+        w.part_log = part.p + part.n / 2u;
+        w.part_cap = (uint32_t)(part.n / 2u);
         w.plog = plog.p ? plog.p : reinterpret_cast<uint2*>(cp.p);
         w.plog_cap = (uint32_t)(plog.p ? plog.n : cp.bytes() / sizeof(uint2));
         w.cframe = cframe.p;
@@ -1364,7 +1383,7 @@ struct WorldBuffers {
                ids.bytes() + pcount.bytes() + poff.bytes() + adj_off.bytes() + adj_cur.bytes() + bmask.bytes() +
                pairs.bytes() + pinfo.bytes() + man0.bytes() + man1.bytes() + ht0.bytes() + ht1.bytes() +
                cons.bytes() + colour.bytes() + pos_of.bytes() + packed_pair.bytes() + adj.bytes() + flag.bytes() +
-               clist.bytes() + part.bytes() + part_log.bytes() + plog.bytes() + cp.bytes() + cm.bytes() + rk.bytes() + ev.bytes() + snap.bytes() + chunk.bytes() + cfr.bytes() +
+               clist.bytes() + part.bytes() + plog.bytes() + cp.bytes() + cm.bytes() + rk.bytes() + ev.bytes() + snap.bytes() + chunk.bytes() + cfr.bytes() +
                ckey.bytes() + cval.bytes() +
                cwriter.bytes() + scan.bytes() + ctr.bytes() + ts.bytes() + dump.bytes() + ocnt.bytes() + ocur.bytes() +
                stat.bytes() + bpmask.bytes() + crow.bytes() + isl_parent.bytes() + isl_flag.bytes() +
@@ -1468,7 +1487,10 @@ struct vxp_ctx {
                 ev_cons = nullptr;
     uint32_t cluster_size = 0;  // CTAs of the cluster that runs the sweeps (0: no cluster launch here)
     uint32_t cluster_smem = 0;  // dynamic shared memory of each of its CTAs
+    uint32_t step_cluster_smem = 0;  // and of a whole step's (0: not available)
     uint32_t cluster_state_cap = 0xFFFFFFFFu;  // of which the sweeps' state may use at most this
+    uint64_t voxels = 0;        // of the moving bodies' collider bounds (step_launch)
+    bool voxels_known = false;
     bool cluster_whole = false;  // the cluster also builds the constraint table and colours it
     bool last_cluster = false;
     bool last_grid = false;
@@ -1523,26 +1545,67 @@ static void cluster_config(cudaLaunchConfig_t* lc, cudaLaunchAttribute* at, uint
 // Longest wait of a block at a grid barrier before it gives up (ERR_TIMEOUT).
 constexpr unsigned long long kGridWaitNs = 10ull * 1000ull * 1000ull * 1000ull;
 
+// How a step is launched when the caller leaves it open: one CTA, one cluster,
+// or the whole grid in three kernels.  The bodies set the number of pairs and
+// barriers, the moving bodies' voxels the probing.  Step kernels, us, one CTA /
+// cluster of 16 / grid:
+//   1 cube 117 / 143 / 204      16 cubes 230 / 241 / 302     64 cubes 382 / 316 / 359
+//   27 boxes 438 / 325 / 366    125 boxes 1218 / 520 / 515   216 cubes 1148 / 503 / 507
+//   343 boxes 2222 / 676 / 616  8 of 40^3 voxels (0.5 M) 1039 / 446 / 499
+//   27 of 64^3 voxels (7 M) 9255 / 1514 / 985
+enum class StepLaunch { kBlock, kCluster, kGrid };
+constexpr uint32_t kBlockBodies = 17, kBlockVoxels = 12 * 1024;
+constexpr uint32_t kClusterBodies = 160, kClusterVoxels = 1024 * 1024;
+StepLaunch step_launch(vxp_ctx* ctx) {
+    if (!ctx->voxels_known) {
+        // the bounds of the moving bodies' colliders, as placed
+        uint64_t v = 0;
+        for (uint32_t ci : ctx->w.moving_collider) {
+            if (ci >= ctx->cols.colliders.size()) continue;
+            const DCollider& d = ctx->cols.colliders[ci].d;
+            uint64_t c = 1;
+            for (int k = 0; k < 3; ++k) c *= (uint64_t)std::max<int64_t>(0, (int64_t)d.max_bound[k] - d.min_bound[k]);
+            v += c;
+        }
+        ctx->voxels = v;
+        ctx->voxels_known = true;
+    }
+    if (ctx->use_grid >= 0) return ctx->use_grid ? StepLaunch::kGrid : StepLaunch::kBlock;
+    const uint32_t n = ctx->w.n_bodies;
+    if (n <= kBlockBodies && ctx->voxels <= kBlockVoxels) return StepLaunch::kBlock;
+    const bool cluster = ctx->solver_flow == VXP_SOLVER_CLUSTER && ctx->cluster_size > 0 && ctx->step_cluster_smem > 0;
+    if (n > kClusterBodies || ctx->voxels > kClusterVoxels) return StepLaunch::kGrid;
+    return cluster ? StepLaunch::kCluster : n <= 64 ? StepLaunch::kBlock : StepLaunch::kGrid;
+}
+
 // Runs the step kernel.  device_pairs: the kernel builds the pair list itself.
 int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, float margin) {
     if (int rc = ctx->cols.sync(ctx->stream, ctx->err)) return rc;
-    const bool grid = ctx->use_grid == 1 || (ctx->use_grid < 0 && ctx->w.n_bodies >= 512);
+    const StepLaunch how = step_launch(ctx);
+    // large colliders: room for the parts their pairs may be cut into, a part
+    // per 512 voxels of bounds, and for those parts' candidates
+    if (ctx->voxels > kClusterVoxels) {
+        const size_t parts = (size_t)std::min<uint64_t>(ctx->voxels / 512u, 1u << 18);
+        if (parts > ctx->w.part.n / 2u || !ctx->w.plog.p)
+            if (int rc = ctx->w.ensure_parts(std::max(parts, ctx->w.part.n / 2u), true, ctx->err)) return rc;
+    }
+    const bool grid = how == StepLaunch::kGrid, one_cluster = how == StepLaunch::kCluster;
     const bool cluster = grid && ctx->solver_flow == VXP_SOLVER_CLUSTER && ctx->cluster_size > 0;
     const uint32_t flow = ctx->solver_flow == VXP_SOLVER_EVENTS ? 1u : 0u;
     WorldDev w = ctx->w.make(ctx->cfg, dt, phases, ctx->solver_div, device_pairs, margin, flow);
     const size_t smem = grid ? grid_smem(w.cache_cap) : block_smem(w.cache_cap);
-    if (!grid) w.cfg.block_smem = (uint32_t)smem;
+    if (!grid && !one_cluster) w.cfg.block_smem = (uint32_t)smem;
     w.cfg.flow_smem_chunks = grid ? flow_chunks(solve_smem()) : 0u;
     w.cfg.heavy_voxels = ctx->heavy_voxels;
     w.cfg.count_bricks = ctx->count_bricks ? 1u : 0u;
-    w.cfg.owner_groups = cluster ? ctx->cluster_size : 1u;
+    w.cfg.owner_groups = cluster ? ctx->cluster_size : one_cluster ? ctx->cluster_size : 1u;
     if (ctx->record_substeps) {
         const size_t need = (size_t)std::max(1u, ctx->cfg.substeps) * std::max(1u, ctx->w.n_bodies) * 13u;
         if (ctx->subrec.reserve(need) != cudaSuccess) return fail(ctx, VXP_ERR_OOM, "substep record buffer");
         w.cfg.record_substeps = 1u;
         w.subrec = ctx->subrec.p;
     }
-    if (!grid) CK(cudaMemcpyAsync(ctx->d_world.p, &w, sizeof(w), cudaMemcpyHostToDevice, ctx->stream));
+    if (!grid && !one_cluster) CK(cudaMemcpyAsync(ctx->d_world.p, &w, sizeof(w), cudaMemcpyHostToDevice, ctx->stream));
     const ColliderSet cs = ctx->cols.set();
     CK(cudaEventRecord(ctx->ev0, ctx->stream));
     if (grid) {
@@ -1568,6 +1631,11 @@ int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, floa
             CK(cudaLaunchKernelEx(&lc, k_solve_cluster, w, std::min(ctx->cluster_smem, ctx->cluster_state_cap),
                                   whole));
         }
+    } else if (one_cluster) {
+        cudaLaunchConfig_t lc = {};
+        cudaLaunchAttribute at[1];
+        cluster_config(&lc, at, ctx->cluster_size, ctx->step_cluster_smem, ctx->stream);
+        CK(cudaLaunchKernelEx(&lc, k_step_cluster, w, cs, std::min(ctx->step_cluster_smem, ctx->cluster_state_cap)));
     } else {
         k_step_block<kBlockThreads><<<1, kBlockThreads, smem, ctx->stream>>>(ctx->d_world.p, cs);
         CK(cudaGetLastError());
@@ -1889,6 +1957,15 @@ int vxp_create(const vxp_config* cfg, int device, vxp_ctx** out) {
         ctx->cluster_smem = (uint32_t)(optin - (int)fa.sharedSizeBytes);
     cudaFuncSetAttribute(k_solve_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaFuncSetAttribute(k_solve_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->cluster_smem);
+    // k_step_cluster: as much as one block may have beside its static shared memory
+    cudaFuncAttributes fs = {};
+    if (cudaFuncGetAttributes(&fs, k_step_cluster) == cudaSuccess && optin > (int)fs.sharedSizeBytes)
+        ctx->step_cluster_smem = (uint32_t)(optin - (int)fs.sharedSizeBytes);
+    if (ctx->step_cluster_smem < step_smem(kClusterThreads, cache_cap) ||
+        cudaFuncSetAttribute(k_step_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaFuncSetAttribute(k_step_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)ctx->step_cluster_smem) != cudaSuccess)
+        ctx->step_cluster_smem = 0;
     for (uint32_t n : {16u, 8u}) {
         cudaLaunchConfig_t lc = {};
         cudaLaunchAttribute at[1];
@@ -1934,6 +2011,7 @@ int vxp_last_error(const vxp_ctx* ctx, char* buf, size_t n) {
 int vxp_collider_upload(vxp_ctx* ctx, uint32_t collider_id, float voxel_size, const vxp_brick* bricks,
                         uint32_t n_bricks) {
     if (!ctx) return VXP_ERR_ARG;
+    ctx->voxels_known = false;
     return ctx->cols.upload(collider_id, voxel_size, bricks, n_bricks, ctx->err);
 }
 
@@ -1941,6 +2019,7 @@ int vxp_collider_edit(vxp_ctx* ctx, uint32_t collider_id, const int32_t* coords,
                       int mode) {
     if (!ctx) return VXP_ERR_ARG;
     if (mode != VXP_EDIT_SET && mode != VXP_EDIT_OCCUPANCY) return fail(ctx, VXP_ERR_ARG, "unknown edit mode %d", mode);
+    ctx->voxels_known = false;
     return ctx->cols.edit(collider_id, coords, values, n, (uint32_t)mode, ctx->stream, ctx->err);
 }
 
@@ -1968,6 +2047,7 @@ int vxp_invalidate_cache_for_body(vxp_ctx* ctx, uint32_t body_id, uint32_t* n_in
 int vxp_bodies_set(vxp_ctx* ctx, const vxp_body* b, uint32_t n) {
     if (!ctx) return VXP_ERR_ARG;
     CK(cudaStreamSynchronize(ctx->stream));
+    ctx->voxels_known = false;
     return ctx->w.set_bodies(b, n, ctx->cols, ctx->err);
 }
 

@@ -40,6 +40,7 @@ struct BlockGroup {
     // batch (the event-ordered sweeps are not compiled for this group).
     static constexpr bool kEventSweeps = false;
     static constexpr bool kDistributed = false;  // shared memory is the CTA's own
+    static constexpr bool kWideGrid = false;
     uint32_t n_pairs = 0;  // pairs of this step
     __device__ uint32_t rank() const { return threadIdx.x; }
     __device__ uint32_t size() const { return blockDim.x; }
@@ -62,6 +63,7 @@ struct GridBar {
 struct GridGroup {
     static constexpr bool kEventSweeps = true;
     static constexpr bool kDistributed = false;
+    static constexpr bool kWideGrid = true;  // a CTA can be spared for one job of a phase
     GridBar* bar;
     uint32_t* err;
     unsigned long long timeout_ns;
@@ -124,22 +126,25 @@ struct GridGroup {
     }
 };
 
-// The CTAs of one thread-block cluster (the grid is exactly one cluster).
+// The CTAs of one thread-block cluster.
 // sync() is the hardware cluster barrier (release / acquire at cluster scope,
 // about 0.2 us for 16 CTAs against about 0.8 us for one flag handed between
 // two SMs through L2).  That barrier cannot time out, so only code whose
-// every block passes the same sequence of sync() calls runs on this group:
-// the solver's colour sweeps and the store, whose barrier count depends only
-// on values every block reads before the first barrier (see
-// world_step_sweeps).  sync() never fails.
+// every block passes the same sequence of sync() calls runs on this group: a
+// step's phases, whose barrier count follows from values that every block
+// reads after the same barrier and no block writes before the next one (the
+// configuration, the pair count, the colours, the position sweeps' early
+// break).  sync() never fails.
 struct ClusterGroup {
     static constexpr bool kEventSweeps = false;
     static constexpr bool kDistributed = true;  // other CTAs' shared memory through mapa
+    static constexpr bool kWideGrid = false;
+    uint32_t cta, ncta;                         // this CTA's rank in the cluster, its CTAs
     uint32_t n_pairs = 0;                       // pairs of this step
-    __device__ uint32_t rank() const { return blockIdx.x * blockDim.x + threadIdx.x; }
-    __device__ uint32_t size() const { return gridDim.x * blockDim.x; }
-    __device__ uint32_t block() const { return blockIdx.x; }
-    __device__ uint32_t nblocks() const { return gridDim.x; }
+    __device__ uint32_t rank() const { return cta * blockDim.x + threadIdx.x; }
+    __device__ uint32_t size() const { return ncta * blockDim.x; }
+    __device__ uint32_t block() const { return cta; }
+    __device__ uint32_t nblocks() const { return ncta; }
     __device__ bool member() const { return true; }
     __device__ ClusterGroup subgroup(uint32_t) const { return *this; }
     __device__ bool sync() {
@@ -147,6 +152,12 @@ struct ClusterGroup {
         return true;
     }
 };
+__device__ __forceinline__ ClusterGroup cluster_group() {
+    uint32_t cta, ncta;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
+    return ClusterGroup{cta, ncta};
+}
 
 // ---------------------------------------------------------------------------
 // Block-level primitives (blockDim.x <= 1024, multiple of 32)
@@ -1998,7 +2009,8 @@ __device__ bool phase_probe(G& g, const WorldDev& w, const ColliderSet& cs, uint
     // nothing: the replay is a chain of dependent rounds, and other work on
     // its SM would slow it more than it is worth), or by one warp of a lone
     // CTA while its other warps start detecting at once
-    const bool replay_cta = w.cfg.use_cache && g.nblocks() > 1u && g.block() == 0u;
+    // (in a cluster too: few CTAs, few lookups)
+    const bool replay_cta = w.cfg.use_cache && G::kWideGrid && g.block() == 0u;
     if (replay_cta && w.cache_cap >= 48u &&
         (size_t)(blockDim.x >> 5) * sizeof(WarpManifold) >= cta_replay_scratch_bytes(w.cache_cap)) {
         cache_replay_cta(w, csm, reinterpret_cast<unsigned char*>(warp_sm));
