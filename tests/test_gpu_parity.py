@@ -430,3 +430,36 @@ def test_launch_chosen_by_size(vxp, boxes, colouring):
     216 boxes lie on either side of the one-CTA / cluster / grid lines."""
     sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=boxes, seed=6)
     lockstep(vxp, sc, 80, mode=-1, colouring=colouring, substeps=8).close()
+
+
+@pytest.mark.parametrize("n,mode", [(255, 0), (256, 0), (700, 0), (4738, 1)])
+def test_broad_phase_by_cells(vxp, n, mode):
+    """The pair list by cells (from 256 bodies on one CTA, past 4736 on the
+    grid) among bodies of very different sizes, at cell edges, on both sides of
+    the origin and far from it: the oracle's pairs, and the step built on them
+    gives the oracle's manifolds."""
+    sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=9 if n < 1000 else 17, seed=4)
+    b = sc.bodies[: n].copy()
+    rng = np.random.default_rng(n)
+    dyn = b["body_type"] == 2
+    k = int(dyn.sum())
+    side = 1.1 * k ** (1.0 / 3.0)
+    b["position"][dyn] = rng.uniform(-side, side, size=(k, 3)).astype(np.float32)
+    b["position"][dyn][: k // 8] = np.floor(b["position"][dyn][: k // 8])
+    b["position"][np.flatnonzero(dyn)[:5]] += np.float32(3.0e6)
+    sc.bodies = b
+    g = vxp.VoxelPhysicsSystem(substeps=8, max_pairs=64 * n)
+    g.load_scene(sc)
+    g.set_launch_mode(mode)
+    r = O.OracleWorld(substeps=8)
+    r.load_scene(sc)
+    dt = np.float32(sc.dt)
+    for s in range(2):
+        pairs = r.pairs()
+        assert g.pairs().tobytes() == pairs.tobytes(), f"step {s}: pair lists differ"
+        g.step(dt)
+        r.step(dt, pairs)
+        assert g.manifolds().tobytes() == r.manifolds().tobytes(), f"step {s}: manifolds differ"
+        assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"step {s}: bodies differ"
+    g.close()
+    r.close()

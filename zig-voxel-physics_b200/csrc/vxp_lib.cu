@@ -99,8 +99,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     if (world_step_narrow(g, w, cs, wsm, csm)) world_step_sweeps(g, w, smem_raw, smem_bytes, true);
 }
 
-// Pair source: world AABB of each body's collider (AABB.transform,
-// math.zig:686-693) inflated by margin.
 // VoxelBody.getWorldAABB (body.zig:430-435): the collider's local AABB
 // through AABB.transform (math.zig:686-693), or the position for a body
 // without a collider.
@@ -124,18 +122,6 @@ __device__ __forceinline__ void body_world_aabb(const DBody& b, const DBodyProp&
         lo = x;
         hi = x;
     }
-}
-
-__global__ void k_body_aabbs(const DBody* body, const DBodyProp* prop, uint32_t n, ColliderSet cs, float margin,
-                             float4* mn, float4* mx) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    F3 lo, hi;
-    body_world_aabb(body[i], prop[i], cs, lo, hi);
-    lo = lo - F3{margin, margin, margin};
-    hi = hi + F3{margin, margin, margin};
-    mn[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
-    mx[i] = make_float4(hi.x, hi.y, hi.z, 0.f);
 }
 
 // The body table as vxp_body records (vxp_bodies_get): one thread a body,
@@ -211,75 +197,16 @@ __global__ void k_export(const DBody* body, const DBodyProp* prop, uint32_t firs
     if (d.sleeping) d.sleeping[j] = prop[i].sleeping ? 1u : 0u;
 }
 
-// Pairs (s < t in id order) whose inflated AABBs overlap and that are not
-// both static.  One warp per row s; lanes sweep t in strides of 32 and a
-// ballot keeps the row's pairs in t order.  Pass 0 counts per row, pass 1
-// writes at the scanned offsets (clamped to cap).
-// masks (row stride mstride words, or null): the count pass keeps each row's
-// 32-column hit masks there and the write pass reads them instead of testing
-// the boxes again.
-__global__ void k_pairs(const uint2* ids, const DBodyProp* prop, uint32_t n, const float4* mn, const float4* mx,
-                        uint32_t* counts, const uint32_t* offsets, uint2* out, uint32_t cap, int pass,
-                        uint32_t* masks, uint32_t mstride) {
-    const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31;
-    if (s >= n) return;
-    const uint2 is = ids[s];
-    if (pass && masks) {
-        const uint32_t nj = (n - 1u - s + 31u) / 32u;
-        const uint32_t* mrow = masks + (size_t)s * mstride;
-        uint32_t o = offsets[s];
-        for (uint32_t jb = 0; jb < nj; jb += 32u) {
-            const uint32_t j = jb + lane;
-            uint32_t mk = j < nj ? mrow[j] : 0u;
-            const uint32_t c = (uint32_t)__popc(mk);
-            const uint32_t inc = warp_incl_scan(c);
-            uint32_t q = o + inc - c;
-            for (; mk; mk &= mk - 1u, ++q)
-                if (q < cap) out[q] = make_uint2(is.x, ids[s + 1u + 32u * j + (uint32_t)(__ffs(mk) - 1)].x);
-            o += __shfl_sync(0xffffffffu, inc, 31);
-        }
-        return;
-    }
-    const float4 a0 = mn[is.y], a1 = mx[is.y];
-    const bool si = prop[is.y].type == 0u;
-    uint32_t o = pass ? offsets[s] : 0u;
-    uint32_t cnt = 0;
-    for (uint32_t t0 = s + 1; t0 < n; t0 += 32u) {
-        const uint32_t t = t0 + lane;
-        bool hit = false;
-        uint2 it = make_uint2(0u, 0u);
-        if (t < n) {
-            it = ids[t];
-            if (!(si && prop[it.y].type == 0u)) {
-                const float4 b0 = mn[it.y], b1 = mx[it.y];
-                hit = a0.x <= b1.x && a1.x >= b0.x && a0.y <= b1.y && a1.y >= b0.y && a0.z <= b1.z && a1.z >= b0.z;
-            }
-        }
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        if (masks && lane == 0) masks[(size_t)s * mstride + (t0 - s - 1u) / 32u] = m;
-        if (pass && hit) {
-            const uint32_t slot = o + __popc(m & ((1u << lane) - 1u));
-            if (slot < cap) out[slot] = make_uint2(is.x, it.x);
-        }
-        o += __popc(m);
-        cnt += __popc(m);
-    }
-    if (!pass && lane == 0) counts[s] = cnt;
-}
-
-// Exclusive scan of counts (single block, n arbitrary); writes total to *total.
-__global__ void __launch_bounds__(1024) k_scan1(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* total) {
-    uint32_t carry = 0;
-    for (uint32_t t0 = 0; t0 < n; t0 += blockDim.x) {
-        const uint32_t i = t0 + threadIdx.x;
-        const uint32_t v = i < n ? in[i] : 0u;
-        uint32_t tile;
-        const uint32_t ex = block_excl_scan(v, &tile);
-        if (i < n) out[i] = carry + ex;
-        carry += tile;
-    }
-    if (threadIdx.x == 0) *total = carry;
+// The pair list of the bodies as they are (vxp_pairs_from_bodies): the step's
+// broad phase alone.  The counters of the last step stay, but for its own two.
+__global__ void __launch_bounds__(512, 1) k_pairs_grid(const __grid_constant__ WorldDev w,
+                                                       const __grid_constant__ ColliderSet cs, GridBar* bar,
+                                                       unsigned long long timeout_ns) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    GridGroup g{bar, &w.ctr[C_ERROR], timeout_ns, gridDim.x};
+    if (g.rank() == 0) w.ctr[C_BP_HITS] = w.ctr[C_BP_LARGE] = 0u;
+    bool overflow = false;  // the host compares the pair count with the buffers
+    phase_broadphase(g, w, cs, &overflow, smem_raw);
 }
 
 // Rebuild a manifold hash table after the manifold buffers were re-allocated.
@@ -346,6 +273,14 @@ constexpr uint32_t kBlockThreads = 512;
 // of 64^3 voxels 675 / 655 / 644 / 605 / 571 / 593 (3951 uncut), of 64 cubes
 // on one CTA 584 / 267 / 159 / 143 / 146 / 148.
 constexpr uint32_t kHeavyVoxels = 1024;
+// Worlds of at least this many bodies build their pair list by cells.  On one
+// CTA (us, every pair of rows / cells): 250 bodies 26 / 27, 512 67 / 38, 1000
+// 203 / 58, 2000 732 / 102, 4000 2925 / 245.  On the grid the rows win while
+// each warp holds one pair of them (148 x 16 x 2 rows: boxes in shared memory):
+// 4096 piled boxes 58 / 75, 8000 in columns 161 / 47; the list of 15000 boxes
+// alone 2308 / 535 with both calls of pairs().
+constexpr uint32_t kCellBodiesBlock = 256, kCellBodiesGrid = 148 * 16 * 2 + 1;
+
 // CTA sizes of the two cooperative grid kernels of a large world's step (one
 // CTA per SM each): the narrow part wants many warps to hide its memory
 // latency, the solve part wants registers for its long dependent chains.
@@ -1014,10 +949,44 @@ struct WorldBuffers {
     bool spill_rows = false;
     std::vector<uint32_t> collider_public;
     std::vector<uint32_t> moving_collider;  // per non-static body its collider's index
+    // of the moving bodies' colliders as placed (measure): the voxels of their
+    // bounds, and the broad phase's cell size
+    bool measured = false;
+    uint64_t voxels = 0;
+    float bp_cell = 1.0f;
+    // The cell: a quarter wider than the bodies' mean diagonal, so that most of
+    // their boxes, in any rotation, span at most two.
+    void measure(const ColliderStore& cols, float margin) {
+        if (measured) return;
+        uint64_t v = 0;
+        double diag = 0.0;
+        size_t k = 0;
+        for (uint32_t ci : moving_collider) {
+            if (ci >= cols.colliders.size()) continue;
+            const DCollider& d = cols.colliders[ci].d;
+            uint64_t c = 1;
+            double q = 0.0;
+            for (int a = 0; a < 3; ++a) {
+                c *= (uint64_t)std::max<int64_t>(0, (int64_t)d.max_bound[a] - d.min_bound[a]);
+                const double e = (double)d.aabb_max[a] - d.aabb_min[a];
+                q += e * e;
+            }
+            if (c == 0) continue;
+            v += c;
+            diag += std::sqrt(q);
+            ++k;
+        }
+        voxels = v;
+        const double cell = (k ? 1.25 * diag / (double)k : 1.0) + 2.0 * std::fabs((double)margin);
+        bp_cell = std::isfinite(cell) && cell > 1e-6 ? (float)cell : 1.0f;
+        measured = true;
+    }
     DBuf<DBody> body;
     DBuf<DBodyProp> prop;
     DBuf<float4> p0, qn, aabb_mn, aabb_mx;
     DBuf<uint2> ids;
+    DBuf<uint32_t> bp_start;
+    DBuf<float4> bp_mn, bp_mx;
     DBuf<uint32_t> pcount, poff, adj_off, adj_cur, bmask, bpmask;
     uint32_t bp_stride = 0, bp_rows = 0;
     // worlds of at most this many bodies keep the broad phase's hit masks
@@ -1172,6 +1141,9 @@ struct WorldBuffers {
         ok &= ids.reserve(cap) == cudaSuccess;
         ok &= pcount.reserve(cap) == cudaSuccess;
         ok &= poff.reserve(cap) == cudaSuccess;
+        ok &= bp_start.reserve(cap) == cudaSuccess;  // (cap is a power of two)
+        ok &= bp_mn.reserve(cap) == cudaSuccess;
+        ok &= bp_mx.reserve(cap) == cudaSuccess;
         ok &= adj_off.reserve((size_t)cap + 1) == cudaSuccess;
         ok &= adj_cur.reserve(cap) == cudaSuccess;
         ok &= bmask.reserve((size_t)cap * 8) == cudaSuccess;
@@ -1208,6 +1180,7 @@ struct WorldBuffers {
         std::vector<uint2> id(n);
         collider_public.resize(n);
         moving_collider.clear();
+        measured = false;
         for (uint32_t i = 0; i < n; ++i) {
             const vxp_body& s = b[i];
             if (s.body_type > 2u) {
@@ -1306,6 +1279,11 @@ struct WorldBuffers {
         w.aabb_mx = aabb_mx.p;
         w.pcount = pcount.p;
         w.poff = poff.p;
+        w.bp_start = bp_start.p;
+        w.bp_buckets = body_cap;
+        w.bp_mn = bp_mn.p;
+        w.bp_mx = bp_mx.p;
+        w.cfg.bp_cell = bp_cell;
         w.bpmask = bp_rows ? bpmask.p : nullptr;
         w.bp_stride = bp_stride;
         w.bp_rows = bp_rows;
@@ -1386,7 +1364,7 @@ struct WorldBuffers {
                clist.bytes() + part.bytes() + plog.bytes() + cp.bytes() + cm.bytes() + rk.bytes() + ev.bytes() + snap.bytes() + chunk.bytes() + cfr.bytes() +
                ckey.bytes() + cval.bytes() +
                cwriter.bytes() + scan.bytes() + ctr.bytes() + ts.bytes() + dump.bytes() + ocnt.bytes() + ocur.bytes() +
-               stat.bytes() + bpmask.bytes() + crow.bytes() + isl_parent.bytes() + isl_flag.bytes() +
+               stat.bytes() + bpmask.bytes() + bp_start.bytes() + bp_mn.bytes() + bp_mx.bytes() + crow.bytes() + isl_parent.bytes() + isl_flag.bytes() +
                isl_size.bytes() + isl_timer.bytes() + isl_keys0.bytes() + isl_keys1.bytes() + isl_state.bytes() +
                export_stage.bytes() + pub_cid.bytes() + pack.bytes();
     }
@@ -1480,7 +1458,6 @@ struct vxp_ctx {
     WorldBuffers w;
     DBuf<WorldDev> d_world;
     DBuf<GridBar> bar;
-    DBuf<uint32_t> pair_counts, pair_offsets;
     uint32_t grid_blocks = 0;
     uint32_t last_pairs = 0;
     cudaEvent_t ev_start = nullptr, ev0 = nullptr, ev1 = nullptr, ev_count = nullptr, ev_mid = nullptr,
@@ -1489,8 +1466,6 @@ struct vxp_ctx {
     uint32_t cluster_smem = 0;  // dynamic shared memory of each of its CTAs
     uint32_t step_cluster_smem = 0;  // and of a whole step's (0: not available)
     uint32_t cluster_state_cap = 0xFFFFFFFFu;  // of which the sweeps' state may use at most this
-    uint64_t voxels = 0;        // of the moving bodies' collider bounds (step_launch)
-    bool voxels_known = false;
     bool cluster_whole = false;  // the cluster also builds the constraint table and colours it
     bool last_cluster = false;
     bool last_grid = false;
@@ -1556,36 +1531,24 @@ constexpr unsigned long long kGridWaitNs = 10ull * 1000ull * 1000ull * 1000ull;
 enum class StepLaunch { kBlock, kCluster, kGrid };
 constexpr uint32_t kBlockBodies = 17, kBlockVoxels = 12 * 1024;
 constexpr uint32_t kClusterBodies = 160, kClusterVoxels = 1024 * 1024;
-StepLaunch step_launch(vxp_ctx* ctx) {
-    if (!ctx->voxels_known) {
-        // the bounds of the moving bodies' colliders, as placed
-        uint64_t v = 0;
-        for (uint32_t ci : ctx->w.moving_collider) {
-            if (ci >= ctx->cols.colliders.size()) continue;
-            const DCollider& d = ctx->cols.colliders[ci].d;
-            uint64_t c = 1;
-            for (int k = 0; k < 3; ++k) c *= (uint64_t)std::max<int64_t>(0, (int64_t)d.max_bound[k] - d.min_bound[k]);
-            v += c;
-        }
-        ctx->voxels = v;
-        ctx->voxels_known = true;
-    }
+StepLaunch step_launch(vxp_ctx* ctx, float margin) {
+    ctx->w.measure(ctx->cols, margin);
     if (ctx->use_grid >= 0) return ctx->use_grid ? StepLaunch::kGrid : StepLaunch::kBlock;
     const uint32_t n = ctx->w.n_bodies;
-    if (n <= kBlockBodies && ctx->voxels <= kBlockVoxels) return StepLaunch::kBlock;
+    if (n <= kBlockBodies && ctx->w.voxels <= kBlockVoxels) return StepLaunch::kBlock;
     const bool cluster = ctx->solver_flow == VXP_SOLVER_CLUSTER && ctx->cluster_size > 0 && ctx->step_cluster_smem > 0;
-    if (n > kClusterBodies || ctx->voxels > kClusterVoxels) return StepLaunch::kGrid;
+    if (n > kClusterBodies || ctx->w.voxels > kClusterVoxels) return StepLaunch::kGrid;
     return cluster ? StepLaunch::kCluster : n <= 64 ? StepLaunch::kBlock : StepLaunch::kGrid;
 }
 
 // Runs the step kernel.  device_pairs: the kernel builds the pair list itself.
 int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, float margin) {
     if (int rc = ctx->cols.sync(ctx->stream, ctx->err)) return rc;
-    const StepLaunch how = step_launch(ctx);
+    const StepLaunch how = step_launch(ctx, margin);
     // large colliders: room for the parts their pairs may be cut into, a part
     // per 512 voxels of bounds, and for those parts' candidates
-    if (ctx->voxels > kClusterVoxels) {
-        const size_t parts = (size_t)std::min<uint64_t>(ctx->voxels / 512u, 1u << 18);
+    if (ctx->w.voxels > kClusterVoxels) {
+        const size_t parts = (size_t)std::min<uint64_t>(ctx->w.voxels / 512u, 1u << 18);
         if (parts > ctx->w.part.n / 2u || !ctx->w.plog.p)
             if (int rc = ctx->w.ensure_parts(std::max(parts, ctx->w.part.n / 2u), true, ctx->err)) return rc;
     }
@@ -1597,6 +1560,7 @@ int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, floa
     if (!grid && !one_cluster) w.cfg.block_smem = (uint32_t)smem;
     w.cfg.flow_smem_chunks = grid ? flow_chunks(solve_smem()) : 0u;
     w.cfg.heavy_voxels = ctx->heavy_voxels;
+    w.cfg.bp_cell_bodies = grid ? kCellBodiesGrid : kCellBodiesBlock;
     w.cfg.count_bricks = ctx->count_bricks ? 1u : 0u;
     w.cfg.owner_groups = cluster ? ctx->cluster_size : one_cluster ? ctx->cluster_size : 1u;
     if (ctx->record_substeps) {
@@ -1667,32 +1631,28 @@ int compute_device_pairs(vxp_ctx* ctx, float margin, uint32_t* n_out) {
         *n_out = 0;
         return VXP_OK;
     }
-    if (ctx->pair_counts.reserve(w.body_cap) != cudaSuccess || ctx->pair_offsets.reserve(w.body_cap) != cudaSuccess)
-        return fail(ctx, VXP_ERR_OOM, "pair scratch");
-    const uint32_t tb = 256, nb = (n + tb - 1) / tb;
-    const uint32_t wb = (n * 32u + tb - 1) / tb;
-    k_body_aabbs<<<nb, tb, 0, ctx->stream>>>(w.body.p, w.prop.p, n, cs, margin, w.aabb_mn.p, w.aabb_mx.p);
-    uint32_t* masks = n <= w.bp_rows ? w.bpmask.p : nullptr;
-    k_pairs<<<wb, tb, 0, ctx->stream>>>(w.ids.p, w.prop.p, n, w.aabb_mn.p, w.aabb_mx.p, ctx->pair_counts.p, nullptr,
-                                        nullptr, 0, 0, masks, w.bp_stride);
-    k_scan1<<<1, 1024, 0, ctx->stream>>>(ctx->pair_counts.p, ctx->pair_offsets.p, n, w.n_pairs_dev.p);
-    CK(cudaGetLastError());
-    // the write pass runs at once into the pair buffers as they are (it
-    // writes no pair past their capacity); only when the total does not fit
-    // are they grown and the pass run again
-    auto write_pass = [&]() {
-        k_pairs<<<wb, tb, 0, ctx->stream>>>(w.ids.p, w.prop.p, n, w.aabb_mn.p, w.aabb_mx.p, nullptr,
-                                            ctx->pair_offsets.p, w.pairs.p, w.pair_cap, 1, masks, w.bp_stride);
-        return cudaGetLastError();
-    };
-    const bool early = w.pairs.p != nullptr && w.pair_cap > 0u;
-    if (early) CK(write_pass());
+    if (w.pair_cap == 0u)
+        if (int rc = w.ensure_pairs(1024, ctx->err)) return rc;
     uint32_t total = 0;
-    CK(cudaMemcpyAsync(&total, w.n_pairs_dev.p, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (!early || total > w.pair_cap) {
+    for (int attempt = 0;; ++attempt) {
+        w.measure(ctx->cols, margin);
+        WorldDev wd = w.make(ctx->cfg, 0.0f, 0u, ctx->solver_div, true, margin, 0u);
+        wd.ts = nullptr;  // the last step's times stay
+        wd.cfg.bp_cell_bodies = kCellBodiesGrid;
+        GridBar* bp = ctx->bar.p;
+        const unsigned long long timeout = ctx->wait_limit_ns ? ctx->wait_limit_ns : kGridWaitNs;
+        void* args[] = {(void*)&wd, (void*)&cs, (void*)&bp, (void*)&timeout};
+        CK(cudaMemsetAsync(ctx->bar.p, 0, sizeof(GridBar), ctx->stream));
+        CK(cudaLaunchCooperativeKernel((const void*)k_pairs_grid, dim3(ctx->grid_blocks), dim3(kGridThreads), args,
+                                       grid_smem(wd.cache_cap), ctx->stream));
+        uint32_t err = 0;
+        CK(cudaMemcpyAsync(&total, w.n_pairs_dev.p, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(&err, w.ctr.p + C_ERROR, sizeof(err), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (err & ERR_TIMEOUT) return w.take_error(ctx->stream, ctx->err);
+        if (total <= w.pair_cap || attempt) break;
+        // the list did not fit: grow and run again
         if (int rc = w.ensure_pairs(total, ctx->err)) return rc;
-        CK(write_pass());
     }
     *n_out = total;
     return VXP_OK;
@@ -1899,6 +1859,8 @@ static int set_kernel_smem(uint32_t cache_cap) {
                              (int)block_smem(kMaxCacheSmem)) != cudaSuccess ||
         cudaFuncSetAttribute(k_step_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)grid_smem(cache_cap)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_pairs_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)grid_smem(cache_cap)) != cudaSuccess ||
         cudaFuncSetAttribute(k_solve_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem()) !=
             cudaSuccess)
         return VXP_ERR_CUDA;
@@ -2011,7 +1973,7 @@ int vxp_last_error(const vxp_ctx* ctx, char* buf, size_t n) {
 int vxp_collider_upload(vxp_ctx* ctx, uint32_t collider_id, float voxel_size, const vxp_brick* bricks,
                         uint32_t n_bricks) {
     if (!ctx) return VXP_ERR_ARG;
-    ctx->voxels_known = false;
+    ctx->w.measured = false;
     return ctx->cols.upload(collider_id, voxel_size, bricks, n_bricks, ctx->err);
 }
 
@@ -2019,7 +1981,7 @@ int vxp_collider_edit(vxp_ctx* ctx, uint32_t collider_id, const int32_t* coords,
                       int mode) {
     if (!ctx) return VXP_ERR_ARG;
     if (mode != VXP_EDIT_SET && mode != VXP_EDIT_OCCUPANCY) return fail(ctx, VXP_ERR_ARG, "unknown edit mode %d", mode);
-    ctx->voxels_known = false;
+    ctx->w.measured = false;
     return ctx->cols.edit(collider_id, coords, values, n, (uint32_t)mode, ctx->stream, ctx->err);
 }
 
@@ -2047,7 +2009,7 @@ int vxp_invalidate_cache_for_body(vxp_ctx* ctx, uint32_t body_id, uint32_t* n_in
 int vxp_bodies_set(vxp_ctx* ctx, const vxp_body* b, uint32_t n) {
     if (!ctx) return VXP_ERR_ARG;
     CK(cudaStreamSynchronize(ctx->stream));
-    ctx->voxels_known = false;
+    ctx->w.measured = false;
     return ctx->w.set_bodies(b, n, ctx->cols, ctx->err);
 }
 
@@ -2641,7 +2603,9 @@ int batch_prepare(vxp_batch* bt, float dt) {
         std::vector<WorldDev> wd(ord.size());
         for (size_t i = 0; i < ord.size(); ++i)
         {
+            bt->slots[ord[i]]->measure(bt->cols, bt->margin);
             wd[i] = bt->slots[ord[i]]->make(bt->cfg, dt, PH_STEP, 128, true, bt->margin, 0u);
+            wd[i].cfg.bp_cell_bodies = kCellBodiesBlock;
             wd[i].cfg.block_smem = (uint32_t)block_smem(bt->cache_cap);
         }
         if (bt->d_worlds.reserve(std::max<size_t>(wd.size(), 1)) != cudaSuccess ||

@@ -579,6 +579,128 @@ __device__ bool phase_begin(G& g, const WorldDev& w, bool skip_test, bool* skipp
 // sweep kept (worlds with mask room), else by sweeping again.  *overflow:
 // the list does not fit pair_cap (nothing is written; the host grows the
 // buffers).
+// The same pair list through a grid of cells, for worlds where testing every
+// pair of rows costs more (it grows with the square of the bodies).
+//
+// A cell is cfg.bp_cell wide; a body is small if its box spans at most two
+// cells on every axis.  Two small bodies whose boxes overlap have the cells of
+// their lower corners at most one apart on every axis: the one with the lower
+// corner reaches the other's corner with its own upper end (the cell of a
+// coordinate is a monotone function of it, so this holds for the rounded
+// values too).  So each small body is tested against those in its own cell
+// and in the thirteen of its 26 neighbours that come after it, which finds
+// every pair once; a body that is not small is tested against all.  Cells are
+// hashed to buckets, the boxes sorted by bucket.
+// The hits are then put in (row, column) order: counted by row, scanned,
+// dealt to the rows' places, and placed by their rank among their row's.
+__device__ __forceinline__ int32_t bp_cell_of(float x, float inv) {
+    return (int32_t)fminf(fmaxf(floorf(x * inv), -1048576.0f), 1048576.0f);
+}
+__device__ __forceinline__ uint32_t bp_bucket(I3 c, uint32_t mask) {
+    uint32_t h = (uint32_t)c.x * 0x8DA6B343u ^ (uint32_t)c.y * 0xD8163841u ^ (uint32_t)c.z * 0xCB1AB31Fu;
+    h ^= h >> 15;
+    return h & mask;
+}
+__device__ __forceinline__ bool bp_overlap(float4 a0, float4 a1, float4 b0, float4 b1) {
+    return !(a0.w != 0.f && b0.w != 0.f) && a0.x <= b1.x && a1.x >= b0.x && a0.y <= b1.y && a1.y >= b0.y &&
+           a0.z <= b1.z && a1.z >= b0.z;
+}
+template <class G>
+__device__ bool broadphase_cells(G& g, const WorldDev& w, bool* overflow) {
+    const uint32_t N = w.n_bodies, T = w.bp_buckets;
+    const float inv = 1.0f / w.cfg.bp_cell;
+    uint2* hits = reinterpret_cast<uint2*>(w.adj);  // (row, column); free until the constraint table
+    uint32_t* cols = w.flag;                        // the columns, row by row
+    uint32_t* large = w.bmask;                      // rows that are not small
+    for (uint32_t i = g.rank(); i < T; i += g.size()) w.bp_start[i] = 0u;
+    for (uint32_t i = g.rank(); i < N; i += g.size()) {
+        w.pcount[i] = 0u;
+        w.adj_cur[i] = 0u;
+    }
+    if (!g.sync()) return false;  // (the boxes are in place too)
+    auto cell = [&](float4 p) { return I3{bp_cell_of(p.x, inv), bp_cell_of(p.y, inv), bp_cell_of(p.z, inv)}; };
+    for (uint32_t s = g.rank(); s < N; s += g.size()) {
+        const I3 a = cell(w.aabb_mn[s]), b = cell(w.aabb_mx[s]);
+        if (b.x - a.x <= 1 && b.y - a.y <= 1 && b.z - a.z <= 1) {
+            const uint32_t k = bp_bucket(a, T - 1u);
+            w.poff[s] = k;
+            atomicAdd(&w.bp_start[k], 1u);
+        } else {
+            w.poff[s] = 0xFFFFFFFFu;
+            large[atomicAdd(&w.ctr[C_BP_LARGE], 1u)] = s;
+        }
+    }
+    if (!g.sync()) return false;
+    uint32_t tot;
+    if (!group_scan(
+            g, T, [&](uint32_t i) { return w.bp_start[i]; }, [&](uint32_t i, uint32_t pre) { w.bp_start[i] = pre; },
+            w.scan, &tot))
+        return false;
+    // boxes sorted by bucket; afterwards bucket k ends at bp_start[k]
+    for (uint32_t s = g.rank(); s < N; s += g.size()) {
+        const uint32_t k = w.poff[s];
+        if (k == 0xFFFFFFFFu) continue;
+        const uint32_t q = atomicAdd(&w.bp_start[k], 1u);
+        const float4 mx = w.aabb_mx[s];
+        w.bp_mn[q] = w.aabb_mn[s];
+        w.bp_mx[q] = make_float4(mx.x, mx.y, mx.z, __uint_as_float(s));
+    }
+    if (!g.sync()) return false;
+    const uint32_t n_large = *(volatile uint32_t*)&w.ctr[C_BP_LARGE], n_small = N - n_large;
+    auto hit = [&](uint32_t r, uint32_t t) {
+        const uint32_t lo = min(r, t), hi = max(r, t);
+        const uint32_t at = atomicAdd(&w.ctr[C_BP_HITS], 1u);
+        if (at < w.pair_cap) hits[at] = make_uint2(lo, hi);
+        atomicAdd(&w.pcount[lo], 1u);
+    };
+    // (a body's own cell, then the thirteen after it, in turn over the
+    // threads: a thread per body and cell)
+    for (uint32_t x = g.rank(); x < n_small * 14u; x += g.size()) {
+        const uint32_t q = x / 14u, o = x - q * 14u + 13u;  // 13: own cell, of the 27 in x, y, z order
+        const float4 a0 = w.bp_mn[q], a1 = w.bp_mx[q];
+        const I3 c = cell(a0);
+        const I3 d{c.x + (int32_t)(o / 9u) - 1, c.y + (int32_t)(o / 3u % 3u) - 1, c.z + (int32_t)(o % 3u) - 1};
+        const uint32_t k = bp_bucket(d, T - 1u);
+        const uint32_t end = w.bp_start[k];
+        for (uint32_t t = o == 13u ? q + 1u : k ? w.bp_start[k - 1u] : 0u; t < end; ++t) {
+            const float4 b0 = w.bp_mn[t], b1 = w.bp_mx[t];
+            if (!bp_overlap(a0, a1, b0, b1)) continue;
+            const I3 e = cell(b0);
+            if (e.x == d.x && e.y == d.y && e.z == d.z) hit(__float_as_uint(a1.w), __float_as_uint(b1.w));
+        }
+    }
+    for (unsigned long long x = g.rank(); x < (unsigned long long)n_large * N; x += g.size()) {
+        const uint32_t s = large[x / N], t = (uint32_t)(x % N);
+        if (t == s || (w.poff[t] == 0xFFFFFFFFu && t < s)) continue;
+        if (bp_overlap(w.aabb_mn[s], w.aabb_mx[s], w.aabb_mn[t], w.aabb_mx[t])) hit(s, t);
+    }
+    if (!g.sync()) return false;
+    if (g.rank() == 0 && w.ts) w.ts[TS_BP_COUNT] = global_ns();
+    uint32_t total = 0;
+    if (!group_scan(
+            g, N, [&](uint32_t i) { return w.pcount[i]; }, [&](uint32_t i, uint32_t pre) { w.poff[i] = pre; }, w.scan,
+            &total))
+        return false;
+    if (g.rank() == 0 && w.ts) w.ts[TS_BP_SCAN] = global_ns();
+    *overflow = total > w.pair_cap;
+    g.n_pairs = total;
+    if (g.rank() == 0) *w.n_pairs_dev = total;
+    if (*overflow) return true;
+    for (uint32_t i = g.rank(); i < total; i += g.size()) {
+        const uint2 h = hits[i];
+        cols[w.poff[h.x] + atomicAdd(&w.adj_cur[h.x], 1u)] = h.y;
+    }
+    if (!g.sync()) return false;
+    for (uint32_t i = g.rank(); i < total; i += g.size()) {
+        const uint2 h = hits[i];
+        const uint32_t off = w.poff[h.x], n = w.pcount[h.x];
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < n; ++j) rank += cols[off + j] < h.y ? 1u : 0u;
+        w.pairs[off + rank] = make_uint2(w.ids[h.x].x, w.ids[h.y].x);
+    }
+    return g.sync();
+}
+
 template <class G>
 __device__ bool phase_broadphase(G& g, const WorldDev& w, const ColliderSet& cs, bool* overflow, unsigned char* smem) {
     const uint32_t N = w.n_bodies;
@@ -613,6 +735,7 @@ __device__ bool phase_broadphase(G& g, const WorldDev& w, const ColliderSet& cs,
         w.aabb_mn[s] = make_float4(lo.x, lo.y, lo.z, w.prop[i].type == 0u ? 1.f : 0.f);
         w.aabb_mx[s] = make_float4(hi.x, hi.y, hi.z, 0.f);
     }
+    if (w.bp_buckets && N >= w.cfg.bp_cell_bodies) return broadphase_cells(g, w, overflow);
     if (!g.sync()) return false;
     const uint32_t lane = threadIdx.x & 31, wid = g.rank() >> 5, nw = g.size() >> 5;
     const bool masks = w.bpmask != nullptr && N <= w.bp_rows;

@@ -161,6 +161,8 @@ struct StepCfg {
     uint32_t solver_div;      // grid launch: solver blocks = manifolds / solver_div
     uint32_t device_pairs;    // 1: the step builds its own pair list (phase_broadphase)
     float margin;             // AABB inflation of that pair list
+    float bp_cell;            // cell size of that pair list's grid
+    uint32_t bp_cell_bodies;  // worlds of at least this many bodies use it
     uint32_t solver_flow;     // 1: sweeps ordered by per-body event counters, 0: colour barriers
     uint32_t flow_smem_chunks;  // constraint chunks per block the launch's shared memory holds
     uint32_t record_substeps;   // 1: write every body's state after each substep to subrec
@@ -203,6 +205,8 @@ enum : uint32_t {
     C_NHEAVY,        // parts of cut pairs listed (w.part)
     C_NLIGHT,        // other pairs to probe (w.colour during the probe)
     C_NLOG,          // candidates in plog
+    C_BP_HITS,       // broad phase by cells: pairs found,
+    C_BP_LARGE,      // bodies tested against all
     C_CONS_M,        // constraint manifolds of the step (solve part split in two kernels)
     C_CONS_NCOL,     // their colours
     C_SWEEP,         // how the cluster sweeps ran (SWEEP_*)
@@ -266,6 +270,10 @@ struct WorldDev {
     uint32_t* bpmask;             // broad-phase hit masks: row s, 32 columns from s + 1 + 32 j at s * bp_stride + j
     uint32_t bp_stride, bp_rows;  // words per row; rows it holds (0: no masks, the sweep runs twice)
     uint32_t* poff;               // their exclusive prefix
+    // the broad phase's cell grid: bucket ends (a power of two), boxes sorted by bucket
+    uint32_t* bp_start;
+    uint32_t bp_buckets;
+    float4 *bp_mn, *bp_mx;
     // pairs
     uint2* pairs;                 // (body_a id, body_b id)
     PairInfo* pinfo;

@@ -59,7 +59,7 @@ def estimate_bytes(n_bodies: int, cache_entries: int = 1024) -> int:
     # + two island key buffers and four narrow-phase parts (16 B each) per pair slot
     per_pair = 64 + 8 + 88 + 2 * 376 + 4 * 6 + 24 + 4 * 31 * 4 + 16 + 8 + 2 * 16 * 2 + 2 * 8
     # + the island arrays, the public collider id and the packed readback record
-    per_body = 112 + 64 + 4 * 16 + 8 + 4 * 4 + 4 * 10 + 16 + 4 + 128
+    per_body = 36 + 112 + 64 + 4 * 16 + 8 + 4 * 4 + 4 * 10 + 16 + 4 + 128
     masks = bcap * ((bcap + 31) // 32) * 4 if bcap <= 8192 else 0
     return (cap * per_pair + max(64, n_bodies) * per_body + masks + cache_entries * (24 + 368 + 4) +
             (64 << 10))
