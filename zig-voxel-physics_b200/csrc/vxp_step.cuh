@@ -2554,8 +2554,12 @@ __device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_
     }
     for (uint32_t i = g.rank(); i <= N; i += g.size()) {
         w.adj_off[i] = 0u;
-        if (i < N) w.adj_cur[i] = 0u;
+        if (i < N) {
+            w.adj_cur[i] = 0u;
+            w.ev[i] = 0u;
+        }
     }
+    if (g.rank() < kMaxOwnerGroups) w.ocnt[kOwnerBodies + g.rank()] = 0u;
     const uint32_t NG = w.cfg.owner_groups > 1u ? min(w.cfg.owner_groups, kMaxOwnerGroups) : 1u;
     for (uint32_t i = g.rank(); i < 257u; i += g.size()) {
         w.colour_cnt[i] = 0u;
@@ -2588,7 +2592,9 @@ __device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_
     if (g.rank() == 0) w.ctr[C_CONSTRAINTS] = M;
 
     // 2. adjacency of the bodies the solver writes (dynamic, awake): the
-    // constraints of each, for the colouring and for event-ordered sweeps
+    // constraints of each, for the colouring and for event-ordered sweeps;
+    // and the bodies the constraints name, for the sweeps' shared memory
+    const bool static_copies = w.n_static <= kMaxStaticReplicas;
     uint32_t kin = 0;
     for (uint32_t k = g.rank(); k < M; k += g.size()) {
         const PairInfo& pi = w.pinfo[w.cons[k]];
@@ -2596,6 +2602,10 @@ __device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_
         const DBodyProp& pb = w.prop[pi.ib];
         if (writable(pa)) atomicAdd(&w.adj_off[pi.ia], 1u);
         if (writable(pb)) atomicAdd(&w.adj_off[pi.ib], 1u);
+        if ((pa.type != 0u || !static_copies) && atomicExch(&w.ev[pi.ia], 1u) == 0u)
+            atomicAdd(&w.ocnt[kOwnerBodies + pi.ia % NG], 1u);
+        if ((pb.type != 0u || !static_copies) && atomicExch(&w.ev[pi.ib], 1u) == 0u)
+            atomicAdd(&w.ocnt[kOwnerBodies + pi.ib % NG], 1u);
         kin += ((pa.type == 1u && !pa.sleeping) || (pb.type == 1u && !pb.sleeping)) ? 1u : 0u;
     }
     kin = warp_sum(kin);
@@ -3999,8 +4009,8 @@ __device__ bool phase_solve_flow(G& g, const WorldDev& w, float* fsm, uint32_t M
 // ---------------------------------------------------------------------------
 // ContactSolver.solve with a barrier after every colour batch, as in
 // phase_solve, with the state the sweeps pass from SM to SM held in the
-// cluster's shared memory instead of L2: body i lives in CTA i % C (slot
-// i / C) and is read and written by the other CTAs through distributed
+// cluster's shared memory instead of L2: a body i that a constraint names
+// lives in CTA i % C and is read and written by the other CTAs through distributed
 // shared memory.  Each CTA prepares and solves its own manifolds with their
 // velocity-sweep fields (CP_NVEL per point; tangent2 is recomputed from the
 // normal and tangent1) in its shared memory: with the packing grouped by
@@ -4030,10 +4040,9 @@ __device__ __forceinline__ T* group_map(T* p, uint32_t rank) {
     else return p;
 }
 
-constexpr uint32_t kMaxStaticReplicas = 32;
-
 struct ClusterSolveSmem {
     DBody* body;     // bcap records
+    uint32_t* idx;   // their body indices
     DBody* rep;      // copies of the static bodies (nrep)
     uint32_t* stat;  // their body indices, ascending
     uint4* man;      // per local slot: body a, body b, points, flags
@@ -4052,7 +4061,7 @@ enum : uint32_t { CM_WA = 1u, CM_WB = 2u, CM_STATIC = 4u, CM_BAD = 8u, CM_RA = 1
 // slots and pcap points.
 __device__ __forceinline__ size_t cluster_smem_bytes(uint32_t bcap, uint32_t nrep, uint32_t scap, uint32_t pcap,
                                                      uint32_t ncol) {
-    return (size_t)(bcap + nrep) * sizeof(DBody) +
+    return (size_t)(bcap + nrep) * sizeof(DBody) + (size_t)bcap * sizeof(uint32_t) +
            (size_t)scap * (sizeof(uint4) + sizeof(float2) + 2u * sizeof(uint32_t)) +
            (size_t)pcap * CP_NVEL * sizeof(float) + (size_t)(ncol + 1u) * sizeof(uint32_t) +
            (size_t)kMaxStaticReplicas * sizeof(uint32_t);
@@ -4080,11 +4089,11 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
     // block at once from the packing's counts (one or two loads a thread,
     // then shared atomics; the same values, so the same verdicts, in every
     // block): [0] slots by owner, [1] slots round-robin, [2] points by owner,
-    // [3] points round-robin
-    __shared__ uint32_t s_tally[4][kMaxOwnerGroups];
+    // [3] points round-robin, [4] bodies that a constraint names
+    __shared__ uint32_t s_tally[5][kMaxOwnerGroups];
     __shared__ int s_bad;
     if (C > kMaxOwnerGroups) return false;
-    for (uint32_t x = t; x < 4u * kMaxOwnerGroups; x += T) (&s_tally[0][0])[x] = 0u;
+    for (uint32_t x = t; x < 5u * kMaxOwnerGroups; x += T) (&s_tally[0][0])[x] = 0u;
     if (t == 0) s_bad = 0;
     __syncthreads();
     const bool owner_ok = by_owner;
@@ -4100,6 +4109,7 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
             if (o) atomicAdd(&s_tally[0][cta], o);
         }
     }
+    if (t < C) s_tally[4][t] = w.ocnt[kOwnerBodies + t];
     const bool tallied = C > 1u && w.cfg.owner_groups == C && C <= kMaxOwnerGroups;
     if (tallied && t < C) {
         s_tally[2][t] = w.ocnt[kOwnerPoints + t];
@@ -4110,7 +4120,16 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
     // the most slots any CTA holds (the same verdict in every block)
     uint32_t need = 0;
     ClusterSolveSmem sm;
+    // Only the bodies that a constraint names live in shared memory; the others
+    // take their substeps in one go before the sweeps (a world of columns in
+    // free fall: 1900 bodies, of which a hundred are in contact).  With the
+    // substep record on, every body does.
+    const bool compact = !cf.record_substeps && (C == 1u ? w.cfg.owner_groups <= 1u : w.cfg.owner_groups == C);
     sm.bcap = (N + C - 1u) / C;
+    if (compact) {
+        sm.bcap = 1u;
+        for (uint32_t cta = 0; cta < C; ++cta) sm.bcap = max(sm.bcap, s_tally[4][cta]);
+    }
     sm.nrep = w.n_static <= kMaxStaticReplicas ? w.n_static : 0u;
     // point rows that do not fit in shared memory may go to w.crow: a CTA's
     // last slots (the point offsets are a prefix in slot order, so once a
@@ -4168,6 +4187,8 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
         p += (size_t)sm.scap * sizeof(uint32_t);
         sm.base = reinterpret_cast<uint32_t*>(p);
         p += (size_t)(ncol + 1u) * sizeof(uint32_t);
+        sm.idx = reinterpret_cast<uint32_t*>(p);
+        p += (size_t)sm.bcap * sizeof(uint32_t);
         sm.stat = reinterpret_cast<uint32_t*>(p);
     }
     // this CTA's first slot per colour (ncol <= 256 <= T): a block scan
@@ -4177,17 +4198,47 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
         if (t < ncol) sm.base[t] = ex;
         if (t == 0) sm.base[ncol] = total;
     }
-    // this CTA's bodies, and a copy of every static body
-    for (uint32_t s = t; s < sm.bcap; s += T) {
-        const uint32_t i = s * C + k;
-        if (i < N) sm.body[s] = w.body[i];
+    const float h = cf.dt / (float)cf.substeps;
+    const F3 grav{cf.gravity[0], cf.gravity[1], cf.gravity[2]};
+    // this CTA's bodies (body i: CTA i % C), their slots to w.ev for the
+    // other CTAs, and a copy of every static body
+    uint32_t nbody = 0;
+    {
+        const uint32_t Q = (N + C - 1u) / C;
+        for (uint32_t q0 = 0; q0 < Q; q0 += T) {
+            const uint32_t i = (q0 + t) * C + k;
+            const bool here = q0 + t < Q && i < N;
+            const bool named = here && (!compact || w.ev[i] != 0u);
+            uint32_t tile = 0;
+            const uint32_t slot = nbody + block_excl_scan(named ? 1u : 0u, &tile);
+            nbody += tile;
+            if (named && slot < sm.bcap) {
+                sm.idx[slot] = i;
+                sm.body[slot] = w.body[i];
+                w.ev[i] = slot;
+            } else if (here && !named) {
+                const DBodyProp pr = w.prop[i];
+                if (pr.type != 0u && !pr.sleeping) {
+                    DBody b = w.body[i];
+                    for (uint32_t s = 0; s < cf.substeps; ++s) {
+                        if (pr.type == 2u) body_gravity(b.v, b.w, pr, grav, h);
+                        body_integrate(b, pr, h, cf.disable_rotation != 0u);
+                    }
+                    w.body[i] = b;
+                }
+            }
+        }
+        if (nbody > sm.bcap) {  // never with the packing's own tallies
+            nbody = sm.bcap;
+            if (t == 0) atomicOr(&w.ctr[C_ERROR], ERR_BOUNDS);
+        }
     }
     for (uint32_t r = t; r < sm.nrep; r += T) {
         const uint32_t i = w.stat_idx[r];
         sm.stat[r] = i < N ? i : 0xFFFFFFFFu;
         if (i < N) sm.rep[r] = w.body[i];
     }
-    __syncthreads();
+    g.sync();  // every block's slots are in w.ev
     // the static copy holding body i, or -1
     auto rep_of = [&](uint32_t i) -> int32_t {
         uint32_t lo = 0, hi = sm.nrep;
@@ -4229,6 +4280,15 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
                     const int32_t r = rep_of(mv.y);
                     if (r >= 0) fl |= CM_RB | ((uint32_t)r << 16);
                 }
+                // from here on a body is its CTA (high byte) and slot
+                const uint32_t sa = (fl & CM_RA) ? 0u : w.ev[mv.x], sb = (fl & CM_RB) ? 0u : w.ev[mv.y];
+                if (sa >= sm.bcap || sb >= sm.bcap) {
+                    atomicOr(&w.ctr[C_ERROR], ERR_BOUNDS);
+                    mv.z = 0u;
+                    fl = CM_BAD;
+                }
+                mv.x = ((mv.x % C) << 24) | min(sa, sm.bcap - 1u);
+                mv.y = ((mv.y % C) << 24) | min(sb, sm.bcap - 1u);
                 mv.w = fl;
             }
             sm.man[slot] = mv;
@@ -4297,24 +4357,17 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
     g.sync();  // every block's bodies are in place (and every block has started)
     if (g.rank() == 0 && w.ts) w.ts[TS_SW_SETUP] = global_ns();
     const SolveFlags sf = solve_flags(cf);
-    const float h = cf.dt / (float)cf.substeps;
     const Soft soft = soft_params(cf.hertz, cf.damping_ratio, h);
     const float hinv = h > kEpsilon ? 1.0f / h : 0.0f;
     const Soft hard{0.f, 1.f, 1.f};
-    const F3 grav{cf.gravity[0], cf.gravity[1], cf.gravity[2]};
     const bool has = M > 0u;
     const uint32_t nslot = sm.base[ncol];
-    // body i's home CTA and its slot there (shift and mask for the usual
-    // power-of-two cluster)
-    const uint32_t csh = (C & (C - 1u)) == 0u ? (uint32_t)(__ffs(C) - 1) : 32u;
-    auto home = [&](uint32_t i) { return csh < 32u ? i & (C - 1u) : i % C; };
-    auto home_slot = [&](uint32_t i) { return csh < 32u ? i >> csh : i / C; };
     // body a (or b) of a manifold: its static copy here, else its home CTA's record
     auto body_a = [&](const uint4& mv) {
-        return (mv.w & CM_RA) ? sm.rep + ((mv.w >> 8) & 0xFFu) : group_map<G>(sm.body + home_slot(mv.x), home(mv.x));
+        return (mv.w & CM_RA) ? sm.rep + ((mv.w >> 8) & 0xFFu) : group_map<G>(sm.body + (mv.x & 0xFFFFFFu), mv.x >> 24);
     };
     auto body_b = [&](const uint4& mv) {
-        return (mv.w & CM_RB) ? sm.rep + ((mv.w >> 16) & 0xFFu) : group_map<G>(sm.body + home_slot(mv.y), home(mv.y));
+        return (mv.w & CM_RB) ? sm.rep + ((mv.w >> 16) & 0xFFu) : group_map<G>(sm.body + (mv.y & 0xFFFFFFu), mv.y >> 24);
     };
     // one manifold of a velocity-type sweep: 0 warm start, 1 velocity, 2 relax
     auto vel_item = [&](uint32_t slot, uint32_t kind) {
@@ -4349,9 +4402,8 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
     };
     for (uint32_t s = 0; s < cf.substeps; ++s) {
         // applyGravity (solver.zig:564-605)
-        for (uint32_t q = t; q < sm.bcap; q += T) {
-            const uint32_t i = q * C + k;
-            if (i >= N) break;
+        for (uint32_t q = t; q < nbody; q += T) {
+            const uint32_t i = sm.idx[q];
             const DBodyProp& pr = w.prop[i];
             if (!(pr.type == 2u && pr.sleeping == 0u)) continue;
             DBody& b = sm.body[q];
@@ -4381,9 +4433,8 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
             for (uint32_t vi = 0; vi < cf.vel_iters; ++vi) sweep(1u);
         }
         // integratePositions (solver.zig:841-845, 341-356)
-        for (uint32_t q = t; q < sm.bcap; q += T) {
-            const uint32_t i = q * C + k;
-            if (i >= N) break;
+        for (uint32_t q = t; q < nbody; q += T) {
+            const uint32_t i = sm.idx[q];
             const DBodyProp& pr = w.prop[i];
             if (pr.type == 0u || pr.sleeping) continue;
             DBody b = sm.body[q];
@@ -4394,9 +4445,8 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
         if (has) sweep(2u);
         // test hook: every body's state after this substep
         if (cf.record_substeps && w.subrec) {
-            for (uint32_t q = t; q < sm.bcap; q += T) {
-                const uint32_t i = q * C + k;
-                if (i >= N) break;
+            for (uint32_t q = t; q < nbody; q += T) {
+                const uint32_t i = sm.idx[q];
                 const DBody b = sm.body[q];
                 float* r = w.subrec + ((size_t)s * N + i) * 13u;
                 r[0] = b.p.x; r[1] = b.p.y; r[2] = b.p.z;
@@ -4483,9 +4533,8 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
     if (g.rank() == 0 && w.ts) w.ts[TS_SW_POSITION] = global_ns();
     // bodies back to the world, impulses and masses back to the packed rows
     // (storeImpulses reads them)
-    for (uint32_t q = t; q < sm.bcap; q += T) {
-        const uint32_t i = q * C + k;
-        if (i >= N) break;
+    for (uint32_t q = t; q < nbody; q += T) {
+        const uint32_t i = sm.idx[q];
         if (w.prop[i].type != 0u) w.body[i] = sm.body[q];
     }
     for (uint32_t slot = pos_rows ? nslot : t; slot < nslot; slot += T) {  // done above when pos_rows

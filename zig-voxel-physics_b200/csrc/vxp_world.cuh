@@ -315,7 +315,7 @@ struct WorldDev {
     // per body the number of sweep events applied so far; per body the state
     // that prepare reads (after gravity), two substeps deep
     uint4* rk;
-    uint32_t* ev;
+    uint32_t* ev;                 // (the cluster sweeps: whether a constraint names the body, then its slot)
     DBody* snap;
     uint2* chunk;                 // [first, end) positions of <= 32 manifolds of one colour
     float* subrec;                // per substep and body: position, rotation, v, w (13 floats)
@@ -356,6 +356,11 @@ constexpr uint32_t kMaxOwnerGroups = 16;
 // After the (colour, owner) offsets in ocnt: the points each sweep CTA holds
 // by owner (kMaxOwnerGroups), then dealt round-robin (kMaxOwnerGroups).
 constexpr uint32_t kOwnerPoints = 256u * kMaxOwnerGroups + 1u;
+// Then the bodies of each sweep CTA that a constraint names, static bodies
+// with a copy in every CTA excepted (kMaxOwnerGroups).
+constexpr uint32_t kOwnerBodies = kOwnerPoints + 2u * kMaxOwnerGroups;
+// Static bodies the sweeps copy into every CTA, if there are no more.
+constexpr uint32_t kMaxStaticReplicas = 32;
 
 // Packed constraint-point fields (ConstraintPoint, solver.zig:122-168).  The
 // first CP_NVEL are the ones the velocity-type sweeps (warm start, velocity,
