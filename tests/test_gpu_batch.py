@@ -183,3 +183,28 @@ def test_reused_slot_matches_new_slot(vxp):
     got["collider_id"] -= 5000
     assert got.tobytes() == run_alone(vxp, scenes[2], 10, dt).tobytes()
     b.close()
+
+
+def test_rows_spilled_from_a_one_cta_world(vxp):
+    """A settled heap whose point rows do not fit a one-CTA world's shared
+    memory: the rest spills, and the world equals the oracle's bit for bit."""
+    sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=8, seed=12)
+    dt = np.float32(sc.dt)
+    s = vxp.VoxelPhysicsSystem(substeps=8, max_pairs=1 << 14)
+    s.load_scene(sc)
+    for _ in range(240):
+        s.step(dt)
+    sc.bodies = s.get_bodies()
+    s.close()
+    b = vxp.VoxelWorldBatch(1, substeps=8)
+    b.load_scene(0, sc, 0)
+    r = O.OracleWorld(substeps=8)
+    r.load_scene(sc)
+    for _ in range(3):
+        b.step(dt)
+        b.synchronize()
+        r.step(dt, r.pairs())
+        assert b.get_world(0).tobytes() == r.get_bodies().tobytes()
+    assert b.world_stats(0)["sweep_path"] == 2
+    b.close()
+    r.close()

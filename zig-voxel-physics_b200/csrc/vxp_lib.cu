@@ -44,16 +44,16 @@ __device__ __forceinline__ CacheSmem cache_smem(unsigned char* raw, uint32_t nwa
 
 // One world per CTA: block b steps worlds[b].
 template <int kThreads>
-__global__ void __launch_bounds__(kThreads, 512 / kThreads) k_step_block(const WorldDev* worlds, const __grid_constant__ ColliderSet cs) {
+__global__ void __launch_bounds__(kThreads, 512 / kThreads) k_step_block(const WorldDev* __restrict__ worlds, const __grid_constant__ ColliderSet cs) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpManifold* wsm = reinterpret_cast<WarpManifold*>(smem_raw);
-    const WorldDev w = worlds[blockIdx.x];
+    const WorldDev& w = worlds[blockIdx.x];
     const CacheSmem csm = cache_smem(smem_raw, blockDim.x / 32u, w.cache_cap);
     BlockGroup g;
     world_step(g, w, cs, wsm, csm, reinterpret_cast<float*>(smem_raw));
 }
-template __global__ void k_step_block<256>(const WorldDev*, const __grid_constant__ ColliderSet);
-template __global__ void k_step_block<512>(const WorldDev*, const __grid_constant__ ColliderSet);
+template __global__ void k_step_block<256>(const WorldDev* __restrict__, const __grid_constant__ ColliderSet);
+template __global__ void k_step_block<512>(const WorldDev* __restrict__, const __grid_constant__ ColliderSet);
 
 // One world over a cooperative grid, in two kernels: the narrow part of the
 // step, then its solve part (barrier words bar[0] and bar[1]).
@@ -296,8 +296,10 @@ constexpr uint32_t kGridFlowChunks = 4;
 size_t grid_smem(uint32_t cache_cap) { return step_smem(kGridThreads, cache_cap); }
 // Dynamic shared memory of a one-CTA world's launch (either CTA size): the
 // narrow part's warp scratch and cache table, then room for the sweeps' state
-// of a small world (bodies, manifold slots, point rows); two 256-thread CTAs
-// still fit on one SM.
+// (bodies, manifold slots, point rows; rows beyond it spill).  Two 256-thread
+// CTAs still fit on one SM.  More for a 512-thread CTA, which has the SM's
+// registers to itself, holds more rows but takes the L1 that the narrow part
+// lives in: 256 worlds 1.50 / 1.55 / 1.74 ms a step at 96 / 136 / 220 KB.
 constexpr size_t kBlockSolveSmem = 96 * 1024;
 size_t block_smem(uint32_t cache_cap) { return std::max(step_smem(512, cache_cap), kBlockSolveSmem); }
 size_t solve_smem() { return (size_t)kGridFlowChunks * kChunkFloats * sizeof(float); }
@@ -1319,7 +1321,11 @@ struct WorldBuffers {
         w.n_static = n_static;
         w.bmask = bmask.p;
         w.cp = cp.p;
-        w.crow = crow.p;
+        // (a batch slot's pair records are free while its world is solved, and
+        // are as large as a point row)
+        static_assert(sizeof(PairInfo) >= CP_NVEL * sizeof(float), "a pair record holds a point row");
+        w.crow = crow.p ? crow.p : reinterpret_cast<float*>(pinfo.p);
+        w.crow_cap = crow.p ? 4u * pair_cap : pair_cap;
         w.isl_parent = isl_parent.p;
         w.isl_flag = isl_flag.p;
         w.isl_size = isl_size.p;

@@ -4156,7 +4156,7 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
         const size_t fixed = cluster_smem_bytes(sm.bcap, sm.nrep, max(need, 1u), 0u, ncol);
         if (!by_owner ||
             (fixed <= smem_bytes &&
-             (w.crow != nullptr || fixed + (size_t)max(needp, 1u) * CP_NVEL * sizeof(float) <= smem_bytes)))
+             (gtot <= w.crow_cap || fixed + (size_t)max(needp, 1u) * CP_NVEL * sizeof(float) <= smem_bytes)))
             break;
         by_owner = false;
     }
@@ -4167,7 +4167,7 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
     // rows in shared memory (the rest spill)
     const uint32_t pcap_s = (uint32_t)min((size_t)sm.pcap, (smem_bytes - fixed) / (CP_NVEL * sizeof(float)));
     const bool spill = pcap_s < sm.pcap;
-    if (spill && (w.crow == nullptr || (size_t)gtot > 4u * (size_t)w.pair_cap)) return false;
+    if (spill && gtot > w.crow_cap) return false;
     if (t == 0 && k == 0) w.ctr[C_SWEEP] = spill ? SWEEP_SPILL : SWEEP_SHARED;
     {
         unsigned char* p = smem;

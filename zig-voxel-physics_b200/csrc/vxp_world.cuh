@@ -246,9 +246,10 @@ struct CacheLook {
 // field is an operand in the constant bank and no copy precedes the launch: a
 // copy per thread, 0.7 KB of stack, is 0.4 MB a CTA, more than the L1 it lives
 // in (kernels of the 4096-body pile's step 1421 -> 1304 us, of 523 boxes 667
-// -> 633).  The one-CTA kernel steps one of many worlds and keeps a copy per
-// thread, whose fields the compiler can hold in registers over the loops' stores; read
-// from shared memory, 256 worlds took 268 ms instead of 260.
+// -> 633).  The one-CTA kernel steps one of many worlds and reads the fields
+// where the worlds' records lie, through a restrict pointer, so that they may stay in
+// registers over the loops' stores (256 worlds 1.51 ms a step with a copy per
+// thread, 1.44 so; from shared memory slower than with the copy).
 struct WorldDev {
     StepCfg cfg;
     uint32_t n_bodies;
@@ -332,8 +333,8 @@ struct WorldDev {
     float* isl_timer;
     unsigned long long* isl_keys[2];
     uint32_t* isl_state;
-    float* crow;                  // CP_NVEL * 4 * pair_cap floats or null: the cluster sweeps'
-                                  // point rows that do not fit in shared memory
+    float* crow;                  // CP_NVEL floats x crow_cap: the cluster and one-CTA sweeps' point
+    uint32_t crow_cap;            // rows that do not fit in shared memory
     uint4* cm;                    // per packed manifold: ia, ib, n, pair
     float2* cfr;                  // per packed manifold: friction, restitution
     // scratch
