@@ -151,6 +151,60 @@ __global__ void k_pack_bodies(const DBody* body, const DBodyProp* prop, const ui
     out[i] = s;
 }
 
+// The contact manager's manifolds for the host (vxp_manifolds_get): first the
+// places of those with contacts, in pair order, by one CTA; then each record
+// packed by a warp straight into pinned host memory, with the slots past its
+// contact count and the padding zeroed.
+__global__ void __launch_bounds__(1024) k_manifold_list(const ManifoldRec* m0, const ManifoldRec* m1,
+                                                        const uint32_t* frame, uint32_t pair_cap, uint32_t* list,
+                                                        uint32_t* count) {
+    const ManifoldRec* m = (frame[0] & 1u) ? m1 : m0;  // the latest narrow phase's
+    const uint32_t P = min(frame[1], pair_cap);
+    uint32_t carry = 0;
+    for (uint32_t p0 = 0; p0 < P; p0 += 4u * blockDim.x) {
+        // four a thread, consecutive
+        const uint32_t p = p0 + 4u * threadIdx.x;
+        uint32_t has = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j)
+            if (p + j < P && m[p + j].n > 0u) has |= 1u << j;
+        uint32_t tile;
+        uint32_t at = carry + block_excl_scan((uint32_t)__popc(has), &tile);
+        for (; has; has &= has - 1u) list[at++] = p + (uint32_t)(__ffs(has) - 1);
+        carry += tile;
+    }
+    if (threadIdx.x == 0) *count = carry;
+}
+__global__ void k_manifold_pack(const ManifoldRec* m0, const ManifoldRec* m1, const uint32_t* frame,
+                                const uint32_t* list, uint32_t n, uint32_t* out) {
+    const ManifoldRec* m = (frame[0] & 1u) ? m1 : m0;
+    constexpr uint32_t kWords = sizeof(ManifoldRec) / 4u, kContact = sizeof(ContactRec) / 4u, kHead = kWords - 4u * kContact;
+    const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (r >= n) return;
+    const ManifoldRec& src = m[list[r]];
+    const uint32_t used = kHead + min(src.n, 4u) * kContact;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(&src);
+    for (uint32_t i = lane; i < kWords; i += 32u) {
+        // the record's padding is word 5, a contact's word 19
+        const bool pad = i < kHead ? i == 5u : (i - kHead) % kContact == 19u;
+        out[(size_t)r * kWords + i] = i < used && !pad ? w[i] : 0u;
+    }
+}
+
+// The state that a new world reads before a step has written it.
+__global__ void k_world_reset(uint32_t* frame, uint32_t* ctr, unsigned long long* cframe, unsigned long long* ts,
+                              uint32_t* n_pairs, CacheKeyRec* ckey, uint32_t cache_cap) {
+    const uint32_t t = threadIdx.x;
+    if (t < 4u) frame[t] = 0u;
+    if (t < C_NCTR) ctr[t] = 0u;
+    if (t < TS_N) ts[t] = 0ull;
+    if (t == 0u) {
+        *cframe = 0ull;
+        *n_pairs = 0u;
+    }
+    for (uint32_t i = t; i < cache_cap; i += blockDim.x) ckey[i] = CacheKeyRec{0u, 0u, 0ull, 0ull, 0u, 0u};
+}
+
 // Bulk state export of bodies [first, first + n): one thread a body, each
 // requested field into its own array (vxp_bodies_export).
 __global__ void k_export(const DBody* body, const DBodyProp* prop, uint32_t first, uint32_t n, ColliderSet cs,
@@ -249,6 +303,77 @@ template <class T> struct DBuf {
     size_t bytes() const { return n * sizeof(T); }
 };
 
+// Pinned host memory for what the library copies to and from the device: a
+// copy to pageable memory is staged by the driver piece by piece, with a wait
+// in each call.  Larger copies than kPinnedMost go to the caller's memory directly.
+constexpr size_t kPinnedMost = (size_t)32 << 20;
+struct Pinned {
+    void* p = nullptr;
+    size_t n = 0;
+    Pinned() = default;
+    Pinned(const Pinned&) = delete;
+    Pinned& operator=(const Pinned&) = delete;
+    ~Pinned() {
+        if (p) cudaFreeHost(p);
+    }
+    // At least `bytes`, or nullptr (too large, or no memory).
+    void* get(size_t bytes) {
+        if (bytes > kPinnedMost) return nullptr;
+        if (bytes > n) {
+            if (p) cudaFreeHost(p);
+            p = nullptr;
+            n = 0;
+            const size_t want = std::min(kPinnedMost, std::max<size_t>(2 * bytes, (size_t)1 << 20));
+            if (cudaMallocHost(&p, want) != cudaSuccess) {
+                cudaGetLastError();
+                p = nullptr;
+                return nullptr;
+            }
+            n = want;
+        }
+        return p;
+    }
+};
+// Pinned buffers for uploads, taken in turn: the copies out of one may still
+// be queued while the next is filled; a buffer's event says when it is free.
+struct UploadRing {
+    static constexpr int kBuffers = 4;
+    Pinned buf[kBuffers];
+    cudaEvent_t done[kBuffers] = {};
+    int turn = 0;
+    UploadRing() = default;
+    UploadRing(const UploadRing&) = delete;
+    UploadRing& operator=(const UploadRing&) = delete;
+    ~UploadRing() {
+        for (cudaEvent_t e : done)
+            if (e) {
+                cudaEventSynchronize(e);
+                cudaEventDestroy(e);
+            }
+    }
+    void* get(size_t bytes) {
+        // a buffer that is free now, the last used first (a new one is pinned
+        // only when the others are busy), else the next in turn once it is
+        for (int k = 0; k < kBuffers; ++k) {
+            const int b = (turn + k) % kBuffers;
+            if (!done[b] || cudaEventQuery(done[b]) == cudaSuccess) {
+                turn = b;
+                break;
+            }
+            if (k + 1 == kBuffers) turn = (turn + 1) % kBuffers;
+        }
+        cudaGetLastError();  // (a busy buffer's query)
+        if (!done[turn] && cudaEventCreateWithFlags(&done[turn], cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            done[turn] = nullptr;
+            return nullptr;
+        }
+        if (cudaEventSynchronize(done[turn]) != cudaSuccess) return nullptr;
+        return buf[turn].get(bytes);
+    }
+    bool queued(cudaStream_t s) { return cudaEventRecord(done[turn], s) == cudaSuccess; }
+};
+
 uint32_t next_pow2(uint32_t x) {
     uint32_t p = 1;
     while (p < x) p <<= 1;
@@ -330,19 +455,33 @@ void collider_metadata(float vs, const int32_t* pos, const uint8_t* vox, size_t 
     for (size_t b = 0; b < nb; ++b) {
         const int32_t* bp = &pos[b * 3];
         const uint8_t* v = &vox[b * 512];
-        uint32_t solid = 0;
+        // the solid voxels' count and extents, a row of eight at a time
+        uint32_t solid = 0, xs = 0, ys = 0, zs = 0;
+        for (int r = 0; r < 64; ++r) {
+            uint64_t q;
+            std::memcpy(&q, v + 8 * r, 8);
+            // bit x of the row: voxel x has a type (a nonzero low three bits)
+            q &= 0x0707070707070707ull;
+            q = (q | (q >> 1) | (q >> 2)) & 0x0101010101010101ull;
+            const uint32_t row = (uint32_t)((q * 0x0102040810204080ull) >> 56);
+            if (!row) continue;
+            solid += (uint32_t)__builtin_popcount(row);
+            xs |= row;
+            ys |= 1u << (r & 7);
+            zs |= 1u << (r >> 3);
+        }
         float bmn[3] = {inf, inf, inf}, bmx[3] = {-inf, -inf, -inf};
-        for (int i = 0; i < 512; ++i) {
-            if ((v[i] & 7u) == 0u) continue;
-            ++solid;
-            const int c[3] = {i % 8, (i / 8) % 8, i / 64};
+        if (solid) {
+            // a voxel's lower and upper corner grow with its coordinate, so the
+            // extremes are the first and last voxel's
+            const uint32_t axis[3] = {xs, ys, zs};
             for (int k = 0; k < 3; ++k) {
-                const float lp = ((float)bp[k] * 8.0f + (float)c[k]) * vs;
-                bmn[k] = std::fmin(bmn[k], lp);
-                bmx[k] = std::fmax(bmx[k], lp + vs);
-                const int32_t vc = bp[k] * 8 + c[k];
-                h.min_bound[k] = std::min(h.min_bound[k], vc);
-                h.max_bound[k] = std::max(h.max_bound[k], vc + 1);
+                const int lo = __builtin_ctz(axis[k]), hi = 31 - __builtin_clz(axis[k]);
+                const float l0 = ((float)bp[k] * 8.0f + (float)lo) * vs, l1 = ((float)bp[k] * 8.0f + (float)hi) * vs;
+                bmn[k] = std::fmin(bmn[k], l0);
+                bmx[k] = std::fmax(bmx[k], l1 + vs);
+                h.min_bound[k] = std::min(h.min_bound[k], bp[k] * 8 + lo);
+                h.max_bound[k] = std::max(h.max_bound[k], bp[k] * 8 + hi + 1);
             }
         }
         if (solid == 0) continue;
@@ -426,6 +565,7 @@ struct ColliderStore {
     };
     Staging stage[2];
     uint32_t turn = 0;
+    Pinned rd;  // what read() copies back
 
     ColliderStore() = default;
     ColliderStore(const ColliderStore&) = delete;
@@ -520,17 +660,25 @@ struct ColliderStore {
             return VXP_ERR_ARG;
         }
         if (int rc = sync(s, err)) return rc;
-        if (cudaStreamSynchronize(s) != cudaSuccess) {
-            err = "collider read: stream failed";
-            return VXP_ERR_CUDA;
-        }
         const Entry& e = colliders[ci];
+        // the record and the bricks asked for, behind the work already queued
+        const uint32_t n = e.d.n_bricks, k = bricks ? std::min(cap, n) : 0u;
         DCollider d;
-        if (cudaMemcpy(&d, d_col.p + ci, sizeof(d), cudaMemcpyDeviceToHost) != cudaSuccess) {
+        std::vector<uint8_t> far;
+        uint8_t* v = static_cast<uint8_t*>(rd.get(sizeof(d) + (size_t)k * 512));
+        if (!v) {
+            far.resize(sizeof(d) + (size_t)k * 512);
+            v = far.data();
+        }
+        if (cudaMemcpyAsync(v, d_col.p + ci, sizeof(d), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            (k && cudaMemcpyAsync(v + sizeof(d), d_vox.p + (size_t)e.d.brick_off * 512, (size_t)k * 512,
+                                  cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
             err = "collider read: copy failed";
             return VXP_ERR_CUDA;
         }
-        const uint32_t n = d.n_bricks;
+        std::memcpy(&d, v, sizeof(d));
+        v += sizeof(d);
         if (info) {
             std::memset(info, 0, sizeof(*info));
             info->voxel_size = d.vs;
@@ -545,17 +693,10 @@ struct ColliderStore {
             info->has_table = d.nb_off != kNoTable ? 1u : 0u;
         }
         if (n_out) *n_out = n;
-        const uint32_t k = bricks ? std::min(cap, n) : 0u;
         if (k) {
-            std::vector<uint8_t> v((size_t)k * 512);
-            if (cudaMemcpy(v.data(), d_vox.p + (size_t)d.brick_off * 512, v.size(), cudaMemcpyDeviceToHost) !=
-                cudaSuccess) {
-                err = "collider read: copy failed";
-                return VXP_ERR_CUDA;
-            }
             for (uint32_t b = 0; b < k; ++b) {
                 for (int q = 0; q < 3; ++q) bricks[b].pos[q] = e.pos[(size_t)b * 3 + q];
-                std::memcpy(bricks[b].voxels, &v[(size_t)b * 512], 512);
+                std::memcpy(bricks[b].voxels, v + (size_t)b * 512, 512);
             }
         }
         return VXP_OK;
@@ -1171,24 +1312,51 @@ struct WorldBuffers {
         return VXP_OK;
     }
 
-    int set_bodies(const vxp_body* b, uint32_t n, const ColliderStore& cols, std::string& err) {
+    // The body table, queued on `stream` from a pinned buffer.
+    int set_bodies(const vxp_body* b, uint32_t n, const ColliderStore& cols, UploadRing& up, cudaStream_t stream,
+                   std::string& err) {
         if (!b && n) {
             err = "null bodies";
             return VXP_ERR_ARG;
         }
         if (int rc = ensure_bodies(n, err)) return rc;
-        std::vector<DBody> db(n);
-        std::vector<DBodyProp> dp(n);
-        std::vector<uint2> id(n);
+        uint32_t statics = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            if (b[i].body_type > 2u) {
+                err = fmt("body %u: bad body_type %u", i, b[i].body_type);
+                return VXP_ERR_ARG;
+            }
+            statics += b[i].body_type == 0u ? 1u : 0u;
+        }
+        if (pub_cid.reserve(n) != cudaSuccess || pack.reserve(n) != cudaSuccess ||
+            stat.reserve(std::max<uint32_t>(statics, 1)) != cudaSuccess) {
+            err = "body buffers: device allocation failed";
+            return VXP_ERR_OOM;
+        }
+        // bodies | properties | (id, index) | collider ids | statics | island state
+        const size_t o_prop = n * sizeof(DBody), o_id = o_prop + n * sizeof(DBodyProp), o_cid = o_id + n * sizeof(uint2),
+                     o_stat = o_cid + n * sizeof(uint32_t), o_isl = o_stat + statics * sizeof(uint32_t),
+                     total = o_isl + IS_N * sizeof(uint32_t);
+        std::vector<DBody> far;  // (aligned as the records are)
+        unsigned char* st = static_cast<unsigned char*>(up.get(total));
+        const bool pinned = st != nullptr;
+        if (!pinned) {
+            far.resize(total / sizeof(DBody) + 1);
+            st = reinterpret_cast<unsigned char*>(far.data());
+        }
+        DBody* db = reinterpret_cast<DBody*>(st);
+        DBodyProp* dp = reinterpret_cast<DBodyProp*>(st + o_prop);
+        uint2* id = reinterpret_cast<uint2*>(st + o_id);
+        uint32_t* cid = reinterpret_cast<uint32_t*>(st + o_cid);
+        uint32_t* stl = reinterpret_cast<uint32_t*>(st + o_stat);
+        uint32_t* isl = reinterpret_cast<uint32_t*>(st + o_isl);
+        static_assert(sizeof(DBody) % 16 == 0 && sizeof(DBodyProp) % 8 == 0, "records follow one another");
         collider_public.resize(n);
         moving_collider.clear();
         measured = false;
+        uint32_t ns = 0;
         for (uint32_t i = 0; i < n; ++i) {
             const vxp_body& s = b[i];
-            if (s.body_type > 2u) {
-                err = fmt("body %u: bad body_type %u", i, s.body_type);
-                return VXP_ERR_ARG;
-            }
             DBody& d = db[i];
             d.p = make_float4(s.position[0], s.position[1], s.position[2], s.inv_mass);
             d.q = make_float4(s.rotation[0], s.rotation[1], s.rotation[2], s.rotation[3]);
@@ -1206,54 +1374,71 @@ struct WorldBuffers {
             p.type = s.body_type;
             p.collider = cols.index_of(s.collider_id);
             if (s.body_type != 0u) moving_collider.push_back(p.collider);
+            else stl[ns++] = i;  // never moved by a step; ascending
             p.sleeping = s.is_sleeping ? 1u : 0u;
-            collider_public[i] = s.collider_id;
+            collider_public[i] = cid[i] = s.collider_id;
             id[i] = make_uint2(s.id, i);
         }
-        std::sort(id.begin(), id.end(), [](const uint2& x, const uint2& y) { return x.x < y.x; });
+        auto by_id = [](const uint2& x, const uint2& y) { return x.x < y.x; };
+        if (!std::is_sorted(id, id + n, by_id)) std::sort(id, id + n, by_id);
         for (uint32_t i = 1; i < n; ++i)
             if (id[i].x == id[i - 1].x) {
                 err = fmt("duplicate body id %u", id[i].x);
                 return VXP_ERR_ARG;
             }
-        if (n && (cudaMemcpy(body.p, db.data(), n * sizeof(DBody), cudaMemcpyHostToDevice) != cudaSuccess ||
-                  cudaMemcpy(prop.p, dp.data(), n * sizeof(DBodyProp), cudaMemcpyHostToDevice) != cudaSuccess ||
-                  cudaMemcpy(ids.p, id.data(), n * sizeof(uint2), cudaMemcpyHostToDevice) != cudaSuccess ||
-                  pub_cid.reserve(n) != cudaSuccess || pack.reserve(n) != cudaSuccess ||
-                  cudaMemcpy(pub_cid.p, collider_public.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice) !=
-                      cudaSuccess)) {
+        // the next solve rebuilds its islands: their roots are body indices
+        // (IslandManager.markDirty, islands.zig:301-303)
+        for (uint32_t k = 0; k < IS_N; ++k) isl[k] = k == IS_DIRTY ? 1u : 0u;
+        auto put = [&](void* dst, size_t off, size_t bytes) {
+            return bytes == 0 || cudaMemcpyAsync(dst, st + off, bytes, cudaMemcpyHostToDevice, stream) == cudaSuccess;
+        };
+        if (!put(body.p, 0, o_prop) || !put(prop.p, o_prop, o_id - o_prop) || !put(ids.p, o_id, o_cid - o_id) ||
+            !put(pub_cid.p, o_cid, o_stat - o_cid) || !put(stat.p, o_stat, o_isl - o_stat) ||
+            !put(isl_state.p, o_isl, total - o_isl) || (pinned && !up.queued(stream)) ||
+            (!pinned && cudaStreamSynchronize(stream) != cudaSuccess)) {
             err = "body upload failed";
             return VXP_ERR_CUDA;
         }
-        // the static bodies (never moved by a step), ascending
-        std::vector<uint32_t> st;
-        for (uint32_t i = 0; i < n; ++i)
-            if (dp[i].type == 0u) st.push_back(i);
-        if (stat.reserve(std::max<size_t>(st.size(), 1)) != cudaSuccess ||
-            (!st.empty() && cudaMemcpy(stat.p, st.data(), st.size() * sizeof(uint32_t), cudaMemcpyHostToDevice) !=
-                                cudaSuccess)) {
-            err = "static body list upload failed";
-            return VXP_ERR_CUDA;
-        }
-        n_static = (uint32_t)st.size();
+        n_static = statics;
         n_bodies = n;
-        mark_islands_dirty();  // the island roots are body indices
         return VXP_OK;
     }
 
-    int get_bodies(vxp_body* b, uint32_t n, cudaStream_t stream, std::string& err) {
+    // The body table back.  check: also read the sticky error word, in the
+    // same wait, and fail with it (nothing is written then).
+    int get_bodies(vxp_body* b, uint32_t n, cudaStream_t stream, Pinned& rd, bool check, std::string& err) {
         if (n != n_bodies) {
+            if (check)
+                if (int rc = take_error(stream, err)) return rc;
             err = fmt("expected %u bodies, got %u", n_bodies, n);
             return VXP_ERR_ARG;
         }
-        if (!n) return VXP_OK;
-        k_pack_bodies<<<(n + 255u) / 256u, 256, 0, stream>>>(body.p, prop.p, pub_cid.p, n, pack.p);
+        const size_t bytes = n * sizeof(vxp_body);
+        unsigned char* st = static_cast<unsigned char*>(rd.get(bytes + 16));
+        if (!st) {
+            if (check)
+                if (int rc = take_error(stream, err)) return rc;
+            if (n) k_pack_bodies<<<(n + 255u) / 256u, 256, 0, stream>>>(body.p, prop.p, pub_cid.p, n, pack.p);
+            if (cudaPeekAtLastError() != cudaSuccess ||
+                cudaMemcpyAsync(b, pack.p, bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+                cudaStreamSynchronize(stream) != cudaSuccess) {
+                err = "body download failed";
+                return VXP_ERR_CUDA;
+            }
+            return VXP_OK;
+        }
+        uint32_t* e = reinterpret_cast<uint32_t*>(st + bytes);
+        *e = 0u;
+        if (n) k_pack_bodies<<<(n + 255u) / 256u, 256, 0, stream>>>(body.p, prop.p, pub_cid.p, n, pack.p);
         if (cudaPeekAtLastError() != cudaSuccess ||
-            cudaMemcpyAsync(b, pack.p, n * sizeof(vxp_body), cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+            (n && cudaMemcpyAsync(st, pack.p, bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess) ||
+            (check && cudaMemcpyAsync(e, ctr.p + C_ERROR, sizeof(*e), cudaMemcpyDeviceToHost, stream) != cudaSuccess) ||
             cudaStreamSynchronize(stream) != cudaSuccess) {
             err = "body download failed";
             return VXP_ERR_CUDA;
         }
+        if (*e) return take_error(stream, err);
+        if (n) std::memcpy(b, st, bytes);
         return VXP_OK;
     }
 
@@ -1347,19 +1532,12 @@ struct WorldBuffers {
         return w;
     }
 
-    // Every device buffer back to zero, as a new allocation is: a batch slot
-    // reused for another world starts from exactly the state of a new one.
-    cudaError_t zero_all(cudaStream_t s) {
-        cudaError_t e = cudaSuccess;
-        auto z = [&](auto& b) {
-            if (b.p && e == cudaSuccess) e = cudaMemsetAsync(b.p, 0, b.bytes(), s);
-        };
-        z(body); z(prop); z(p0); z(qn); z(aabb_mn); z(aabb_mx); z(ids); z(pcount); z(poff); z(adj_off); z(adj_cur);
-        z(bmask); z(pairs); z(n_pairs_dev); z(pinfo); z(man0); z(man1); z(ht0); z(ht1); z(frame); z(cons); z(colour);
-        z(pos_of); z(packed_pair); z(adj); z(flag); z(clist); z(cp); z(cm); z(rk); z(cfr); z(ev); z(snap); z(chunk);
-        z(colour_cnt); z(colour_cur); z(scan); z(ctr); z(cwriter); z(ts); z(cframe); z(ckey); z(cval); z(dump);
-        z(ocnt); z(ocur); z(stat); z(bpmask);
-        return e;
+    // A batch slot reused for another world starts as a new one: the words
+    // that a step reads before it writes them, and nothing else (the pair
+    // tables count as empty while their sizes in frame are zero).
+    cudaError_t reset(cudaStream_t s) {
+        k_world_reset<<<1, 256, 0, s>>>(frame.p, ctr.p, cframe.p, ts.p, n_pairs_dev.p, ckey.p, cache_cap);
+        return cudaGetLastError();
     }
 
     size_t device_bytes() const {
@@ -1475,7 +1653,9 @@ struct vxp_ctx {
     bool cluster_whole = false;  // the cluster also builds the constraint table and colours it
     bool last_cluster = false;
     bool last_grid = false;
-    uint32_t* h_count = nullptr;  // pinned mirror of the device pair count
+    uint32_t* h_count = nullptr;  // pinned words: [0] mirror of the device pair count, [1], [2] read back in calls
+    UploadRing up;
+    Pinned rd;
     bool count_pending = false;
     int use_grid = -1;  // -1 auto, 0 block, 1 grid
     uint32_t solver_div = 128;
@@ -1623,8 +1803,9 @@ int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, floa
 }
 
 int check_device_error(vxp_ctx* ctx) {
+    CK(cudaMemcpyAsync(ctx->h_count + 1, ctx->w.ctr.p + C_ERROR, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    return ctx->w.take_error(ctx->stream, ctx->err);
+    return ctx->h_count[1] ? ctx->w.take_error(ctx->stream, ctx->err) : VXP_OK;
 }
 
 // The pair list of the current body state into ctx->w.pairs (host waits).
@@ -1651,11 +1832,11 @@ int compute_device_pairs(vxp_ctx* ctx, float margin, uint32_t* n_out) {
         CK(cudaMemsetAsync(ctx->bar.p, 0, sizeof(GridBar), ctx->stream));
         CK(cudaLaunchCooperativeKernel((const void*)k_pairs_grid, dim3(ctx->grid_blocks), dim3(kGridThreads), args,
                                        grid_smem(wd.cache_cap), ctx->stream));
-        uint32_t err = 0;
-        CK(cudaMemcpyAsync(&total, w.n_pairs_dev.p, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaMemcpyAsync(&err, w.ctr.p + C_ERROR, sizeof(err), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(ctx->h_count + 2, w.n_pairs_dev.p, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(ctx->h_count + 1, w.ctr.p + C_ERROR, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        if (err & ERR_TIMEOUT) return w.take_error(ctx->stream, ctx->err);
+        total = ctx->h_count[2];
+        if (ctx->h_count[1] & ERR_TIMEOUT) return w.take_error(ctx->stream, ctx->err);
         if (total <= w.pair_cap || attempt) break;
         // the list did not fit: grow and run again
         if (int rc = w.ensure_pairs(total, ctx->err)) return rc;
@@ -1900,7 +2081,7 @@ int vxp_create(const vxp_config* cfg, int device, vxp_ctx** out) {
         cudaEventCreate(&ctx->ev_cons) != cudaSuccess ||
         cudaEventCreateWithFlags(&ctx->ev_count, cudaEventDisableTiming) != cudaSuccess)
         return bail(VXP_ERR_CUDA);
-    if (cudaMallocHost(&ctx->h_count, sizeof(uint32_t)) != cudaSuccess) return bail(VXP_ERR_OOM);
+    if (cudaMallocHost(&ctx->h_count, 4 * sizeof(uint32_t)) != cudaSuccess) return bail(VXP_ERR_OOM);
     *ctx->h_count = 0;
     const uint32_t cache_cap = cfg->brick_pair_cache_size ? cfg->brick_pair_cache_size : 1024u;
     if (set_kernel_smem(cache_cap)) return bail(VXP_ERR_CUDA);
@@ -2014,15 +2195,14 @@ int vxp_invalidate_cache_for_body(vxp_ctx* ctx, uint32_t body_id, uint32_t* n_in
 
 int vxp_bodies_set(vxp_ctx* ctx, const vxp_body* b, uint32_t n) {
     if (!ctx) return VXP_ERR_ARG;
-    CK(cudaStreamSynchronize(ctx->stream));
-    ctx->w.measured = false;
-    return ctx->w.set_bodies(b, n, ctx->cols, ctx->err);
+    if (n > ctx->w.body_cap) CK(cudaStreamSynchronize(ctx->stream));  // buffers are replaced
+    return ctx->w.set_bodies(b, n, ctx->cols, ctx->up, ctx->stream, ctx->err);
 }
 
 // vxp_bodies_export / vxp_batch_world_export on one world's buffers.
 static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_view* dst, uint32_t first,
-                        uint32_t n, int device_memory, void* consumer, cudaStream_t stream, int device,
-                        std::string& err) {
+                        uint32_t n, int device_memory, void* consumer, cudaStream_t stream, int device, Pinned& rd,
+                        bool check, std::string& err) {
     if (!dst) {
         err = "null state view";
         return VXP_ERR_ARG;
@@ -2073,6 +2253,10 @@ static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_
         if (ptr[f]) total += (per[f] * n + 15u) & ~(size_t)15u;
     }
     if (total == 0) return VXP_OK;
+    // the staging buffer comes back in one copy, with the error word (check)
+    unsigned char* back = static_cast<unsigned char*>(rd.get(total + 16));
+    if (check && !back)
+        if (int rc = w.take_error(stream, err)) return rc;
     if (w.export_stage.reserve(total) != cudaSuccess) {
         err = "export staging: device allocation failed";
         return VXP_ERR_OOM;
@@ -2091,6 +2275,20 @@ static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_
         err = fmt("export launch: %s", cudaGetErrorString(cudaGetLastError()));
         return VXP_ERR_CUDA;
     }
+    if (back) {
+        uint32_t* e = reinterpret_cast<uint32_t*>(back + total);
+        *e = 0u;
+        if (cudaMemcpyAsync(back, st, total, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+            (check && cudaMemcpyAsync(e, w.ctr.p + C_ERROR, sizeof(*e), cudaMemcpyDeviceToHost, stream) != cudaSuccess) ||
+            cudaStreamSynchronize(stream) != cudaSuccess) {
+            err = "export: copy to host failed";
+            return VXP_ERR_CUDA;
+        }
+        if (*e) return w.take_error(stream, err);
+        for (int f = 0; f < 7; ++f)
+            if (ptr[f]) std::memcpy(ptr[f], back + off[f], per[f] * n);
+        return VXP_OK;
+    }
     for (int f = 0; f < 7; ++f) {
         if (!ptr[f]) continue;
         if (cudaMemcpyAsync(ptr[f], st + off[f], per[f] * n, cudaMemcpyDeviceToHost, stream) != cudaSuccess) {
@@ -2108,18 +2306,17 @@ static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_
 int vxp_bodies_export(vxp_ctx* ctx, const vxp_state_view* dst, uint32_t first, uint32_t n, int device_memory,
                       void* consumer_stream) {
     if (!ctx) return VXP_ERR_ARG;
-    if (!device_memory) {
+    if (!device_memory && (n == 0 || !dst || first > ctx->w.n_bodies || n > ctx->w.n_bodies - first)) {
         if (int rc = check_device_error(ctx)) return rc;
     }
     if (int rc = ctx->cols.sync(ctx->stream, ctx->err)) return rc;
     return export_world(ctx->w, ctx->cols.set(), dst, first, n, device_memory, consumer_stream, ctx->stream,
-                        ctx->device, ctx->err);
+                        ctx->device, ctx->rd, !device_memory, ctx->err);
 }
 
 int vxp_bodies_get(vxp_ctx* ctx, vxp_body* b, uint32_t n) {
     if (!ctx || (!b && n)) return fail(ctx, VXP_ERR_ARG, "null argument");
-    if (int rc = check_device_error(ctx)) return rc;
-    return ctx->w.get_bodies(b, n, ctx->stream, ctx->err);
+    return ctx->w.get_bodies(b, n, ctx->stream, ctx->rd, true, ctx->err);
 }
 
 int vxp_mass_properties(float vs, const vxp_brick* bricks, uint32_t n, float density, float* inv_mass,
@@ -2237,28 +2434,25 @@ int vxp_solve(vxp_ctx* ctx, float dt) {
 int vxp_manifolds_get(vxp_ctx* ctx, vxp_manifold* out, uint32_t cap, uint32_t* n_out) {
     if (!ctx || !n_out) return VXP_ERR_ARG;
     if (int rc = check_device_error(ctx)) return rc;
-    uint32_t fr[2];
-    CK(cudaMemcpy(fr, ctx->w.frame.p, sizeof(fr), cudaMemcpyDeviceToHost));
-    // the latest narrow phase wrote man[frame & 1] with fr[1] slots
-    const uint32_t slot = fr[0] & 1u;
-    const ManifoldRec* m = slot ? ctx->w.man1.p : ctx->w.man0.p;
-    const uint32_t P = std::min<uint32_t>(fr[1], ctx->w.pair_cap);
-    std::vector<ManifoldRec> hm(P);
-    if (P) CK(cudaMemcpy(hm.data(), m, P * sizeof(ManifoldRec), cudaMemcpyDeviceToHost));
-    uint32_t k = 0;
-    for (uint32_t p = 0; p < P; ++p) {
-        if (hm[p].n == 0u) continue;
-        if (k < cap && out) {
-            // slots past contact_count hold stale data on the device
-            ManifoldRec r = hm[p];
-            r._pad = 0u;
-            for (uint32_t i = r.n; i < 4u; ++i) std::memset(&r.c[i], 0, sizeof(ContactRec));
-            for (uint32_t i = 0; i < r.n; ++i) r.c[i]._pad = 0u;
-            std::memcpy(&out[k], &r, sizeof(vxp_manifold));
-        }
-        ++k;
+    // (flag is scratch between steps)
+    WorldBuffers& w = ctx->w;
+    k_manifold_list<<<1, 1024, 0, ctx->stream>>>(w.man0.p, w.man1.p, w.frame.p, w.pair_cap, w.flag.p, ctx->h_count + 2);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(ctx->stream));
+    const uint32_t n = ctx->h_count[2];
+    *n_out = n;
+    // in pieces of what the pinned buffer may hold
+    const uint32_t k = out ? std::min(n, cap) : 0u, piece = (uint32_t)(kPinnedMost / sizeof(ManifoldRec));
+    for (uint32_t at = 0; at < k; at += piece) {
+        const uint32_t m = std::min(piece, k - at);
+        void* st = ctx->rd.get(m * sizeof(ManifoldRec));
+        if (!st) return fail(ctx, VXP_ERR_OOM, "pinned memory for %u manifolds", m);
+        k_manifold_pack<<<(m + 7u) / 8u, 256, 0, ctx->stream>>>(w.man0.p, w.man1.p, w.frame.p, w.flag.p + at, m,
+                                                                static_cast<uint32_t*>(st));
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(ctx->stream));
+        std::memcpy(out + at, st, m * sizeof(ManifoldRec));
     }
-    *n_out = k;
     return VXP_OK;
 }
 
@@ -2318,10 +2512,14 @@ int vxp_pairs_from_bodies(vxp_ctx* ctx, float margin, vxp_pair* out, uint32_t ca
     if (!ctx || !n_out) return VXP_ERR_ARG;
     uint32_t n = 0;
     if (int rc = compute_device_pairs(ctx, margin, &n)) return rc;
-    CK(cudaStreamSynchronize(ctx->stream));
     *n_out = n;
     const uint32_t k = std::min(n, cap);
-    if (k && out) CK(cudaMemcpy(out, ctx->w.pairs.p, k * sizeof(vxp_pair), cudaMemcpyDeviceToHost));
+    if (k && out) {
+        void* st = ctx->rd.get(k * sizeof(vxp_pair));
+        CK(cudaMemcpyAsync(st ? st : out, ctx->w.pairs.p, k * sizeof(vxp_pair), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (st) std::memcpy(out, st, k * sizeof(vxp_pair));
+    }
     return n > cap ? fail(ctx, VXP_ERR_CAP, "pair output holds %u, need %u", cap, n) : VXP_OK;
 }
 
@@ -2542,6 +2740,8 @@ struct vxp_batch {
     ColliderSet graph_cs{};
     uint32_t graph_n = 0, graph_threads = 0;
     DBuf<uint32_t> d_word;  // a count read back by the host
+    UploadRing up;
+    Pinned rd;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     uint32_t cache_cap = 1024;
 };
@@ -2772,23 +2972,23 @@ int vxp_batch_invalidate_cache_for_body(vxp_batch* bt, uint32_t world, uint32_t 
 
 int vxp_batch_world_set(vxp_batch* bt, uint32_t world, const vxp_body* bodies, uint32_t n, uint32_t pair_capacity) {
     if (!bt || world >= bt->slots.size()) return bfail(bt, VXP_ERR_ARG, "world index out of range");
-    BK(cudaStreamSynchronize(bt->stream));
     auto& slot = bt->slots[world];
+    const uint32_t want = pair_capacity ? pair_capacity : std::max<uint32_t>(1024, 16u * n);
     // a fresh world starts with an empty contact manager and cache; a slot
     // that held an earlier world keeps its buffers (no allocation, no free,
-    // which would wait for the whole device) and starts from them zeroed
+    // which would wait for the whole device), reset behind the steps queued
     if (slot) {
-        BK(slot->zero_all(bt->stream));
-        BK(cudaStreamSynchronize(bt->stream));
+        if (n > slot->body_cap || want > slot->pair_cap) BK(cudaStreamSynchronize(bt->stream));
+        BK(slot->reset(bt->stream));
         slot->n_bodies = 0;
         slot->collider_public.clear();
     } else {
+        BK(cudaStreamSynchronize(bt->stream));
         slot.reset(new WorldBuffers);
+        if (int rc = slot->init(bt->cache_cap, 1, bt->err)) return rc;
     }
     slot->live = true;
-    if (int rc = slot->init(bt->cache_cap, 1, bt->err)) return rc;
-    if (int rc = slot->set_bodies(bodies, n, bt->cols, bt->err)) return rc;
-    const uint32_t want = pair_capacity ? pair_capacity : std::max<uint32_t>(1024, 16u * n);
+    if (int rc = slot->set_bodies(bodies, n, bt->cols, bt->up, bt->stream, bt->err)) return rc;
     if (int rc = slot->ensure_pairs(want, bt->err)) return rc;
     bt->active[world] = n ? 1 : 0;
     bt->est_ms[world] = 0.0f;
@@ -2798,7 +2998,6 @@ int vxp_batch_world_set(vxp_batch* bt, uint32_t world, const vxp_body* bodies, u
 
 int vxp_batch_world_clear(vxp_batch* bt, uint32_t world) {
     if (!bt || world >= bt->slots.size()) return bfail(bt, VXP_ERR_ARG, "world index out of range");
-    BK(cudaStreamSynchronize(bt->stream));
     if (bt->slots[world]) bt->slots[world]->live = false;
     bt->active[world] = 0;
     bt->rebuild = true;
@@ -2817,18 +3016,17 @@ int vxp_batch_world_release(vxp_batch* bt, uint32_t world) {
 int vxp_batch_world_get(vxp_batch* bt, uint32_t world, vxp_body* bodies, uint32_t n) {
     if (!bt || world >= bt->slots.size() || !bt->slots[world] || !bt->slots[world]->live)
         return bfail(bt, VXP_ERR_ARG, "no such world");
-    BK(cudaStreamSynchronize(bt->stream));
-    return bt->slots[world]->get_bodies(bodies, n, bt->stream, bt->err);
+    if (!bodies && n) return bfail(bt, VXP_ERR_ARG, "null argument");
+    return bt->slots[world]->get_bodies(bodies, n, bt->stream, bt->rd, false, bt->err);
 }
 
 int vxp_batch_world_export(vxp_batch* bt, uint32_t world, const vxp_state_view* dst, uint32_t first, uint32_t n,
                            int device_memory, void* consumer_stream) {
     if (!bt || world >= bt->slots.size() || !bt->slots[world] || !bt->slots[world]->live)
         return bfail(bt, VXP_ERR_ARG, "no such world");
-    if (!device_memory) BK(cudaStreamSynchronize(bt->stream));
     if (int rc = bt->cols.sync(bt->stream, bt->err)) return rc;
     return export_world(*bt->slots[world], bt->cols.set(), dst, first, n, device_memory, consumer_stream, bt->stream,
-                        bt->device, bt->err);
+                        bt->device, bt->rd, false, bt->err);
 }
 
 int vxp_batch_world_stats(vxp_batch* bt, uint32_t world, vxp_stats* s) {

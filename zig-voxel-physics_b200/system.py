@@ -42,12 +42,15 @@ def _edit_args(coords, values, mode):
 def _read_collider(fn, handle, collider_id):
     info = np.zeros(1, dtype=abi.COLLIDER_INFO_DTYPE)
     n = ctypes.c_uint32(0)
-    rc = fn(handle, int(collider_id), abi.ptr(info), None, 0, ctypes.byref(n))
-    if rc != 0:
-        return rc, None, None
-    bricks = np.zeros(n.value, dtype=abi.BRICK_DTYPE)
-    rc = fn(handle, int(collider_id), abi.ptr(info), abi.ptr(bricks), len(bricks), ctypes.byref(n))
-    return rc, info[0], bricks
+    cap = 1024  # bricks; usually enough, else once more with the count
+    while True:
+        bricks = np.empty(cap, dtype=abi.BRICK_DTYPE)
+        rc = fn(handle, int(collider_id), abi.ptr(info), abi.ptr(bricks), cap, ctypes.byref(n))
+        if rc != 0:
+            return rc, None, None
+        if n.value <= cap:
+            return rc, info[0], bricks[: n.value]
+        cap = n.value
 
 
 class VoxelPhysicsSystem:
@@ -127,7 +130,7 @@ class VoxelPhysicsSystem:
         self.n_bodies = len(bodies)
 
     def get_bodies(self) -> np.ndarray:
-        out = np.zeros(self.n_bodies, dtype=abi.BODY_DTYPE)
+        out = np.empty(self.n_bodies, dtype=abi.BODY_DTYPE)
         self._check(self.lib.vxp_bodies_get(self.ctx, abi.ptr(out), self.n_bodies))
         return out
 
@@ -254,19 +257,24 @@ class VoxelPhysicsSystem:
     def pairs(self, margin: float | None = None) -> np.ndarray:
         m = self.pair_margin if margin is None else margin
         n = ctypes.c_uint32(0)
-        rc = self.lib.vxp_pairs_from_bodies(self.ctx, np.float32(m), None, 0, ctypes.byref(n))
-        if rc not in (0, abi.VXP_ERR_CAP):
-            self._check(rc)
-        out = np.zeros(n.value, dtype=abi.PAIR_DTYPE)
-        self._check(self.lib.vxp_pairs_from_bodies(self.ctx, np.float32(m), abi.ptr(out), len(out), ctypes.byref(n)))
-        return out
+        cap = max(256, 8 * self.n_bodies)  # usually enough; else once more with the count
+        while True:
+            out = np.empty(cap, dtype=abi.PAIR_DTYPE)
+            rc = self.lib.vxp_pairs_from_bodies(self.ctx, np.float32(m), abi.ptr(out), cap, ctypes.byref(n))
+            if rc != abi.VXP_ERR_CAP or n.value <= cap:
+                self._check(rc)
+                return out[: n.value]
+            cap = n.value
 
     def manifolds(self) -> np.ndarray:
         n = ctypes.c_uint32(0)
-        self._check(self.lib.vxp_manifolds_get(self.ctx, None, 0, ctypes.byref(n)))
-        out = np.zeros(n.value, dtype=abi.MANIFOLD_DTYPE)
-        self._check(self.lib.vxp_manifolds_get(self.ctx, abi.ptr(out), len(out), ctypes.byref(n)))
-        return out
+        cap = max(64, 4 * self.n_bodies)  # usually enough; else once more with the count
+        while True:
+            out = np.empty(cap, dtype=abi.MANIFOLD_DTYPE)
+            self._check(self.lib.vxp_manifolds_get(self.ctx, abi.ptr(out), cap, ctypes.byref(n)))
+            if n.value <= cap:
+                return out[: n.value]
+            cap = n.value
 
     def stats(self) -> dict:
         s = abi.Stats()
@@ -377,7 +385,7 @@ class VoxelWorldBatch:
         self.sizes.pop(int(world), None)
 
     def get_world(self, world: int) -> np.ndarray:
-        out = np.zeros(self.sizes[int(world)], dtype=abi.BODY_DTYPE)
+        out = np.empty(self.sizes[int(world)], dtype=abi.BODY_DTYPE)
         self._check(self.lib.vxp_batch_world_get(self.b, int(world), abi.ptr(out), len(out)))
         return out
 
