@@ -2535,6 +2535,72 @@ __device__ bool phase_islands(G& g, const WorldDev& w, uint32_t cur, uint32_t* s
     return g.sync();
 }
 
+// The colour of manifold g.rank() by its thread (M <= g.size()).  Its
+// higher-priority neighbours are found once; then it polls only those not yet
+// seen coloured, one L2 round trip a poll.  (Found anew for every poll,
+// through the pair, the bodies and the adjacency, a poll was five.)  The
+// higher-priority neighbours' threads all run, the highest-priority uncoloured
+// manifold waits for nobody, and the wait is bounded by kColourTimeoutNs.
+template <class G>
+__device__ void colour_polled(G& g, const WorldDev& w, uint32_t M) {
+    const uint32_t k = g.rank();
+    if (k >= M) return;
+    const PairInfo& pi = w.pinfo[w.cons[k]];
+    const bool wa = writable(w.prop[pi.ia]), wb = writable(w.prop[pi.ib]);
+    const uint32_t a0 = wa ? w.adj_off[pi.ia] : 0u, na = wa ? w.adj_off[pi.ia + 1u] - a0 : 0u;
+    const uint32_t b0 = wb ? w.adj_off[pi.ib] : 0u, nt = na + (wb ? w.adj_off[pi.ib + 1u] - b0 : 0u);
+    volatile uint32_t* vc = w.colour;
+    auto neighbour = [&](uint32_t t) { return w.adj[t < na ? a0 + t : b0 + (t - na)]; };
+    uint32_t used[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const unsigned long long t_start = global_ns();
+    uint32_t polls = 0;
+    for (uint32_t t0 = 0; t0 < nt; t0 += 64u) {
+        // the next 64 neighbours: those that come before this manifold
+        unsigned long long wait = 0ull;
+        const uint32_t n = min(64u, nt - t0);
+        for (uint32_t t = 0; t < n; ++t) {
+            const uint32_t j = neighbour(t0 + t);
+            if (j != k && jp_before(j, k)) wait |= 1ull << t;
+        }
+        while (wait) {
+            // sixteen at a time, every load of a group issued before any is used
+            for (unsigned long long m = wait; m;) {
+                uint32_t t[16], c[16];
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    t[q] = m ? (uint32_t)(__ffsll((long long)m) - 1) : 64u;
+                    m &= m - 1ull;
+                }
+#pragma unroll
+                for (int q = 0; q < 16; ++q) c[q] = t[q] < 64u ? neighbour(t0 + t[q]) : 0xFFFFFFFFu;
+#pragma unroll
+                for (int q = 0; q < 16; ++q) c[q] = c[q] != 0xFFFFFFFFu ? vc[c[q]] : 0xFFFFFFFFu;
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    if (c[q] == 0xFFFFFFFFu) continue;
+                    wait &= ~(1ull << t[q]);
+                    const uint32_t word = c[q] >> 5, bit = 1u << (c[q] & 31u);
+#pragma unroll
+                    for (uint32_t wd = 0; wd < 8u; ++wd) used[wd] |= word == wd ? bit : 0u;
+                }
+            }
+            if (wait && (++polls & 63u) == 0u) {
+                if (global_ns() - t_start > kColourTimeoutNs) atomicOr(&w.ctr[C_ERROR], ERR_TIMEOUT);
+                if ((*(volatile uint32_t*)&w.ctr[C_ERROR] & ERR_TIMEOUT) != 0u) return;
+            }
+        }
+    }
+    uint32_t c = 256u;
+#pragma unroll
+    for (uint32_t wd = 0; wd < 8u; ++wd)
+        if (c == 256u && used[wd] != 0xFFFFFFFFu) c = wd * 32u + (uint32_t)(__ffs(~used[wd]) - 1);
+    if (c >= 256u) {
+        atomicOr(&w.ctr[C_ERROR], ERR_COLOURS);
+        c = 255u;
+    }
+    vc[k] = c;
+}
+
 template <class G>
 __device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_t* M_out, uint32_t* ncol_out,
                                   bool islands = true) {
@@ -2656,16 +2722,22 @@ __device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_
     } else {
         // Jones-Plassmann over writable bodies == greedy in priority order.
         // A manifold is coloured once every higher-priority neighbour is
-        // (then no lower-priority one is yet).  On one CTA: rounds, a barrier
-        // after each.  On several, no barrier: each thread polls its
-        // manifolds until all are coloured (the highest-priority uncoloured
-        // manifold can always be coloured by its thread, so this ends; the
-        // wait is bounded by kColourTimeoutNs, ERR_TIMEOUT).
+        // (then no lower-priority one is yet).  With a thread for each
+        // manifold, each polls its own (colour_polled).  Else, on one CTA:
+        // rounds, a barrier after each; on several, no barrier: each thread
+        // polls its manifolds until all are coloured (the highest-priority
+        // uncoloured manifold can always be coloured by its thread, so this
+        // ends; the wait is bounded by kColourTimeoutNs, ERR_TIMEOUT).
+        const bool one_each = M <= g.size();
+        if (one_each) {
+            colour_polled(g, w, M);
+            if (!g.sync()) return false;
+        }
         const bool polling = g.nblocks() > 1u;
         const unsigned long long t_start = polling ? global_ns() : 0ull;
         // rounds: three rotating counters at scan[nblocks .. nblocks+3)
         uint32_t* rem = w.scan + g.nblocks();
-        for (uint32_t round = 0;; ++round) {
+        for (uint32_t round = 0; !one_each; ++round) {
             if (!polling && round > M + 1u) {
                 if (g.rank() == 0) atomicOr(&w.ctr[C_ERROR], ERR_COLOURS);
                 break;
@@ -2737,7 +2809,7 @@ __device__ bool phase_constraints(G& g, const WorldDev& w, uint32_t cur, uint32_
             const uint32_t r = *(volatile uint32_t*)&rem[round % 3u];
             if (r == 0u) break;
         }
-        if (polling && !g.sync()) return false;
+        if (!one_each && polling && !g.sync()) return false;
     }
     // 4. colour-major packing + ContactSolver.addManifold (solver.zig:449-491).
     // With owner groups, each colour is packed group by group: group =
