@@ -252,12 +252,13 @@ __global__ void k_export(const DBody* body, const DBodyProp* prop, uint32_t firs
 }
 
 // The pair list of the bodies as they are (vxp_pairs_from_bodies): the step's
-// broad phase alone.  The counters of the last step stay, but for its own two.
+// broad phase alone, with an error word of its own (a step's may wait to be
+// read).  The counters of the last step stay, but for its own two.
 __global__ void __launch_bounds__(512, 1) k_pairs_grid(const __grid_constant__ WorldDev w,
                                                        const __grid_constant__ ColliderSet cs, GridBar* bar,
-                                                       unsigned long long timeout_ns) {
+                                                       uint32_t* err, unsigned long long timeout_ns) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    GridGroup g{bar, &w.ctr[C_ERROR], timeout_ns, gridDim.x};
+    GridGroup g{bar, err, timeout_ns, gridDim.x};
     if (g.rank() == 0) w.ctr[C_BP_HITS] = w.ctr[C_BP_LARGE] = 0u;
     bool overflow = false;  // the host compares the pair count with the buffers
     phase_broadphase(g, w, cs, &overflow, smem_raw);
@@ -1190,10 +1191,11 @@ struct WorldBuffers {
         return VXP_OK;
     }
 
-    // Room for n parts of cut pairs.  own_log: with a buffer of their own for
-    // their candidates (a world of few pairs with very large regions).
-    int ensure_parts(size_t n, bool own_log, std::string& err) {
-        if (part.reserve(2u * n) != cudaSuccess || (own_log && plog.reserve(32u * n) != cudaSuccess)) {
+    // Room for n parts of cut pairs and 32 candidates each: in cp, or, where
+    // few pairs have very large regions, in a buffer of their own.
+    int ensure_parts(size_t n, std::string& err) {
+        if (part.reserve(2u * std::max(n, part.n / 2u)) != cudaSuccess ||
+            (32u * n > cp.bytes() / sizeof(uint2) && plog.reserve(32u * n) != cudaSuccess)) {
             err = fmt("device allocation of %zu pair parts failed", n);
             return VXP_ERR_OOM;
         }
@@ -1221,8 +1223,8 @@ struct WorldBuffers {
         ok &= flag.reserve(cap) == cudaSuccess;
         ok &= clist.reserve(cap) == cudaSuccess;
         ok &= cp.reserve((size_t)CP_NFIELDS * 4 * cap) == cudaSuccess;
-        // parts of cut pairs, four a pair; their candidates go to cp
-        if (int rc = ensure_parts(4u * cap, false, err)) return rc;
+        // parts of cut pairs, four a pair
+        ok &= part.reserve(2u * std::max<size_t>(4u * cap, part.n / 2u)) == cudaSuccess;
         if (spill_rows) ok &= crow.reserve((size_t)CP_NVEL * 4 * cap) == cudaSuccess;
         ok &= isl_keys0.reserve(cap, true) == cudaSuccess;
         ok &= isl_keys1.reserve(cap, true) == cudaSuccess;
@@ -1733,11 +1735,9 @@ int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, floa
     const StepLaunch how = step_launch(ctx, margin);
     // large colliders: room for the parts their pairs may be cut into, a part
     // per 512 voxels of bounds, and for those parts' candidates
-    if (ctx->w.voxels > kClusterVoxels) {
-        const size_t parts = (size_t)std::min<uint64_t>(ctx->w.voxels / 512u, 1u << 18);
-        if (parts > ctx->w.part.n / 2u || !ctx->w.plog.p)
-            if (int rc = ctx->w.ensure_parts(std::max(parts, ctx->w.part.n / 2u), true, ctx->err)) return rc;
-    }
+    if (ctx->w.voxels > kClusterVoxels)
+        if (int rc = ctx->w.ensure_parts((size_t)std::min<uint64_t>(ctx->w.voxels / 512u, 1u << 18), ctx->err))
+            return rc;
     const bool grid = how == StepLaunch::kGrid, one_cluster = how == StepLaunch::kCluster;
     const bool cluster = grid && ctx->solver_flow == VXP_SOLVER_CLUSTER && ctx->cluster_size > 0;
     const uint32_t flow = ctx->solver_flow == VXP_SOLVER_EVENTS ? 1u : 0u;
@@ -1828,15 +1828,16 @@ int compute_device_pairs(vxp_ctx* ctx, float margin, uint32_t* n_out) {
         wd.cfg.bp_cell_bodies = kCellBodiesGrid;
         GridBar* bp = ctx->bar.p;
         const unsigned long long timeout = ctx->wait_limit_ns ? ctx->wait_limit_ns : kGridWaitNs;
-        void* args[] = {(void*)&wd, (void*)&cs, (void*)&bp, (void*)&timeout};
-        CK(cudaMemsetAsync(ctx->bar.p, 0, sizeof(GridBar), ctx->stream));
+        uint32_t* ep = reinterpret_cast<uint32_t*>(ctx->bar.p + 3);
+        void* args[] = {(void*)&wd, (void*)&cs, (void*)&bp, (void*)&ep, (void*)&timeout};
+        CK(cudaMemsetAsync(ctx->bar.p, 0, 4 * sizeof(GridBar), ctx->stream));
         CK(cudaLaunchCooperativeKernel((const void*)k_pairs_grid, dim3(ctx->grid_blocks), dim3(kGridThreads), args,
                                        grid_smem(wd.cache_cap), ctx->stream));
         CK(cudaMemcpyAsync(ctx->h_count + 2, w.n_pairs_dev.p, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaMemcpyAsync(ctx->h_count + 1, w.ctr.p + C_ERROR, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaMemcpyAsync(ctx->h_count + 1, ep, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         total = ctx->h_count[2];
-        if (ctx->h_count[1] & ERR_TIMEOUT) return w.take_error(ctx->stream, ctx->err);
+        if (ctx->h_count[1]) return fail(ctx, VXP_ERR_TIMEOUT, "a grid barrier of the pair list ran out");
         if (total <= w.pair_cap || attempt) break;
         // the list did not fit: grow and run again
         if (int rc = w.ensure_pairs(total, ctx->err)) return rc;
@@ -2129,7 +2130,7 @@ int vxp_create(const vxp_config* cfg, int device, vxp_ctx** out) {
     ctx->solver_flow = ctx->cluster_size ? VXP_SOLVER_CLUSTER : VXP_SOLVER_EVENTS;
     ctx->w.spill_rows = true;
     if (ctx->w.init(cache_cap, ctx->grid_blocks, ctx->err)) return bail(VXP_ERR_OOM);
-    if (ctx->d_world.reserve(1) != cudaSuccess || ctx->bar.reserve(3) != cudaSuccess) return bail(VXP_ERR_OOM);
+    if (ctx->d_world.reserve(1) != cudaSuccess || ctx->bar.reserve(4) != cudaSuccess) return bail(VXP_ERR_OOM);
     if (ctx->w.ensure_pairs(std::max<uint32_t>(cfg->max_pairs, 1024), ctx->err)) return bail(VXP_ERR_OOM);
     if (ctx->w.ensure_bodies(std::max<uint32_t>(cfg->max_bodies, 256), ctx->err)) return bail(VXP_ERR_OOM);
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(VXP_ERR_CUDA);
