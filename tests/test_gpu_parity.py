@@ -463,3 +463,40 @@ def test_broad_phase_by_cells(vxp, n, mode):
         assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"step {s}: bodies differ"
     g.close()
     r.close()
+
+
+@pytest.mark.parametrize("m", [511, 512, 513, 544])
+def test_colours_by_thread_and_in_rounds(vxp, m):
+    """Constraint tables of about as many manifolds as one CTA has threads: up
+    to 512 each thread colours its own, from 513 on they are coloured in
+    rounds; the colours fix the order of the sweeps."""
+    sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=8, seed=5)
+    dt = np.float32(sc.dt)
+    o = O.OracleWorld(substeps=8)
+    o.load_scene(sc)
+    for _ in range(250):
+        o.step(dt, o.pairs())
+    sc.bodies = o.get_bodies()
+    o.close()
+    r = O.OracleWorld(substeps=8, reference_caps=0)
+    r.load_scene(sc)
+    r.narrow_phase(r.pairs())
+    touching = r.manifolds()[:m]
+    r.close()
+    r = O.OracleWorld(substeps=8, reference_caps=0)
+    r.load_scene(sc)
+    pairs = r.pairs()[:m].copy()
+    for name, column in zip(pairs.dtype.names, ("body_a_id", "body_b_id")):
+        pairs[name] = touching[column]
+    g = vxp.VoxelPhysicsSystem(substeps=8, reference_caps=0)
+    g.load_scene(sc)
+    g.set_launch_mode(0)
+    for s in range(2):
+        g.step(dt, pairs)
+        r.step(dt, pairs)
+        if s == 0:
+            assert len(r.manifolds()) == m
+        assert g.manifolds().tobytes() == r.manifolds().tobytes(), f"step {s}: manifolds differ"
+        assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"step {s}: bodies differ"
+    g.close()
+    r.close()
