@@ -375,7 +375,7 @@ def ours(args):
     # bytes), after the grid's constraint table and colouring when those do
     # not run on the cluster (k_solve_grid: no per-unit byte count, time only)
     nb_parts = [alg_bytes(s, substeps, n_dyn_awake, n_nonstatic) for s in stats]
-    grid = n_dyn >= 512
+    grid = all(x[1] > 0.0 for x in part_ms)  # the launch the library chose: one kernel, or the grid's two or three
     cluster = grid and all(x[1] > 0.0 for x in split_ms)
     kernels = {}
     if grid:
@@ -397,7 +397,8 @@ def ours(args):
                                       "frac": b / t / 1e9 / peak})
         dominant = max((k for k in kernels if kernels[k]["achieved"] is not None), key=lambda k: kernels[k]["ms_mean"])
     else:
-        dominant = "k_step_block"
+        # one cluster sweeps with its rows in shared memory too (sweep_path)
+        dominant = "k_step_block" if args.launch_mode == 0 or n_dyn <= 16 else "k_step_cluster"
         kernels[dominant] = {"ms_mean": statistics.mean(kern_ms), "alg_bytes_per_launch": statistics.mean(nb),
                              "achieved": achieved, "frac": achieved / peak}
 

@@ -308,7 +308,8 @@ template <class T> struct DBuf {
 // copy to pageable memory is staged by the driver piece by piece, with a wait
 // in each call.  The driver pins 2 MB at a time (1.2-2.8 ms) and small buffers
 // share a piece, so none takes more than it needs: with 1 MB at least for each,
-// a new context's first edit took 3.3 ms, now 0.7 (later ones 0.6).  Larger copies than kPinnedMost go to the caller's memory directly.
+// a new context's first edit took 3.3 ms, now 0.7 (later ones 0.6).  Larger
+// copies than kPinnedMost go to the caller's memory directly.
 constexpr size_t kPinnedMost = (size_t)32 << 20;
 struct Pinned {
     void* p = nullptr;
