@@ -65,10 +65,10 @@ SOLVER_V, SOLVER_Q = 1, 2
 # carries the commit next to the figure.
 _PILE_PROFILE = "profiles/k_step_grid_k_solve_grid_k_solve_cluster_config2_pile.md"
 PROFILED_TRAFFIC = {
-    ("config2_pile_4096", "k_step_grid"): (54_253_312, _PILE_PROFILE, "d08c536"),
-    ("config2_pile_4096", "k_solve_grid"): (7_303_680, _PILE_PROFILE, "d08c536"),
-    ("config2_pile_4096", "k_solve_cluster"): (4_125_184, _PILE_PROFILE, "8a7312f"),
-    ("config4_stress_512", "k_step_grid"): (755_527_680, "profiles/k_step_grid_config4_stress.md", "d08c536"),
+    ("config2_pile_4096", "k_step_grid"): (36_022_272, _PILE_PROFILE, "29faf74"),
+    ("config2_pile_4096", "k_solve_grid"): (6_544_384, _PILE_PROFILE, "29faf74"),
+    ("config2_pile_4096", "k_solve_cluster"): (4_157_440, _PILE_PROFILE, "29faf74"),
+    ("config4_stress_512", "k_step_grid"): (716_822_272, "profiles/k_step_grid_config4_stress.md", "29faf74"),
 }
 
 

@@ -372,8 +372,8 @@ int vxp_substeps_get(vxp_ctx* ctx, float* out, uint32_t cap_floats, uint32_t* n_
 
 /* Device time (ms) of the last step's kernels: [narrow part, solve part].  A
  * world stepped by the cooperative grid runs them as two kernels
- * (k_step_grid, k_solve_grid); a world stepped by one CTA runs both parts in
- * one kernel, reported in out[0] with out[1] = 0. */
+ * (k_step_grid, k_solve_grid); a world stepped by one CTA or one cluster runs
+ * both parts in one kernel, reported in out[0] with out[1] = 0. */
 int vxp_last_kernel_ms(vxp_ctx* ctx, float out[2]);
 
 /* Step calls queue work on the context's stream and return; a call that

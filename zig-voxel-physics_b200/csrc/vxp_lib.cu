@@ -1917,8 +1917,9 @@ __global__ void k_noalloc_aabbs(const float4* pos, const float4* rot, const floa
     s.mx[i] = make_float4(hi.x, hi.y, hi.z, 0.f);
 }
 
-// Same sweep as k_pairs over caller arrays (ids ascending, so row order is id
-// order).  Pass 0 counts per row, pass 1 writes at the scanned offsets.
+// The sweep of every pair of rows over caller arrays (ids ascending, so row
+// order is id order).  Pass 0 counts per row, pass 1 writes at the scanned
+// offsets.
 __global__ void k_noalloc_pairs(const uint32_t* ids, const uint32_t* types, uint32_t n, unsigned char* base,
                                 uint2* out, uint32_t cap, int pass) {
     const uint32_t sidx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
