@@ -1,0 +1,65 @@
+"""Calls that are refused leave what was there before them as it was."""
+import numpy as np
+import pytest
+
+import oracle_api as O
+
+pytestmark = pytest.mark.gpu
+
+
+def refused_table(vxp, n, statics, why):
+    """A table of n bodies, the first of them static, that set_bodies refuses."""
+    b = np.zeros(n, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = np.arange(1000, 1000 + n)
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["body_type"][:statics] = vxp.abi.BODY_STATIC
+    b["rotation"][:, 3] = 1.0
+    if why == "duplicate id":
+        b["id"][-1] = b["id"][0]
+    else:
+        b["body_type"][-1] = 3
+    return b
+
+
+@pytest.mark.parametrize("why", ["duplicate id", "bad body_type"])
+@pytest.mark.parametrize("n", [29, 200, 300])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_refused_bodies_leave_the_world(vxp, n, why, mode):
+    """27 boxes resting on two static bodies; then a table is refused that is
+    larger than any before it (within the body capacity of 256 and past it),
+    with more static bodies: the bodies read back as they were, and the next
+    steps are the oracle's."""
+    sc = vxp.scenes.config2(mass_fn=O.mass_fn, n_side=3, seed=8)
+    dt = np.float32(sc.dt)
+    settled = O.OracleWorld(substeps=8)
+    settled.load_scene(sc)
+    for _ in range(180):
+        settled.step(dt)
+    assert {1, 2} & {int(m["body_a_id"]) for m in settled.manifolds()}
+    sc.bodies = settled.get_bodies()
+    settled.close()
+    r = O.OracleWorld(substeps=8)
+    r.load_scene(sc)
+    g = vxp.VoxelPhysicsSystem(substeps=8)
+    g.load_scene(sc)
+    g.set_launch_mode(mode)
+    for s in range(3):
+        with pytest.raises(vxp.system.VxpError) as e:
+            g.set_bodies(refused_table(vxp, n, 9, why))
+        assert e.value.code == vxp.abi.VXP_ERR_ARG and why.split()[0] in str(e.value)
+        assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"step {s}: the refused table was felt"
+        pairs = r.pairs()
+        assert g.pairs().tobytes() == pairs.tobytes(), f"step {s}"
+        g.step(dt, pairs)
+        r.step(dt, pairs)
+        assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"step {s}: bodies differ"
+    # an accepted table in another order than its ids'
+    b = r.get_bodies()[::-1].copy()
+    g.set_bodies(b)
+    r.set_bodies(b)
+    for s in range(3):
+        g.step(dt)
+        r.step(dt)
+        assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"reversed table, step {s}: bodies differ"
+    g.close()
+    r.close()

@@ -1317,24 +1317,48 @@ struct WorldBuffers {
         return VXP_OK;
     }
 
-    // The body table, queued on `stream` from a pinned buffer.
-    int set_bodies(const vxp_body* b, uint32_t n, const ColliderStore& cols, UploadRing& up, cudaStream_t stream,
-                   std::string& err) {
+    // What set_bodies refuses, and nothing else: a refused table leaves the
+    // world as it is.  by_id: (id, index) in id order, left empty where the
+    // table is in that order already.  statics: the static bodies.
+    static int check_bodies(const vxp_body* b, uint32_t n, std::vector<uint2>& by_id, uint32_t& statics,
+                            std::string& err) {
+        by_id.clear();
+        statics = 0;
         if (!b && n) {
             err = "null bodies";
             return VXP_ERR_ARG;
         }
-        if (int rc = ensure_bodies(n, err)) return rc;
-        uint32_t statics = 0;
+        bool ascending = true;
         for (uint32_t i = 0; i < n; ++i) {
             if (b[i].body_type > 2u) {
                 err = fmt("body %u: bad body_type %u", i, b[i].body_type);
                 return VXP_ERR_ARG;
             }
             statics += b[i].body_type == 0u ? 1u : 0u;
+            ascending = ascending && (i == 0u || b[i - 1].id < b[i].id);
         }
-        if (pub_cid.reserve(n) != cudaSuccess || pack.reserve(n) != cudaSuccess ||
-            stat.reserve(std::max<uint32_t>(statics, 1)) != cudaSuccess) {
+        if (ascending) return VXP_OK;
+        by_id.resize(n);
+        for (uint32_t i = 0; i < n; ++i) by_id[i] = make_uint2(b[i].id, i);
+        std::sort(by_id.begin(), by_id.end(), [](const uint2& x, const uint2& y) { return x.x < y.x; });
+        for (uint32_t i = 1; i < n; ++i)
+            if (by_id[i].x == by_id[i - 1].x) {
+                err = fmt("duplicate body id %u", by_id[i].x);
+                return VXP_ERR_ARG;
+            }
+        return VXP_OK;
+    }
+
+    // The body table, queued on `stream` from a pinned buffer.
+    int set_bodies(const vxp_body* b, uint32_t n, const ColliderStore& cols, UploadRing& up, cudaStream_t stream,
+                   std::string& err) {
+        std::vector<uint2> by_id;
+        uint32_t statics = 0;
+        if (int rc = check_bodies(b, n, by_id, statics, err)) return rc;
+        if (int rc = ensure_bodies(n, err)) return rc;
+        // (kept when they grow: the table in place stays whole if a later one fails)
+        if (pub_cid.reserve(n, true) != cudaSuccess || pack.reserve(n) != cudaSuccess ||
+            stat.reserve(std::max<uint32_t>(statics, 1), true) != cudaSuccess) {
             err = "body buffers: device allocation failed";
             return VXP_ERR_OOM;
         }
@@ -1382,15 +1406,8 @@ struct WorldBuffers {
             else stl[ns++] = i;  // never moved by a step; ascending
             p.sleeping = s.is_sleeping ? 1u : 0u;
             collider_public[i] = cid[i] = s.collider_id;
-            id[i] = make_uint2(s.id, i);
+            id[i] = by_id.empty() ? make_uint2(s.id, i) : by_id[i];
         }
-        auto by_id = [](const uint2& x, const uint2& y) { return x.x < y.x; };
-        if (!std::is_sorted(id, id + n, by_id)) std::sort(id, id + n, by_id);
-        for (uint32_t i = 1; i < n; ++i)
-            if (id[i].x == id[i - 1].x) {
-                err = fmt("duplicate body id %u", id[i].x);
-                return VXP_ERR_ARG;
-            }
         // the next solve rebuilds its islands: their roots are body indices
         // (IslandManager.markDirty, islands.zig:301-303)
         for (uint32_t k = 0; k < IS_N; ++k) isl[k] = k == IS_DIRTY ? 1u : 0u;
