@@ -280,7 +280,9 @@ int vxp_collider_read(vxp_ctx* ctx, uint32_t collider_id, vxp_collider_info* inf
 int vxp_invalidate_cache_for_body(vxp_ctx* ctx, uint32_t body_id, uint32_t* n_invalidated);
 
 /* Replaces the per-slot body state that step() reads and writes.  Bodies are
- * kept in the order given (the solver's addBody order, src/system.zig:677-681). */
+ * kept in the order given (the solver's addBody order, src/system.zig:677-681).
+ * A table refused with VXP_ERR_ARG (two bodies of one id, an unknown
+ * body_type) leaves the bodies set before as they are. */
 int vxp_bodies_set(vxp_ctx* ctx, const vxp_body* bodies, uint32_t n);
 int vxp_bodies_get(vxp_ctx* ctx, vxp_body* bodies, uint32_t n);
 
@@ -501,8 +503,9 @@ int vxp_batch_invalidate_cache_for_body(vxp_batch* b, uint32_t world, uint32_t b
                                         uint32_t* n_invalidated);
 /* (Re)starts world slot `world` with these bodies: empty contact manager and
  * brick-pair cache.  pair_capacity 0 = 16 x n (grown on demand).  A slot
- * that held a world before reuses its device buffers (zeroed, grown when too
- * small): no allocation, and the same results as a new slot. */
+ * that held a world before reuses its device buffers (reset, grown when too
+ * small): no allocation, and the same results as a new slot.  A table refused
+ * with VXP_ERR_ARG leaves the slot as it was. */
 int vxp_batch_world_set(vxp_batch* b, uint32_t world, const vxp_body* bodies, uint32_t n, uint32_t pair_capacity);
 /* Empties the slot; its device memory stays with it for the next world set
  * there (vxp_batch_world_release frees it). */

@@ -63,3 +63,42 @@ def test_refused_bodies_leave_the_world(vxp, n, why, mode):
         assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"reversed table, step {s}: bodies differ"
     g.close()
     r.close()
+
+
+@pytest.mark.parametrize("why", ["duplicate id", "bad body_type"])
+@pytest.mark.parametrize("n", [20, 400])
+def test_refused_batch_world_leaves_the_slot(vxp, n, why):
+    """A table refused for a stepped slot of a batch, smaller and larger than
+    the slot's buffers: the slot's world and its neighbour's step on as the
+    oracle's do; refused for an empty slot, the slot stays empty."""
+    dt = np.float32(1 / 60)
+    rng = np.random.default_rng(12)
+    worlds = [vxp.scenes.world_for_batch(rng, k, O.mass_fn) for k in (30, 12)]
+    b = vxp.VoxelWorldBatch(3, substeps=4)
+    refs = []
+    for i, sc in enumerate(worlds):
+        b.load_scene(i, sc, collider_offset=1000 * (i + 1))
+        r = O.OracleWorld(substeps=4)
+        r.load_scene(sc)
+        refs.append(r)
+    touching = 0
+    for s in range(130):
+        if s in (110, 120):
+            for w in (0, 2):
+                with pytest.raises(vxp.system.VxpError) as e:
+                    b.set_world(w, refused_table(vxp, n, 9, why))
+                assert e.value.code == vxp.abi.VXP_ERR_ARG and why.split()[0] in str(e.value)
+            assert b.lib.vxp_batch_world_bytes(b.b, 2) == 0
+        b.step(dt)
+        b.synchronize()
+        for r in refs:
+            r.step(dt)
+        touching += s >= 110 and len(refs[0].manifolds()) > 0
+        if s >= 109:
+            for i, r in enumerate(refs):
+                got, want = b.get_world(i), r.get_bodies()
+                for f in got.dtype.names:
+                    if f != "collider_id":
+                        assert got[f].tobytes() == want[f].tobytes(), f"step {s}, world {i}: {f} differs"
+    assert touching >= 10, "the refusals fell into free flight"
+    b.close()

@@ -1317,13 +1317,14 @@ struct WorldBuffers {
         return VXP_OK;
     }
 
-    // What set_bodies refuses, and nothing else: a refused table leaves the
-    // world as it is.  by_id: (id, index) in id order, left empty where the
-    // table is in that order already.  statics: the static bodies.
-    static int check_bodies(const vxp_body* b, uint32_t n, std::vector<uint2>& by_id, uint32_t& statics,
-                            std::string& err) {
-        by_id.clear();
-        statics = 0;
+    // What a table of bodies is refused for, found before anything of the
+    // world changes: a refused table leaves the world as it is.
+    struct BodyOrder {
+        std::vector<uint2> by_id;  // (id, index) in id order, empty where the table is in that order already
+        uint32_t statics = 0;      // static bodies
+    };
+    static int check_bodies(const vxp_body* b, uint32_t n, BodyOrder& order, std::string& err) {
+        std::vector<uint2>& by_id = order.by_id;
         if (!b && n) {
             err = "null bodies";
             return VXP_ERR_ARG;
@@ -1334,7 +1335,7 @@ struct WorldBuffers {
                 err = fmt("body %u: bad body_type %u", i, b[i].body_type);
                 return VXP_ERR_ARG;
             }
-            statics += b[i].body_type == 0u ? 1u : 0u;
+            order.statics += b[i].body_type == 0u ? 1u : 0u;
             ascending = ascending && (i == 0u || b[i - 1].id < b[i].id);
         }
         if (ascending) return VXP_OK;
@@ -1349,12 +1350,10 @@ struct WorldBuffers {
         return VXP_OK;
     }
 
-    // The body table, queued on `stream` from a pinned buffer.
-    int set_bodies(const vxp_body* b, uint32_t n, const ColliderStore& cols, UploadRing& up, cudaStream_t stream,
-                   std::string& err) {
-        std::vector<uint2> by_id;
-        uint32_t statics = 0;
-        if (int rc = check_bodies(b, n, by_id, statics, err)) return rc;
+    // The body table (checked), queued on `stream` from a pinned buffer.
+    int set_bodies(const vxp_body* b, uint32_t n, const BodyOrder& order, const ColliderStore& cols, UploadRing& up,
+                   cudaStream_t stream, std::string& err) {
+        const uint32_t statics = order.statics;
         if (int rc = ensure_bodies(n, err)) return rc;
         // (kept when they grow: the table in place stays whole if a later one fails)
         if (pub_cid.reserve(n, true) != cudaSuccess || pack.reserve(n) != cudaSuccess ||
@@ -1406,7 +1405,7 @@ struct WorldBuffers {
             else stl[ns++] = i;  // never moved by a step; ascending
             p.sleeping = s.is_sleeping ? 1u : 0u;
             collider_public[i] = cid[i] = s.collider_id;
-            id[i] = by_id.empty() ? make_uint2(s.id, i) : by_id[i];
+            id[i] = order.by_id.empty() ? make_uint2(s.id, i) : order.by_id[i];
         }
         // the next solve rebuilds its islands: their roots are body indices
         // (IslandManager.markDirty, islands.zig:301-303)
@@ -2217,8 +2216,10 @@ int vxp_invalidate_cache_for_body(vxp_ctx* ctx, uint32_t body_id, uint32_t* n_in
 
 int vxp_bodies_set(vxp_ctx* ctx, const vxp_body* b, uint32_t n) {
     if (!ctx) return VXP_ERR_ARG;
+    WorldBuffers::BodyOrder order;
+    if (int rc = WorldBuffers::check_bodies(b, n, order, ctx->err)) return rc;
     if (n > ctx->w.body_cap) CK(cudaStreamSynchronize(ctx->stream));  // buffers are replaced
-    return ctx->w.set_bodies(b, n, ctx->cols, ctx->up, ctx->stream, ctx->err);
+    return ctx->w.set_bodies(b, n, order, ctx->cols, ctx->up, ctx->stream, ctx->err);
 }
 
 // vxp_bodies_export / vxp_batch_world_export on one world's buffers.
@@ -2994,6 +2995,8 @@ int vxp_batch_invalidate_cache_for_body(vxp_batch* bt, uint32_t world, uint32_t 
 
 int vxp_batch_world_set(vxp_batch* bt, uint32_t world, const vxp_body* bodies, uint32_t n, uint32_t pair_capacity) {
     if (!bt || world >= bt->slots.size()) return bfail(bt, VXP_ERR_ARG, "world index out of range");
+    WorldBuffers::BodyOrder order;
+    if (int rc = WorldBuffers::check_bodies(bodies, n, order, bt->err)) return rc;  // the slot stays as it is
     auto& slot = bt->slots[world];
     const uint32_t want = pair_capacity ? pair_capacity : std::max<uint32_t>(1024, 16u * n);
     // a fresh world starts with an empty contact manager and cache; a slot
@@ -3010,7 +3013,7 @@ int vxp_batch_world_set(vxp_batch* bt, uint32_t world, const vxp_body* bodies, u
         if (int rc = slot->init(bt->cache_cap, 1, bt->err)) return rc;
     }
     slot->live = true;
-    if (int rc = slot->set_bodies(bodies, n, bt->cols, bt->up, bt->stream, bt->err)) return rc;
+    if (int rc = slot->set_bodies(bodies, n, order, bt->cols, bt->up, bt->stream, bt->err)) return rc;
     if (int rc = slot->ensure_pairs(want, bt->err)) return rc;
     bt->active[world] = n ? 1 : 0;
     bt->est_ms[world] = 0.0f;
