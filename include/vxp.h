@@ -505,7 +505,8 @@ int vxp_batch_invalidate_cache_for_body(vxp_batch* b, uint32_t world, uint32_t b
  * brick-pair cache.  pair_capacity 0 = 16 x n (grown on demand).  A slot
  * that held a world before reuses its device buffers (reset, grown when too
  * small): no allocation, and the same results as a new slot.  A table refused
- * with VXP_ERR_ARG leaves the slot as it was. */
+ * with VXP_ERR_ARG leaves the slot as it was; after any other error the slot
+ * is empty and its device memory freed. */
 int vxp_batch_world_set(vxp_batch* b, uint32_t world, const vxp_body* bodies, uint32_t n, uint32_t pair_capacity);
 /* Empties the slot; its device memory stays with it for the next world set
  * there (vxp_batch_world_release frees it). */

@@ -102,3 +102,62 @@ def test_refused_batch_world_leaves_the_slot(vxp, n, why):
                         assert got[f].tobytes() == want[f].tobytes(), f"step {s}, world {i}: {f} differs"
     assert touching >= 10, "the refusals fell into free flight"
     b.close()
+
+
+@pytest.mark.parametrize("fresh", [False, True])
+def test_batch_world_without_memory_leaves_an_empty_slot(vxp, fresh):
+    """A world whose pair buffers no GPU holds (2^28 pairs, about 400 GB), for
+    a stepped slot and for one that never held a world: the slot is empty
+    afterwards and out of the launches, its neighbour steps on as the oracle's
+    world does, and the slot takes the next world."""
+    dt = np.float32(1 / 60)
+    rng = np.random.default_rng(13)
+    worlds = [vxp.scenes.world_for_batch(rng, k, O.mass_fn) for k in (12, 25)]
+    tables = []
+    b = vxp.VoxelWorldBatch(2, substeps=4)
+    for i, sc in enumerate(worlds):
+        for c in sc.colliders:
+            b.add_collider(1000 * i + c.id, c.voxel_size, c.bricks)
+        t = sc.bodies.copy()
+        t["collider_id"] += 1000 * i
+        tables.append(t)
+    refs = [O.OracleWorld(substeps=4) for _ in worlds]
+    for r, sc in zip(refs, worlds):
+        r.load_scene(sc)
+
+    def check(i):
+        got, want = b.get_world(i), refs[i].get_bodies()
+        for f in got.dtype.names:
+            if f != "collider_id":
+                assert got[f].tobytes() == want[f].tobytes(), f"world {i}: {f} differs"
+
+    b.set_world(1, tables[1])
+    if not fresh:
+        b.set_world(0, tables[0])
+    for _ in range(90):
+        b.step(dt)
+        refs[1].step(dt)
+    b.synchronize()
+    with pytest.raises(vxp.system.VxpError) as e:
+        b.set_world(0, tables[0], pair_capacity=1 << 28)
+    assert e.value.code == vxp.abi.VXP_ERR_OOM
+    assert b.lib.vxp_batch_world_bytes(b.b, 0) == 0
+    out = np.zeros(len(tables[0]), dtype=vxp.abi.BODY_DTYPE)
+    assert b.lib.vxp_batch_world_get(b.b, 0, vxp.abi.ptr(out), len(out)) != 0
+    b.times()  # the last step's launch table is gone with the slot
+    check(1)
+    for _ in range(10):
+        b.step(dt)
+        refs[1].step(dt)
+    b.synchronize()
+    check(1)
+    b.set_world(0, tables[0])
+    for _ in range(70):
+        b.step(dt)
+        for r in refs:
+            r.step(dt)
+    b.synchronize()
+    b.times()
+    check(0)
+    check(1)
+    b.close()

@@ -293,7 +293,10 @@ template <class T> struct DBuf {
         T* q = nullptr;
         const size_t bytes = std::max<size_t>(k, 1) * sizeof(T);
         cudaError_t e = cudaMalloc(&q, bytes);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            cudaGetLastError();  // reported by the caller, and no later launch's error
+            return e;
+        }
         cudaMemset(q, 0, bytes);
         if (keep && p && n) cudaMemcpy(q, p, n * sizeof(T), cudaMemcpyDeviceToDevice);
         if (p) cudaFree(p);
@@ -2999,25 +3002,38 @@ int vxp_batch_world_set(vxp_batch* bt, uint32_t world, const vxp_body* bodies, u
     if (int rc = WorldBuffers::check_bodies(bodies, n, order, bt->err)) return rc;  // the slot stays as it is
     auto& slot = bt->slots[world];
     const uint32_t want = pair_capacity ? pair_capacity : std::max<uint32_t>(1024, 16u * n);
-    // a fresh world starts with an empty contact manager and cache; a slot
-    // that held an earlier world keeps its buffers (no allocation, no free,
-    // which would wait for the whole device), reset behind the steps queued
-    if (slot) {
-        if (n > slot->body_cap || want > slot->pair_cap) BK(cudaStreamSynchronize(bt->stream));
-        BK(slot->reset(bt->stream));
-        slot->n_bodies = 0;
-        slot->collider_public.clear();
-    } else {
-        BK(cudaStreamSynchronize(bt->stream));
-        slot.reset(new WorldBuffers);
-        if (int rc = slot->init(bt->cache_cap, 1, bt->err)) return rc;
+    // Out of every launch until the new world is whole: a step between would
+    // run the old record, whose buffers the new world's may replace.
+    bt->active[world] = 0;
+    bt->rebuild = true;
+    auto fill = [&]() -> int {
+        // a fresh world starts with an empty contact manager and cache; a slot
+        // that held an earlier world keeps its buffers (no allocation, no free,
+        // which would wait for the whole device), reset behind the steps queued
+        if (slot) {
+            if (n > slot->body_cap || want > slot->pair_cap) BK(cudaStreamSynchronize(bt->stream));
+            BK(slot->reset(bt->stream));
+            slot->n_bodies = 0;
+            slot->collider_public.clear();
+        } else {
+            BK(cudaStreamSynchronize(bt->stream));
+            slot.reset(new WorldBuffers);
+            if (int rc = slot->init(bt->cache_cap, 1, bt->err)) return rc;
+        }
+        if (int rc = slot->set_bodies(bodies, n, order, bt->cols, bt->up, bt->stream, bt->err)) return rc;
+        return slot->ensure_pairs(want, bt->err);
+    };
+    if (int rc = fill()) {
+        // the slot may hold some of its buffers and not others: it gives them
+        // back and is empty, and so does the launch table that names them
+        cudaStreamSynchronize(bt->stream);
+        slot.reset();
+        bt->order.clear();
+        return rc;
     }
     slot->live = true;
-    if (int rc = slot->set_bodies(bodies, n, order, bt->cols, bt->up, bt->stream, bt->err)) return rc;
-    if (int rc = slot->ensure_pairs(want, bt->err)) return rc;
     bt->active[world] = n ? 1 : 0;
     bt->est_ms[world] = 0.0f;
-    bt->rebuild = true;
     return VXP_OK;
 }
 
