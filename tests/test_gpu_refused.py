@@ -161,3 +161,22 @@ def test_batch_world_without_memory_leaves_an_empty_slot(vxp, fresh):
     check(0)
     check(1)
     b.close()
+
+
+def test_times_after_a_world_is_released(vxp):
+    """The per-world times of the last step outlive the buffers of a world
+    released since (the launch table that names them does not)."""
+    rng = np.random.default_rng(14)
+    b = vxp.VoxelWorldBatch(3, substeps=4)
+    for i, sc in enumerate(vxp.scenes.world_for_batch(rng, k, O.mass_fn) for k in (12, 20, 16)):
+        b.load_scene(i, sc, collider_offset=1000 * (i + 1))
+    b.step(np.float32(1 / 60), 3)
+    b.release_world(1)
+    total, per = b.times()
+    assert total > 0 and per[0] > 0 and per[2] > 0 and per[1] == 0
+    b.synchronize()
+    b.step(np.float32(1 / 60), 1)
+    b.synchronize()
+    _, per = b.times()
+    assert per[0] > 0 and per[2] > 0 and per[1] == 0
+    b.close()

@@ -3048,6 +3048,11 @@ int vxp_batch_world_clear(vxp_batch* bt, uint32_t world) {
 int vxp_batch_world_release(vxp_batch* bt, uint32_t world) {
     if (!bt || world >= bt->slots.size()) return bfail(bt, VXP_ERR_ARG, "world index out of range");
     BK(cudaStreamSynchronize(bt->stream));
+    // the launch table names the buffers about to be freed: the last step's
+    // times are taken from it now, and it is gone until the next step
+    if (bt->slots[world] && !bt->order.empty())
+        if (int rc = vxp_batch_times(bt, nullptr, nullptr, 0)) return rc;
+    bt->order.clear();
     bt->slots[world].reset();
     bt->active[world] = 0;
     bt->rebuild = true;
