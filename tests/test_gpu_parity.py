@@ -500,3 +500,41 @@ def test_colours_by_thread_and_in_rounds(vxp, m):
         assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"step {s}: bodies differ"
     g.close()
     r.close()
+
+
+@pytest.mark.parametrize("z0", [127070, -127071, 3])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_bricks_far_along_an_axis(vxp, z0, mode):
+    """Colliders of 130 x 130 brick cells a layer whose bricks lie on both
+    sides of |z| = 127 070, where cell numbers counted from the collider's
+    origin pass 2^31 (and near the origin): manifolds and counters are the
+    oracle's."""
+    vs = np.float32(0.125)
+    corners = [(0, 0, 0), (127, 127, 0), (0, 0, 1), (127, 0, 2), (63, 64, 1)]
+    bricks = np.zeros(len(corners), dtype=vxp.abi.BRICK_DTYPE)
+    bricks["pos"] = np.array(corners) + (0, 0, z0)
+    bricks["voxels"] = vxp.scenes.readme_box(8)["voxels"][0]
+    b = np.zeros(2, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = (1, 2)
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["collider_id"] = 7
+    b["rotation"][:, 3] = 1.0
+    b["inv_mass"] = 1.0
+    b["position"][0] = (0.0, 0.0, -z0)
+    b["position"][1] = (0.4, 0.85, -z0 + 0.1)
+    pair = np.array([(1, 2)], dtype=vxp.abi.PAIR_DTYPE)
+    g = vxp.VoxelPhysicsSystem(use_brick_sat=0)
+    r = O.OracleWorld(use_brick_sat=0)
+    for w in (g, r):
+        w.add_collider(7, vs, bricks)
+        w.set_bodies(b)
+    g.set_launch_mode(mode)
+    g.narrow_phase(pair)
+    r.narrow_phase(pair)
+    gs, rs = g.stats(), r.stats()
+    assert rs["manifolds"] == 1 and rs["candidates"] > 100
+    for k in STAT_KEYS:
+        assert gs[k] == rs[k], f"stats[{k}] gpu {gs[k]} oracle {rs[k]}"
+    assert g.manifolds().tobytes() == r.manifolds().tobytes()
+    g.close()
+    r.close()

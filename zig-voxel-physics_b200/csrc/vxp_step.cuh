@@ -1799,9 +1799,13 @@ __device__ __forceinline__ void probe_range(const WorldDev& w, const ColliderSet
     const DCollider& ca = *geo.ca;
     const DCollider& cb = *geo.cb;
     // A's bricks: the region lies in A's bounds, which the brick grid covers
-    // with a brick to spare, so a lookup needs no bounds test
-    const int32_t bdx = ca.bdim[0], bdxy = bdx * ca.bdim[1];
-    const int32_t* agrid = cs.grid + ca.grid_off - (ca.bmin[0] + bdx * ca.bmin[1] + bdxy * ca.bmin[2]);
+    // with a brick to spare, so a lookup needs no bounds test.  A cell is
+    // bdx, bdxy and 1 times the brick coordinates, less the same of the grid's
+    // corner; far from the collider's origin each product passes 2^31, and in
+    // unsigned arithmetic their difference is still the cell.
+    const uint32_t bdx = (uint32_t)ca.bdim[0], bdxy = bdx * (uint32_t)ca.bdim[1];
+    const uint32_t corner = (uint32_t)ca.bmin[0] + bdx * (uint32_t)ca.bmin[1] + bdxy * (uint32_t)ca.bmin[2];
+    const int32_t* agrid = cs.grid + ca.grid_off;
     const uint8_t* avox = cs.vox + (size_t)ca.brick_off * 512u;
     const bool table = cb.nb_off != kNoTable;
     const uint4* btab = cs.nb + cb.nb_off;
@@ -1842,7 +1846,8 @@ __device__ __forceinline__ void probe_range(const WorldDev& w, const ColliderSet
     auto fetch = [&](unsigned long long l) {
         Vox v{nat, kEmpty};
         if (l < end) {
-            const int32_t slot = __ldg(agrid + (nat.x >> 3) + bdx * (nat.y >> 3) + bdxy * (nat.z >> 3));
+            const uint32_t cell = (uint32_t)(nat.x >> 3) + bdx * (uint32_t)(nat.y >> 3) + bdxy * (uint32_t)(nat.z >> 3);
+            const int32_t slot = __ldg(agrid + (cell - corner));
             if (slot >= 0)
                 v.v = __ldg(avox + (size_t)(uint32_t)slot * 512u +
                             (uint32_t)((nat.x & 7) + 8 * (nat.y & 7) + 64 * (nat.z & 7)));
