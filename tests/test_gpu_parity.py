@@ -538,3 +538,44 @@ def test_bricks_far_along_an_axis(vxp, z0, mode):
     assert g.manifolds().tobytes() == r.manifolds().tobytes()
     g.close()
     r.close()
+
+
+@pytest.mark.parametrize("angle", [0.0, 1e-3, 0.4])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_overlap_region_past_2_27_voxels(vxp, angle, mode):
+    """Two sparse colliders of 520^3 voxels of bounds, deep in one another: the
+    overlap region is shared out among the warps like any other large one (one
+    warp alone would outlast the wait limit that the grid launch is given), and
+    gives the oracle's contacts."""
+    rng = np.random.default_rng(16)
+    pos = np.unique(np.concatenate([rng.integers(0, 65, size=(300, 3)), [(0, 0, 0), (64, 64, 64)]]), axis=0)
+    _, first = np.unique(vxp.scenes.hash_brick_pos(*pos.T), return_index=True)
+    bricks = np.zeros(len(first), dtype=vxp.abi.BRICK_DTYPE)
+    bricks["pos"] = pos[np.sort(first)]
+    bricks["voxels"] = vxp.scenes.readme_box(8)["voxels"][0]
+    b = np.zeros(2, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = (1, 2)
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["collider_id"] = 7
+    b["inv_mass"] = 1.0
+    b["rotation"][:, 3] = 1.0
+    b["rotation"][1] = (0.0, 0.0, np.sin(angle / 2), np.cos(angle / 2))
+    b["position"][1] = (0.03, 0.02, 0.01)
+    pair = np.array([(1, 2)], dtype=vxp.abi.PAIR_DTYPE)
+    g = vxp.VoxelPhysicsSystem(use_brick_sat=0)
+    r = O.OracleWorld(use_brick_sat=0)
+    for w in (g, r):
+        w.add_collider(7, 0.1, bricks)
+        w.set_bodies(b)
+    g.set_launch_mode(mode)
+    g.set_wait_limit_ns(500_000_000)
+    r.narrow_phase(pair)
+    for _ in range(2):  # contacts of the first one warm-start the second
+        g.narrow_phase(pair)
+        gs, rs = g.stats(), r.stats()
+        assert rs["manifolds"] == 1 and rs["candidates"] > 50
+        for k in STAT_KEYS[:5]:
+            assert gs[k] == rs[k], f"stats[{k}] gpu {gs[k]} oracle {rs[k]}"
+        assert g.manifolds().tobytes() == r.manifolds().tobytes()
+    g.close()
+    r.close()

@@ -888,6 +888,9 @@ __device__ bool phase_broadphase(G& g, const WorldDev& w, const ColliderSet& cs,
 // Phase: pairs (system.narrowPhase filter + processPair head)
 // ---------------------------------------------------------------------------
 constexpr uint32_t kMaxParts = 32, kMaxPartVoxels = 1024;
+// A part's log names a voxel by its place in the part, in 27 bits.
+constexpr unsigned long long kMaxCutVoxels = (unsigned long long)kMaxParts << 27;
+static_assert(kMaxCutVoxels == 1ull << 32, "a voxel's place in the region is 32 bits");
 template <class G>
 __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint32_t cur) {
     const uint32_t P = g.n_pairs;
@@ -986,7 +989,7 @@ __device__ bool phase_pairs(G& g, const WorldDev& w, const ColliderSet& cs, uint
                                              (unsigned long long)(rmax.y - rmin.y + 1) *
                                              (unsigned long long)(rmax.z - rmin.z + 1);
                 uint32_t parts = 0;
-                if (w.cfg.heavy_voxels && V >= w.cfg.heavy_voxels && V < (1ull << 27) && !w.cfg.dump_candidates) {
+                if (w.cfg.heavy_voxels && V >= w.cfg.heavy_voxels && V <= kMaxCutVoxels && !w.cfg.dump_candidates) {
                     const uint32_t len = max(32u, min(kMaxPartVoxels, w.cfg.heavy_voxels / 4u));
                     parts = (uint32_t)min((unsigned long long)kMaxParts, (V + len - 1u) / len);
                     pi.parts = parts;
@@ -1646,7 +1649,7 @@ constexpr uint32_t kLanePens = 8;
 // Per-warp shared state of phase_probe.
 struct WarpManifold {
     ContactRec c[4];              // the pair's contacts, built when it ends
-    uint2 log[kPartLog];          // (penetration, A voxel | probe << 27) of a part's entering candidates
+    uint2 log[kPartLog];          // (penetration, A voxel of the part | probe << 27): its entering candidates
     float pens[kLanePens][32];
     unsigned long long fid[4];    // feature ids of the manifold's slots (regions wider than their 16 bits)
 };
@@ -1977,7 +1980,7 @@ __device__ __forceinline__ void probe_range(const WorldDev& w, const ColliderSet
             const uint32_t cli = (uint32_t)base + src;
             candidate_add(geo, sm, m, cpen, cli, ck);
             if (lane == src) {
-                if (logged < kPartLog) sm.log[logged] = make_uint2(__float_as_uint(cpen), cli | (ck << 27));
+                if (logged < kPartLog) sm.log[logged] = make_uint2(__float_as_uint(cpen), (cli - (uint32_t)first) | (ck << 27));
                 keep &= keep - 1u;
                 ++j;
                 pen = next_pen();
@@ -2118,7 +2121,7 @@ __device__ __forceinline__ void probe_item(const WorldDev& w, const ColliderSet&
                     const uint32_t src = __ffs(who) - 1;
                     const float cpen = __shfl_sync(0xffffffffu, pen, src);
                     const uint32_t rec = __shfl_sync(0xffffffffu, r.y, src);
-                    candidate_add(g, sm, m, cpen, rec & 0x7FFFFFFu, rec >> 27);
+                    candidate_add(g, sm, m, cpen, (uint32_t)(len * q) + (rec & 0x7FFFFFFu), rec >> 27);
                     if (lane <= src) pen = -__int_as_float(0x7f800000);
                 }
             }
