@@ -579,3 +579,47 @@ def test_overlap_region_past_2_27_voxels(vxp, angle, mode):
         assert g.manifolds().tobytes() == r.manifolds().tobytes()
     g.close()
     r.close()
+
+
+@pytest.mark.parametrize("tables", [True, False])
+@pytest.mark.parametrize("origin", [(0, 0, 0), (-2, -1, -3), (5, -4, 2)])
+def test_probe_masks_of_random_voxels(vxp, origin, tables):
+    """Colliders of 3 x 3 x 3 bricks with every voxel type at random, a third of
+    the bricks missing: the probe masks, from the table and from the bricks,
+    around centres in and between bricks, give the oracle's contacts and
+    counters."""
+    rng = np.random.default_rng(sum(origin) + 20)
+    cells = np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    g = vxp.VoxelPhysicsSystem(use_brick_sat=0)
+    r = O.OracleWorld(use_brick_sat=0)
+    g.set_probe_tables(tables)
+    n = 6
+    for c in range(n):
+        pos = cells[rng.permutation(27)[:18]] + origin
+        _, first = np.unique(vxp.scenes.hash_brick_pos(*pos.T), return_index=True)
+        bricks = np.zeros(len(first), dtype=vxp.abi.BRICK_DTYPE)
+        bricks["pos"] = pos[first]
+        t = rng.integers(0, 5, size=(len(first), 512), dtype=np.uint8)
+        bricks["voxels"] = np.where(t, t | (rng.integers(0, 26, size=t.shape, dtype=np.uint8) << 3), 0)
+        for w in (g, r):
+            w.add_collider(c, 0.1, bricks)
+    b = np.zeros(n, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = np.arange(1, n + 1)
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["collider_id"] = np.arange(n)
+    b["inv_mass"] = 1.0
+    b["rotation"] = vxp.scenes.shoemake_quat(rng, n)
+    b["rotation"][0] = (0, 0, 0, 1)
+    middle = np.tile((np.array(origin) * 8 + 12) * 0.1, (n, 1))
+    b["position"] = vxp.scenes.origin_for_centre(rng.uniform(-1.0, 1.0, size=(n, 3)), b["rotation"], middle)
+    pairs = np.array([(i + 1, j + 1) for i in range(n) for j in range(i + 1, n)], dtype=vxp.abi.PAIR_DTYPE)
+    for w in (g, r):
+        w.set_bodies(b)
+        w.narrow_phase(pairs)
+    gs, rs = g.stats(), r.stats()
+    assert rs["manifolds"] > 5 and rs["candidates"] > 1000
+    for k in STAT_KEYS:
+        assert gs[k] == rs[k], f"stats[{k}] gpu {gs[k]} oracle {rs[k]}"
+    assert g.manifolds().tobytes() == r.manifolds().tobytes()
+    g.close()
+    r.close()

@@ -1495,26 +1495,55 @@ __device__ void generate_contact(const ProbeCtx& c, uint32_t va, I3 ia, F3 wa, u
 // The masks of the 27 probes of checkNeighborhood (narrow_phase.zig:796-857)
 // around B's voxel cbv, bit dz*9 + dy*3 + dx (offsets from -1), clipped to B's
 // voxel bounds (a probe outside them is skipped, isValidCoord): non-empty,
-// corner, corner or edge, inside.  From B's table; without one, by the same
-// 27 lookups that build a table entry.
+// corner, corner or edge, inside.  From B's table; without one, from the nine
+// rows of three voxels: the rows in the centre's brick share its grid cell, a
+// row is one load of the brick's eight voxels, and its three types are tested
+// side by side, a byte each.  (Deep plates of 512 x 512 voxels without tables
+// on one CTA: 27 lookups of a cell and a voxel each 34.3 ms, so 21.2.)
 __device__ __noinline__ uint4 probe_masks_lookup(const ColliderSet& cs, const DCollider& cb, I3 cbv) {
-    uint32_t ne = 0u, co = 0u, ec = 0u, in = 0u;
-    for (int32_t dz = -1; dz <= 1; ++dz)
-        for (int32_t dy = -1; dy <= 1; ++dy)
-            for (int32_t dx = -1; dx <= 1; ++dx) {
-                // 64-bit: a centre saturated by the float conversion must not wrap
-                const long long bx = (long long)cbv.x + dx, by = (long long)cbv.y + dy, bz = (long long)cbv.z + dz;
-                if (bx < cb.min_bound[0] || bx >= cb.max_bound[0] || by < cb.min_bound[1] || by >= cb.max_bound[1] ||
-                    bz < cb.min_bound[2] || bz >= cb.max_bound[2])
-                    continue;
-                const uint32_t tb = vtype(voxel_at(cs, cb, (int32_t)bx, (int32_t)by, (int32_t)bz));
-                const uint32_t bit = 1u << ((dz + 1) * 9 + (dy + 1) * 3 + (dx + 1));
-                if (tb != kEmpty) ne |= bit;
-                if (tb == kCorner) co |= bit;
-                if (tb == kCorner || tb == kEdge) ec |= bit;
-                if (tb == kInside) in |= bit;
-            }
-    return make_uint4(ne, co, ec, in);
+    const int32_t x = cbv.x, y = cbv.y, z = cbv.z;
+    // 64-bit: a centre saturated by the float conversion must not wrap
+    auto near = [](int32_t v, int32_t lo, int32_t hi) {
+        return (long long)v >= (long long)lo - 1ll && (long long)v <= (long long)hi;
+    };
+    if (!near(x, cb.min_bound[0], cb.max_bound[0]) || !near(y, cb.min_bound[1], cb.max_bound[1]) ||
+        !near(z, cb.min_bound[2], cb.max_bound[2]))
+        return make_uint4(0u, 0u, 0u, 0u);
+    auto in = [](int32_t v, int32_t lo, int32_t hi) { return v >= lo && v < hi; };
+    uint32_t inx = 0u;
+    for (int32_t dx = -1; dx <= 1; ++dx) inx |= (uint32_t)in(x + dx, cb.min_bound[0], cb.max_bound[0]) << (dx + 1);
+    const int32_t cx = x & 7, centre = brick_slot(cs, cb, x >> 3, y >> 3, z >> 3);
+    // bits 3, 11 and 19, set where a byte's low three bits are not zero, as bits 0 to 2
+    auto some = [](uint32_t t) {
+        const uint32_t m = (t + 0x070707u) >> 3 & 0x010101u;
+        return (m | m >> 7 | m >> 14) & 7u;
+    };
+    uint32_t ne = 0u, co = 0u, ec = 0u, ins = 0u;
+    for (int32_t dz = -1; dz <= 1; ++dz) {
+        if (!in(z + dz, cb.min_bound[2], cb.max_bound[2])) continue;
+        for (int32_t dy = -1; dy <= 1; ++dy) {
+            if (!in(y + dy, cb.min_bound[1], cb.max_bound[1])) continue;
+            const int32_t yy = y + dy, zz = z + dz;
+            const bool same = (yy >> 3) == (y >> 3) && (zz >> 3) == (z >> 3);
+            const int32_t slot = same ? centre : brick_slot(cs, cb, x >> 3, yy >> 3, zz >> 3);
+            unsigned long long row = 0ull;
+            if (slot >= 0)
+                row = __ldg(reinterpret_cast<const unsigned long long*>(
+                    cs.vox + (size_t)(cb.brick_off + (uint32_t)slot) * 512u + (uint32_t)(8 * (yy & 7) + 64 * (zz & 7))));
+            uint32_t t;
+            if (cx == 0) t = (uint32_t)row << 8 | voxel_at(cs, cb, x - 1, yy, zz);
+            else if (cx == 7) t = (uint32_t)(row >> 48) | voxel_at(cs, cb, x + 1, yy, zz) << 16;
+            else t = (uint32_t)(row >> (8 * (cx - 1)));
+            t &= 0x070707u;
+            const int sh = (dz + 1) * 9 + (dy + 1) * 3;
+            const uint32_t corner = ~some(t ^ kCorner * 0x010101u) & inx, edge = ~some(t ^ kEdge * 0x010101u) & inx;
+            ne |= (some(t) & inx) << sh;
+            co |= corner << sh;
+            ec |= (corner | edge) << sh;
+            ins |= (~some(t ^ kInside * 0x010101u) & inx) << sh;
+        }
+    }
+    return make_uint4(ne, co, ec, ins);
 }
 
 // floor(p / vs) with the quotient rounded as an IEEE division, through the
