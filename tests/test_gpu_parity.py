@@ -623,3 +623,45 @@ def test_probe_masks_of_random_voxels(vxp, origin, tables):
     assert g.manifolds().tobytes() == r.manifolds().tobytes()
     g.close()
     r.close()
+
+
+def test_pairs_at_changing_margins(vxp):
+    """The pair list by cells with margins in turn, from boxes shrunk past
+    nothing to boxes a cell wide: the oracle's pairs each time, and a list does
+    not take longer for the margin asked for before it (each margin has cells
+    of its own width)."""
+    import time
+
+    cube = vxp.scenes.readme_box(8)
+    n = 18 ** 3
+    rng = np.random.default_rng(17)
+    b = np.zeros(n, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = np.arange(1, n + 1)
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["inv_mass"] = 1.0
+    b["rotation"] = vxp.scenes.shoemake_quat(rng, n)
+    b["position"] = np.stack(np.meshgrid(*[np.arange(18)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)
+    b["position"] += rng.uniform(-0.2, 0.2, size=(n, 3)).astype(np.float32)
+    g = vxp.VoxelPhysicsSystem(max_bodies=n, max_pairs=1 << 20)
+    r = O.OracleWorld()
+    for w in (g, r):
+        w.add_collider(0, 0.1, cube)
+        w.set_bodies(b)
+    for margin in (0.1, -50.0, 0.1, 0.7, -0.2, 0.0):
+        assert g.pairs(margin).tobytes() == r.pairs(margin).tobytes(), f"margin {margin}"
+
+    def median_s(first):
+        g.set_bodies(b)
+        if first is not None:
+            g.pairs(first)
+        out = []
+        for _ in range(7):
+            t0 = time.perf_counter()
+            g.pairs(0.1)
+            out.append(time.perf_counter() - t0)
+        return sorted(out)[3]
+
+    alone = median_s(None)
+    assert median_s(-50.0) < 3 * alone, "the cells are still as wide as the margin before"
+    g.close()
+    r.close()

@@ -554,6 +554,7 @@ struct ColliderStore {
     size_t grid_used = 0, brick_used = 0, nb_used = 0;
     size_t grid_dead = 0, brick_dead = 0, nb_dead = 0;
     uint32_t n_dev = 0;
+    uint64_t placements = 1;  // grows with every placement: what was measured of the colliders is old then
     bool dirty = false;    // colliders wait for placement
     bool replace = false;  // every collider is placed again (tables switched)
     // neighbourhood-mask tables: colliders with at most kNbMaxCentres probe
@@ -915,6 +916,7 @@ struct ColliderStore {
     // writes their records and builds their tables.
     int place(const std::vector<uint32_t>& todo, cudaStream_t s, std::string& err) {
         if (todo.empty()) return VXP_OK;
+        ++placements;
         std::vector<int32_t> grid;
         std::vector<uint8_t> vox;
         std::vector<int4> bpos;
@@ -1100,14 +1102,12 @@ struct WorldBuffers {
     std::vector<uint32_t> collider_public;
     std::vector<uint32_t> moving_collider;  // per non-static body its collider's index
     // of the moving bodies' colliders as placed (measure): the voxels of their
-    // bounds, and the broad phase's cell size
-    bool measured = false;
+    // bounds, and the mean of their boxes' diagonals (0: no moving collider)
+    uint64_t measured = 0;  // the placement of the colliders it was taken from (0: none)
     uint64_t voxels = 0;
-    float bp_cell = 1.0f;
-    // The cell: a quarter wider than the bodies' mean diagonal, so that most of
-    // their boxes, in any rotation, span at most two.
-    void measure(const ColliderStore& cols, float margin) {
-        if (measured) return;
+    double diagonal = 0.0;
+    void measure(const ColliderStore& cols) {
+        if (measured == cols.placements) return;
         uint64_t v = 0;
         double diag = 0.0;
         size_t k = 0;
@@ -1127,9 +1127,15 @@ struct WorldBuffers {
             ++k;
         }
         voxels = v;
-        const double cell = (k ? 1.25 * diag / (double)k : 1.0) + 2.0 * std::fabs((double)margin);
-        bp_cell = std::isfinite(cell) && cell > 1e-6 ? (float)cell : 1.0f;
-        measured = true;
+        diagonal = k ? diag / (double)k : 0.0;
+        measured = cols.placements;
+    }
+    // The broad phase's cell for boxes inflated by this margin: a quarter wider
+    // than the bodies' mean diagonal, so that most of their boxes, in any
+    // rotation, span at most two.
+    float bp_cell(float margin) const {
+        const double cell = (diagonal > 0.0 ? 1.25 * diagonal : 1.0) + 2.0 * std::fabs((double)margin);
+        return std::isfinite(cell) && cell > 1e-6 ? (float)cell : 1.0f;
     }
     DBuf<DBody> body;
     DBuf<DBodyProp> prop;
@@ -1384,7 +1390,7 @@ struct WorldBuffers {
         static_assert(sizeof(DBody) % 16 == 0 && sizeof(DBodyProp) % 8 == 0, "records follow one another");
         collider_public.resize(n);
         moving_collider.clear();
-        measured = false;
+        measured = 0;
         uint32_t ns = 0;
         for (uint32_t i = 0; i < n; ++i) {
             const vxp_body& s = b[i];
@@ -1494,7 +1500,7 @@ struct WorldBuffers {
         w.bp_buckets = body_cap;
         w.bp_mn = bp_mn.p;
         w.bp_mx = bp_mx.p;
-        w.cfg.bp_cell = bp_cell;
+        w.cfg.bp_cell = bp_cell(margin);
         w.bpmask = bp_rows ? bpmask.p : nullptr;
         w.bp_stride = bp_stride;
         w.bp_rows = bp_rows;
@@ -1741,8 +1747,8 @@ constexpr unsigned long long kGridWaitNs = 10ull * 1000ull * 1000ull * 1000ull;
 enum class StepLaunch { kBlock, kCluster, kGrid };
 constexpr uint32_t kBlockBodies = 17, kBlockVoxels = 12 * 1024;
 constexpr uint32_t kClusterBodies = 160, kClusterVoxels = 1024 * 1024;
-StepLaunch step_launch(vxp_ctx* ctx, float margin) {
-    ctx->w.measure(ctx->cols, margin);
+StepLaunch step_launch(vxp_ctx* ctx) {
+    ctx->w.measure(ctx->cols);
     if (ctx->use_grid >= 0) return ctx->use_grid ? StepLaunch::kGrid : StepLaunch::kBlock;
     const uint32_t n = ctx->w.n_bodies;
     if (n <= kBlockBodies && ctx->w.voxels <= kBlockVoxels) return StepLaunch::kBlock;
@@ -1754,7 +1760,7 @@ StepLaunch step_launch(vxp_ctx* ctx, float margin) {
 // Runs the step kernel.  device_pairs: the kernel builds the pair list itself.
 int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, float margin) {
     if (int rc = ctx->cols.sync(ctx->stream, ctx->err)) return rc;
-    const StepLaunch how = step_launch(ctx, margin);
+    const StepLaunch how = step_launch(ctx);
     // large colliders: room for the parts their pairs may be cut into, a part
     // per 512 voxels of bounds, and for those parts' candidates
     if (ctx->w.voxels > kClusterVoxels)
@@ -1844,7 +1850,7 @@ int compute_device_pairs(vxp_ctx* ctx, float margin, uint32_t* n_out) {
         if (int rc = w.ensure_pairs(1024, ctx->err)) return rc;
     uint32_t total = 0;
     for (int attempt = 0;; ++attempt) {
-        w.measure(ctx->cols, margin);
+        w.measure(ctx->cols);
         WorldDev wd = w.make(ctx->cfg, 0.0f, 0u, ctx->solver_div, true, margin, 0u);
         wd.ts = nullptr;  // the last step's times stay
         wd.cfg.bp_cell_bodies = kCellBodiesGrid;
@@ -2184,7 +2190,6 @@ int vxp_last_error(const vxp_ctx* ctx, char* buf, size_t n) {
 int vxp_collider_upload(vxp_ctx* ctx, uint32_t collider_id, float voxel_size, const vxp_brick* bricks,
                         uint32_t n_bricks) {
     if (!ctx) return VXP_ERR_ARG;
-    ctx->w.measured = false;
     return ctx->cols.upload(collider_id, voxel_size, bricks, n_bricks, ctx->err);
 }
 
@@ -2192,7 +2197,6 @@ int vxp_collider_edit(vxp_ctx* ctx, uint32_t collider_id, const int32_t* coords,
                       int mode) {
     if (!ctx) return VXP_ERR_ARG;
     if (mode != VXP_EDIT_SET && mode != VXP_EDIT_OCCUPANCY) return fail(ctx, VXP_ERR_ARG, "unknown edit mode %d", mode);
-    ctx->w.measured = false;
     return ctx->cols.edit(collider_id, coords, values, n, (uint32_t)mode, ctx->stream, ctx->err);
 }
 
@@ -2759,6 +2763,7 @@ struct vxp_batch {
     uint32_t graph_tile = 0, graph_nbig = 0;
     float margin = 0.1f;
     float built_dt = -1.0f;
+    uint64_t built_placements = 0;    // the colliders' placement that d_worlds was measured from
     bool rebuild = true;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -2811,7 +2816,7 @@ __global__ void k_batch_status(const WorldDev* worlds, uint32_t n, uint32_t* out
 // Launch order, device WorldDev array and the graph of one step.
 int batch_prepare(vxp_batch* bt, float dt) {
     if (int rc = bt->cols.sync(bt->stream, bt->err)) return rc;
-    if (bt->rebuild || dt != bt->built_dt) {
+    if (bt->rebuild || dt != bt->built_dt || bt->built_placements != bt->cols.placements) {
         std::vector<uint32_t> ord;
         for (uint32_t s = 0; s < bt->slots.size(); ++s)
             if (bt->active[s] && bt->slots[s]) ord.push_back(s);
@@ -2835,7 +2840,7 @@ int batch_prepare(vxp_batch* bt, float dt) {
         std::vector<WorldDev> wd(ord.size());
         for (size_t i = 0; i < ord.size(); ++i)
         {
-            bt->slots[ord[i]]->measure(bt->cols, bt->margin);
+            bt->slots[ord[i]]->measure(bt->cols);
             wd[i] = bt->slots[ord[i]]->make(bt->cfg, dt, PH_STEP, 128, true, bt->margin, 0u);
             wd[i].cfg.bp_cell_bodies = kCellBodiesBlock;
             wd[i].cfg.block_smem = (uint32_t)block_smem(bt->cache_cap);
@@ -2849,6 +2854,7 @@ int batch_prepare(vxp_batch* bt, float dt) {
                                bt->stream));
         BK(cudaStreamSynchronize(bt->stream));
         bt->built_dt = dt;
+        bt->built_placements = bt->cols.placements;
         bt->rebuild = false;
     }
     const ColliderSet cs = bt->cols.set();
