@@ -41,3 +41,35 @@ def test_substep_states_match_oracle(vxp, mode, solver, colouring):
     assert recorded >= 4 * 40
     g.close()
     r.close()
+
+
+@pytest.mark.parametrize("shared", [None, 24 * 1024, 0])
+@pytest.mark.parametrize("colouring", [1, 0])
+def test_substep_states_on_one_cluster(vxp, colouring, shared):
+    """64 cubes stepped as the library launches them by itself, the whole step
+    on one cluster: with the state of its sweeps in shared memory, with room
+    for less of it, and in L2."""
+    sc = vxp.scenes.config1(O.mass_fn)
+    cfg = dict(substeps=4, colouring=colouring)
+    g = vxp.VoxelPhysicsSystem(**cfg)
+    g.load_scene(sc)
+    assert g.cluster_size() > 0
+    if shared is not None:
+        g.set_cluster_shared_bytes(shared)
+    g.set_substep_record(True)
+    r = O.OracleWorld(**cfg)
+    r.load_scene(sc)
+    r.set_substep_record(True)
+    dt = np.float32(sc.dt)
+    recorded = 0
+    for s in range(80):
+        pairs = r.pairs()
+        g.step(dt, pairs)
+        r.step(dt, pairs)
+        gs, rs = g.substeps(), r.substeps()
+        assert gs.shape == rs.shape and gs.tobytes() == rs.tobytes(), f"step {s}: substep states differ"
+        recorded += gs.shape[0]
+        assert g.get_bodies().tobytes() == r.get_bodies().tobytes(), f"step {s}: bodies differ"
+    assert recorded >= 4 * 40
+    g.close()
+    r.close()

@@ -88,14 +88,18 @@ __global__ void __launch_bounds__(256, 1) k_solve_cluster(const __grid_constant_
 }
 // A whole step of a world too small to fill the GPU on one cluster: one launch
 // and hardware barriers (0.2 us) where the grid's three kernels pay 2 us a
-// barrier and 6 us a launch, and sixteen times the warps of one CTA for the
-// pairs and voxels.
+// barrier and 6 us a launch, and eight times the warps of one CTA (four where
+// the cluster has 8 CTAs) for the pairs and voxels.
 __global__ void __launch_bounds__(kClusterThreads, 1)
     k_step_cluster(const __grid_constant__ WorldDev w, const __grid_constant__ ColliderSet cs, uint32_t smem_bytes) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpManifold* wsm = reinterpret_cast<WarpManifold*>(smem_raw);
     const CacheSmem csm = cache_smem(smem_raw, blockDim.x / 32u, w.cache_cap);
     ClusterGroup g = cluster_group();
+    if (g.ncta != gridDim.x) {  // launch constants: the same verdict in every block
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&w.ctr[C_ERROR], ERR_BOUNDS);
+        return;
+    }
     if (world_step_narrow(g, w, cs, wsm, csm)) world_step_sweeps(g, w, smem_raw, smem_bytes, true);
 }
 
@@ -2145,16 +2149,22 @@ int vxp_create(const vxp_config* cfg, int device, vxp_ctx** out) {
         cudaFuncSetAttribute(k_step_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)ctx->step_cluster_smem) != cudaSuccess)
         ctx->step_cluster_smem = 0;
-    for (uint32_t n : {16u, 8u}) {
+    auto schedules = [&](auto kernel, uint32_t n, uint32_t smem) {
         cudaLaunchConfig_t lc = {};
         cudaLaunchAttribute at[1];
-        cluster_config(&lc, at, n, ctx->cluster_smem, ctx->stream);
+        cluster_config(&lc, at, n, smem, ctx->stream);
         int active = 0;
-        if (cudaOccupancyMaxActiveClusters(&active, k_solve_cluster, &lc) == cudaSuccess && active >= 1) {
+        return cudaOccupancyMaxActiveClusters(&active, kernel, &lc) == cudaSuccess && active >= 1;
+    };
+    for (uint32_t n : {16u, 8u})
+        if (schedules(k_solve_cluster, n, ctx->cluster_smem)) {
             ctx->cluster_size = n;
             break;
         }
-    }
+    // a whole step on one cluster: of the same size, or not at all
+    if (ctx->step_cluster_smem &&
+        (!ctx->cluster_size || !schedules(k_step_cluster, ctx->cluster_size, ctx->step_cluster_smem)))
+        ctx->step_cluster_smem = 0;
     cudaGetLastError();  // a refused size is not an error of this context
     ctx->solver_flow = ctx->cluster_size ? VXP_SOLVER_CLUSTER : VXP_SOLVER_EVENTS;
     ctx->w.spill_rows = true;
