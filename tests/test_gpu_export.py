@@ -98,3 +98,24 @@ def test_batch_world_export(vxp):
         assert e["angular_velocity"].tobytes() == np.ascontiguousarray(b["angular_velocity"]).tobytes()
         assert (e["sleeping"] == b["is_sleeping"]).all()
     bt.close()
+
+
+@pytest.mark.parametrize("fields,n", [([], None), (None, 0), (None, 500), (None, None)])
+def test_export_reports_a_pending_error(vxp, fields, n):
+    """A step left undone for want of pair buffers (200 bodies in one place) is
+    reported by the next export to host memory, also one without a field, one
+    of no bodies and one past the bodies; the report clears it."""
+    b = np.zeros(200, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = np.arange(1, 201)
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["inv_mass"] = 1.0
+    b["rotation"][:, 3] = 1.0
+    g = vxp.VoxelPhysicsSystem(max_pairs=1024)
+    g.add_collider(0, 0.1, vxp.scenes.readme_box(8))
+    g.set_bodies(b)
+    g.step(np.float32(1 / 60))
+    with pytest.raises(vxp.system.VxpError) as e:
+        g.export_state(fields, n=n)
+    assert e.value.code == vxp.abi.VXP_ERR_CAP
+    assert g.export_state(["position"])["position"].tobytes() == b["position"].tobytes()
+    g.close()

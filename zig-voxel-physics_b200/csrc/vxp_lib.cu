@@ -2239,6 +2239,15 @@ int vxp_bodies_set(vxp_ctx* ctx, const vxp_body* b, uint32_t n) {
     return ctx->w.set_bodies(b, n, order, ctx->cols, ctx->up, ctx->stream, ctx->err);
 }
 
+// Whether an export to host memory has anything to copy: one that has not, or
+// that is refused, waits for the stream and reports a pending error all the
+// same.
+static bool export_copies(const WorldBuffers& w, const vxp_state_view* dst, uint32_t first, uint32_t n) {
+    return dst && n && first <= w.n_bodies && n <= w.n_bodies - first &&
+           (dst->position || dst->rotation || dst->linear_velocity || dst->angular_velocity || dst->aabb_min ||
+            dst->aabb_max || dst->sleeping);
+}
+
 // vxp_bodies_export / vxp_batch_world_export on one world's buffers.
 static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_view* dst, uint32_t first,
                         uint32_t n, int device_memory, void* consumer, cudaStream_t stream, int device, Pinned& rd,
@@ -2346,9 +2355,9 @@ static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_
 int vxp_bodies_export(vxp_ctx* ctx, const vxp_state_view* dst, uint32_t first, uint32_t n, int device_memory,
                       void* consumer_stream) {
     if (!ctx) return VXP_ERR_ARG;
-    if (!device_memory && (n == 0 || !dst || first > ctx->w.n_bodies || n > ctx->w.n_bodies - first)) {
+    // (the others read the error word with their copy)
+    if (!device_memory && !export_copies(ctx->w, dst, first, n))
         if (int rc = check_device_error(ctx)) return rc;
-    }
     if (int rc = ctx->cols.sync(ctx->stream, ctx->err)) return rc;
     return export_world(ctx->w, ctx->cols.set(), dst, first, n, device_memory, consumer_stream, ctx->stream,
                         ctx->device, ctx->rd, !device_memory, ctx->err);
@@ -3086,6 +3095,7 @@ int vxp_batch_world_export(vxp_batch* bt, uint32_t world, const vxp_state_view* 
                            int device_memory, void* consumer_stream) {
     if (!bt || world >= bt->slots.size() || !bt->slots[world] || !bt->slots[world]->live)
         return bfail(bt, VXP_ERR_ARG, "no such world");
+    if (!device_memory && !export_copies(*bt->slots[world], dst, first, n)) BK(cudaStreamSynchronize(bt->stream));
     if (int rc = bt->cols.sync(bt->stream, bt->err)) return rc;
     return export_world(*bt->slots[world], bt->cols.set(), dst, first, n, device_memory, consumer_stream, bt->stream,
                         bt->device, bt->rd, false, bt->err);
