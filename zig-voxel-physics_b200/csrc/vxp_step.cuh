@@ -2170,7 +2170,7 @@ __device__ bool phase_probe(G& g, const WorldDev& w, const ColliderSet& cs, uint
     // its SM would slow it more than it is worth), or by one warp of a lone
     // CTA while its other warps start detecting at once
     // (in a cluster too: few CTAs, few lookups)
-    const bool replay_cta = w.cfg.use_cache && G::kWideGrid && g.block() == 0u;
+    const bool replay_cta = w.cfg.use_cache && G::kWideGrid && g.nblocks() > 1u && g.block() == 0u;
     if (replay_cta && w.cache_cap >= 48u &&
         (size_t)(blockDim.x >> 5) * sizeof(WarpManifold) >= cta_replay_scratch_bytes(w.cache_cap)) {
         cache_replay_cta(w, csm, reinterpret_cast<unsigned char*>(warp_sm));
