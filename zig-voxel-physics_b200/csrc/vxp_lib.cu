@@ -2494,13 +2494,15 @@ int vxp_manifolds_get(vxp_ctx* ctx, vxp_manifold* out, uint32_t cap, uint32_t* n
     const uint32_t k = out ? std::min(n, cap) : 0u, piece = (uint32_t)(kPinnedMost / sizeof(ManifoldRec));
     for (uint32_t at = 0; at < k; at += piece) {
         const uint32_t m = std::min(piece, k - at);
+        // (without pinned memory through cp, which is scratch between steps)
+        static_assert(CP_NFIELDS * 4 * sizeof(float) >= sizeof(ManifoldRec), "cp holds a record for every pair");
         void* st = ctx->rd.get(m * sizeof(ManifoldRec));
-        if (!st) return fail(ctx, VXP_ERR_OOM, "pinned memory for %u manifolds", m);
-        k_manifold_pack<<<(m + 7u) / 8u, 256, 0, ctx->stream>>>(w.man0.p, w.man1.p, w.frame.p, w.flag.p + at, m,
-                                                                static_cast<uint32_t*>(st));
+        uint32_t* to = st ? static_cast<uint32_t*>(st) : reinterpret_cast<uint32_t*>(w.cp.p);
+        k_manifold_pack<<<(m + 7u) / 8u, 256, 0, ctx->stream>>>(w.man0.p, w.man1.p, w.frame.p, w.flag.p + at, m, to);
         CK(cudaGetLastError());
+        if (!st) CK(cudaMemcpyAsync(out + at, to, m * sizeof(ManifoldRec), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        std::memcpy(out + at, st, m * sizeof(ManifoldRec));
+        if (st) std::memcpy(out + at, st, m * sizeof(ManifoldRec));
     }
     return VXP_OK;
 }
