@@ -119,3 +119,30 @@ def test_export_reports_a_pending_error(vxp, fields, n):
     assert e.value.code == vxp.abi.VXP_ERR_CAP
     assert g.export_state(["position"])["position"].tobytes() == b["position"].tobytes()
     g.close()
+
+
+def test_large_tables_first_and_later(vxp):
+    """Body tables of more than 1 MB (9000 bodies), which the first calls of a
+    context copy to and from pageable memory and later ones through pinned
+    memory: every byte comes back, in both directions and from an export."""
+    rng = np.random.default_rng(18)
+    n = 9000
+    g = vxp.VoxelPhysicsSystem(max_bodies=n)
+    g.add_collider(0, 0.1, vxp.scenes.readme_box(8))
+    for turn in range(4):
+        b = np.zeros(n, dtype=vxp.abi.BODY_DTYPE)
+        b["id"] = rng.permutation(n) + 1
+        b["body_type"] = rng.integers(0, 3, size=n)
+        b["inv_mass"] = rng.uniform(0.1, 1.0, size=n)
+        b["inv_inertia_local"][:, [0, 4, 8]] = rng.uniform(0.1, 1.0, size=(n, 3))
+        b["position"] = rng.uniform(-500, 500, size=(n, 3))
+        b["linear_velocity"] = rng.uniform(-1, 1, size=(n, 3))
+        b["rotation"] = vxp.scenes.shoemake_quat(rng, n)
+        g.set_bodies(b)
+        if turn != 1:
+            assert g.get_bodies().tobytes() == b.tobytes(), f"turn {turn}"
+        for _ in range(2):
+            out = g.export_state()
+            for f in ("position", "rotation", "linear_velocity"):
+                assert out[f].tobytes() == np.ascontiguousarray(b[f]).tobytes(), f"turn {turn}: {f}"
+    g.close()

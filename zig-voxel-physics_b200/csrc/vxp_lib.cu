@@ -316,16 +316,31 @@ template <class T> struct DBuf {
 // in each call.  The driver pins 2 MB at a time (1.2-2.8 ms) and small buffers
 // share a piece, so none takes more than it needs: with 1 MB at least for each,
 // a new context's first edit took 3.3 ms, now 0.7 (later ones 0.6).  Larger
-// copies than kPinnedMost go to the caller's memory directly.
-constexpr size_t kPinnedMost = (size_t)32 << 20;
+// copies than kPinnedMost go to the caller's memory directly.  So does a
+// context's first body table, and its first one read back, of more than
+// kPinnedAtOnce: pinning costs what many such copies save, and a context may
+// need only one.  First vxp_bodies_set of a new context, pinned at once /
+// pageable: 8000 bodies (1.5 MB) 2.3 / 0.40 ms, 15000 (2.8 MB) 4.5 / 1.0; first
+// vxp_bodies_get of 15000 (1.9 MB) 2.8 / 0.20.  (4000 bodies, 0.75 MB, pinned
+// 0.46, pageable copies 0.65.)
+constexpr size_t kPinnedMost = (size_t)32 << 20, kPinnedAtOnce = (size_t)1 << 20;
 struct Pinned {
     void* p = nullptr;
     size_t n = 0;
+    bool large_before = false;  // more than kPinnedAtOnce was asked of wait_and_see
     Pinned() = default;
     Pinned(const Pinned&) = delete;
     Pinned& operator=(const Pinned&) = delete;
     ~Pinned() {
         if (p) cudaFreeHost(p);
+    }
+    // As get, but nullptr the first time that more than kPinnedAtOnce is asked for.
+    void* wait_and_see(size_t bytes) {
+        if (bytes > kPinnedAtOnce && !large_before) {
+            large_before = true;
+            return nullptr;
+        }
+        return get(bytes);
     }
     // At least `bytes`, or nullptr (too large, or no memory).
     void* get(size_t bytes) {
@@ -352,6 +367,7 @@ struct UploadRing {
     Pinned buf[kBuffers];
     cudaEvent_t done[kBuffers] = {};
     int turn = 0;
+    bool large_before = false;  // more than kPinnedAtOnce was asked for
     UploadRing() = default;
     UploadRing(const UploadRing&) = delete;
     UploadRing& operator=(const UploadRing&) = delete;
@@ -363,6 +379,10 @@ struct UploadRing {
             }
     }
     void* get(size_t bytes) {
+        if (bytes > kPinnedAtOnce && !large_before) {
+            large_before = true;
+            return nullptr;
+        }
         // a buffer that is free now, the last used first (a new one is pinned
         // only when the others are busy), else the next in turn once it is
         for (int k = 0; k < kBuffers; ++k) {
@@ -1448,7 +1468,7 @@ struct WorldBuffers {
             return VXP_ERR_ARG;
         }
         const size_t bytes = n * sizeof(vxp_body);
-        unsigned char* st = static_cast<unsigned char*>(rd.get(bytes + 16));
+        unsigned char* st = static_cast<unsigned char*>(rd.wait_and_see(bytes + 16));
         if (!st) {
             if (check)
                 if (int rc = take_error(stream, err)) return rc;
@@ -2303,7 +2323,7 @@ static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_
     }
     if (total == 0) return VXP_OK;
     // the staging buffer comes back in one copy, with the error word (check)
-    unsigned char* back = static_cast<unsigned char*>(rd.get(total + 16));
+    unsigned char* back = static_cast<unsigned char*>(rd.wait_and_see(total + 16));
     if (check && !back)
         if (int rc = w.take_error(stream, err)) return rc;
     if (w.export_stage.reserve(total) != cudaSuccess) {
