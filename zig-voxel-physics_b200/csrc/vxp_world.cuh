@@ -206,7 +206,8 @@ enum : uint32_t {
     C_NLIGHT,        // other pairs to probe (w.colour during the probe)
     C_NLOG,          // candidates in plog
     C_BP_HITS,       // broad phase by cells: pairs found,
-    C_BP_LARGE,      // bodies tested against all
+    C_BP_LARGE,      // bodies too large for the cells: moving,
+    C_BP_LARGE_STATIC,  // and static
     C_CONS_M,        // constraint manifolds of the step (solve part split in two kernels)
     C_CONS_NCOL,     // their colours
     C_SWEEP,         // how the cluster sweeps ran (SWEEP_*)
