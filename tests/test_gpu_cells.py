@@ -1,6 +1,6 @@
 """The pair list by cells, where its cells and rows have edges: boxes whose
-corners lie on cell faces, and worlds with large bodies, few or most, moving and
-static."""
+corners lie on cell faces, bodies that touch very many others, and worlds of
+mostly large bodies, moving and static."""
 import time
 
 import numpy as np
@@ -120,12 +120,37 @@ def test_large_bodies_among_small(vxp, n, mode, large, static):
     r.close()
 
 
-@pytest.mark.parametrize("kind,limit", [("level", 2)])
+@pytest.mark.parametrize("at", [1, 40000, 66000])
+def test_row_longer_than_its_bitmap(vxp, at):
+    """One body that 65999 others touch, none of which touch each other: its row
+    is longer than the 65536 columns put in order at a time."""
+    n = 66000
+    b = table(vxp, n)
+    s = 41
+    pos = np.stack(np.meshgrid(*[np.arange(s)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)[:n]
+    b["position"] = pos * 2.0
+    wide = at - 1
+    b["collider_id"][wide] = 2
+    b["position"][wide] = -10.0
+    b["body_type"][wide] = vxp.abi.BODY_STATIC
+    g = vxp.VoxelPhysicsSystem(max_bodies=n, max_pairs=1 << 17)
+    add_box_colliders(vxp, g)
+    g.set_bodies(b)
+    others = np.setdiff1d(np.arange(1, n + 1), [at])
+    want = np.zeros(n - 1, dtype=vxp.abi.PAIR_DTYPE)
+    want["body_a"] = np.minimum(others, at)
+    want["body_b"] = np.maximum(others, at)
+    assert g.pairs(0.1).tobytes() == want.tobytes()
+    g.close()
+
+
+@pytest.mark.parametrize("kind,limit", [("wide", 10), ("level", 2)])
 def test_time_of_lists_with_large_bodies(vxp, kind, limit):
-    """15000 cubes' own list of 0.14 million pairs against one of as many bodies:
-    a level of 14000 static chunks ten times the cubes' size with 1000 cubes
-    (0.03 million pairs, once 4.8 times as long, every chunk tested against every
-    body)."""
+    """15000 cubes' own list of 0.14 million pairs against two of as many bodies:
+    64 static ones under all the cubes (a million pairs in rows of up to 15000,
+    once 30 times as long, each pair looked for in its whole row), and a level of
+    14000 static chunks ten times the cubes' size with 1000 cubes (0.03 million
+    pairs, once 4.8 times as long, every chunk tested against every body)."""
     n, s = 15000, 25
     rng = np.random.default_rng(3)
     b = table(vxp, n)
@@ -145,7 +170,12 @@ def test_time_of_lists_with_large_bodies(vxp, kind, limit):
         return sorted(out)[4]
 
     plain = median_s()
-    if kind == "level":
+    if kind == "wide":
+        b["collider_id"][:64] = 2
+        b["position"][:64] = -100.0
+        b["rotation"][:64] = (0, 0, 0, 1)
+        b["body_type"][:64] = vxp.abi.BODY_STATIC
+    else:
         chunks = np.arange(n) % 15 != 0
         b["collider_id"][chunks] = 1
         b["body_type"][chunks] = vxp.abi.BODY_STATIC

@@ -257,14 +257,14 @@ __global__ void k_export(const DBody* body, const DBodyProp* prop, uint32_t firs
 
 // The pair list of the bodies as they are (vxp_pairs_from_bodies): the step's
 // broad phase alone, with an error word of its own (a step's may wait to be
-// read).  The counters of the last step stay, but for its own three.
+// read).  The counters of the last step stay, but for its own four.
 __global__ void __launch_bounds__(512, 1) k_pairs_grid(const __grid_constant__ WorldDev w,
                                                        const __grid_constant__ ColliderSet cs, GridBar* bar,
                                                        uint32_t* err, unsigned long long timeout_ns) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     GridGroup g{bar, err, timeout_ns, gridDim.x};
     if (g.rank() == 0)
-        w.ctr[C_BP_HITS] = w.ctr[C_BP_LARGE] = w.ctr[C_BP_LARGE_STATIC] = 0u;
+        w.ctr[C_BP_HITS] = w.ctr[C_BP_LARGE] = w.ctr[C_BP_LARGE_STATIC] = w.ctr[C_BP_LONG] = 0u;
     bool overflow = false;  // the host compares the pair count with the buffers
     phase_broadphase(g, w, cs, &overflow, smem_raw);
 }

@@ -586,7 +586,10 @@ __device__ bool phase_begin(G& g, const WorldDev& w, bool skip_test, bool* skipp
 // 14000 static chunks and 1000 moving boxes 2.1 ms with every one against all,
 // so 0.15, by rows 1.6; a step of 3600 and 400 on one CTA 39.7 / 2.0 / 11.4).
 // The hits are then put in (row, column) order: counted by row, scanned,
-// dealt to the rows' places, and placed by their rank among their row's.
+// dealt to the rows' places, and placed by their rank among their row's; a
+// long row's through a bitmap (the rank reads the row once a hit: list of 15000
+// boxes with one body under all of them 1.20 ms by ranks, 0.53 so, with 64 such
+// 13.6 and 2.3; by rows 1.45 and 2.9).
 __device__ __forceinline__ int32_t bp_cell_of(float x, float inv) {
     return (int32_t)fminf(fmaxf(floorf(x * inv), -1048576.0f), 1048576.0f);
 }
@@ -599,14 +602,45 @@ __device__ __forceinline__ bool bp_overlap(float4 a0, float4 a1, float4 b0, floa
     return !(a0.w != 0.f && b0.w != 0.f) && a0.x <= b1.x && a1.x >= b0.x && a0.y <= b1.y && a1.y >= b0.y &&
            a0.z <= b1.z && a1.z >= b0.z;
 }
+// A row of more hits than this is put in order by a CTA (bp_long_row).
+constexpr uint32_t kBpLongRow = 256;
+// The pairs of row r from its columns in any order: the columns' bits are set in
+// shared memory, as many at a time as `bits` holds, and read back in order.
+__device__ __noinline__ void bp_long_row(const WorldDev& w, uint32_t r, const uint32_t* cols, uint32_t* bits,
+                                         uint32_t words) {
+    const uint32_t N = w.n_bodies, n = w.pcount[r], id = w.ids[r].x;
+    uint32_t at = w.poff[r];
+    cols += at;
+    for (uint32_t c0 = r & ~31u; c0 < N; c0 += 32u * words) {
+        const uint32_t nw = min(words, (N - c0 + 31u) / 32u);
+        __syncthreads();
+        for (uint32_t x = threadIdx.x; x < nw; x += blockDim.x) bits[x] = 0u;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const uint32_t c = cols[i] - c0;  // (a column before this piece wraps past its end)
+            if (c < 32u * nw) atomicOr(&bits[c >> 5], 1u << (c & 31u));
+        }
+        __syncthreads();
+        for (uint32_t x0 = 0; x0 < nw; x0 += blockDim.x) {
+            const uint32_t x = x0 + threadIdx.x;
+            uint32_t m = x < nw ? bits[x] : 0u, tile;
+            uint32_t q = at + block_excl_scan((uint32_t)__popc(m), &tile);
+            for (; m; m &= m - 1u) w.pairs[q++] = make_uint2(id, w.ids[c0 + 32u * x + (uint32_t)(__ffs(m) - 1)].x);
+            at += tile;
+        }
+    }
+    __syncthreads();
+}
+
 template <class G>
-__device__ bool broadphase_cells(G& g, const WorldDev& w, bool* overflow) {
+__device__ bool broadphase_cells(G& g, const WorldDev& w, bool* overflow, unsigned char* smem) {
     const uint32_t N = w.n_bodies, T = w.bp_buckets;
     const float inv = 1.0f / w.cfg.bp_cell;
     uint2* hits = reinterpret_cast<uint2*>(w.adj);  // (row, column); free until the constraint table
     uint32_t* cols = w.flag;                        // the columns, row by row
     uint32_t* large = w.bmask;                      // rows that are not small: moving,
     uint32_t* large_static = w.bmask + N;           // and static
+    uint32_t* long_rows = w.bmask + 2u * N;         // rows of more than kBpLongRow hits
     for (uint32_t i = g.rank(); i < T; i += g.size()) w.bp_start[i] = 0u;
     for (uint32_t i = g.rank(); i < N; i += g.size()) {
         w.pcount[i] = 0u;
@@ -728,14 +762,23 @@ __device__ bool broadphase_cells(G& g, const WorldDev& w, bool* overflow) {
     g.n_pairs = total;
     if (g.rank() == 0) *w.n_pairs_dev = total;
     if (*overflow) return true;
+    uint32_t dyn = 0;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+    const uint32_t words = smem ? min(2048u, dyn / 4u) : 0u, longest = words ? kBpLongRow : 0xFFFFFFFFu;
+    for (uint32_t i = g.rank(); i < N; i += g.size())
+        if (w.pcount[i] > longest) long_rows[atomicAdd(&w.ctr[C_BP_LONG], 1u)] = i;
     for (uint32_t i = g.rank(); i < total; i += g.size()) {
         const uint2 h = hits[i];
         cols[w.poff[h.x] + atomicAdd(&w.adj_cur[h.x], 1u)] = h.y;
     }
     if (!g.sync()) return false;
+    const uint32_t n_long = *(volatile uint32_t*)&w.ctr[C_BP_LONG];
+    for (uint32_t i = g.block(); i < n_long; i += g.nblocks())
+        bp_long_row(w, long_rows[i], cols, reinterpret_cast<uint32_t*>(smem), words);
     for (uint32_t i = g.rank(); i < total; i += g.size()) {
         const uint2 h = hits[i];
         const uint32_t off = w.poff[h.x], n = w.pcount[h.x];
+        if (n > longest) continue;
         uint32_t rank = 0;
         for (uint32_t j = 0; j < n; ++j) rank += cols[off + j] < h.y ? 1u : 0u;
         w.pairs[off + rank] = make_uint2(w.ids[h.x].x, w.ids[h.y].x);
@@ -787,7 +830,7 @@ __device__ bool phase_broadphase(G& g, const WorldDev& w, const ColliderSet& cs,
         w.aabb_mn[s] = make_float4(lo.x, lo.y, lo.z, w.prop[i].type == 0u ? 1.f : 0.f);
         w.aabb_mx[s] = make_float4(hi.x, hi.y, hi.z, 0.f);
     }
-    if (w.bp_buckets && N >= w.cfg.bp_cell_bodies) return broadphase_cells(g, w, overflow);
+    if (w.bp_buckets && N >= w.cfg.bp_cell_bodies) return broadphase_cells(g, w, overflow, smem);
     if (!g.sync()) return false;
     const uint32_t lane = threadIdx.x & 31, wid = g.rank() >> 5, nw = g.size() >> 5;
     const bool masks = w.bpmask != nullptr && N <= w.bp_rows;

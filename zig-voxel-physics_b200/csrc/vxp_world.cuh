@@ -208,6 +208,7 @@ enum : uint32_t {
     C_BP_HITS,       // broad phase by cells: pairs found,
     C_BP_LARGE,      // bodies too large for the cells: moving,
     C_BP_LARGE_STATIC,  // and static
+    C_BP_LONG,       // rows of more than kBpLongRow pairs
     C_CONS_M,        // constraint manifolds of the step (solve part split in two kernels)
     C_CONS_NCOL,     // their colours
     C_SWEEP,         // how the cluster sweeps ran (SWEEP_*)
