@@ -122,9 +122,9 @@ def test_export_reports_a_pending_error(vxp, fields, n):
 
 
 def test_large_tables_first_and_later(vxp):
-    """Body tables of more than 1 MB (9000 bodies), which the first calls of a
-    context copy to and from pageable memory and later ones through pinned
-    memory: every byte comes back, in both directions and from an export."""
+    """Body tables of more than a pinned buffer holds (9000 bodies, over 1 MB), in
+    a context's first calls and later: every byte comes back, in both directions
+    and from an export."""
     rng = np.random.default_rng(18)
     n = 9000
     g = vxp.VoxelPhysicsSystem(max_bodies=n)
@@ -145,4 +145,98 @@ def test_large_tables_first_and_later(vxp):
             out = g.export_state()
             for f in ("position", "rotation", "linear_velocity"):
                 assert out[f].tobytes() == np.ascontiguousarray(b[f]).tobytes(), f"turn {turn}: {f}"
+    g.close()
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 4096, 4097, 6145])
+def test_tables_at_the_edges_of_upload_buffers(vxp, n):
+    """Tables of about one, two and three buffers of 2048 bodies, ids in another
+    order than the table's, cubes resting on static ones on both sides of each
+    edge: the table comes back, and the pair list and the steps (which read the
+    id order and the list of static bodies) are the oracle's."""
+    rng = np.random.default_rng(n)
+    b = np.zeros(n, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = rng.permutation(n) + 1
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["inv_mass"] = 1.0
+    b["inv_inertia_local"][:, [0, 4, 8]] = 1.0
+    b["friction"] = 0.5
+    b["rotation"][:, 3] = 1.0
+    b["position"] = np.stack(np.meshgrid(*[np.arange(19)] * 3, indexing="ij"), axis=-1).reshape(-1, 3)[:n] * 3.0
+    edges = sorted({i for e in range(0, n + 1, 2048) for i in (e - 1, e) if 0 <= i < n} | {n - 1})
+    for i in edges:
+        b["body_type"][i] = vxp.abi.BODY_STATIC
+        b["inv_mass"][i] = 0.0
+        on = (i + n // 2) % n
+        if on in edges:
+            on = (on + 7) % n
+        b["position"][on] = b["position"][i] + np.array([0.1, 0.78, 0.05], dtype=np.float32)
+    g = vxp.VoxelPhysicsSystem(substeps=4, max_bodies=n)
+    r = O.OracleWorld(substeps=4)
+    for w in (g, r):
+        w.add_collider(0, 0.1, vxp.scenes.readme_box(8))
+    dt = np.float32(1 / 60)
+    for turn in range(2):
+        for w in (g, r):
+            w.set_bodies(b)
+        assert g.get_bodies().tobytes() == b.tobytes()
+        for s in range(2):
+            pairs = r.pairs()
+            assert g.pairs().tobytes() == pairs.tobytes()
+            g.step(dt)
+            r.step(dt, pairs)
+            assert len(r.manifolds()) >= len(edges) // 2
+            assert g.manifolds().tobytes() == r.manifolds().tobytes()
+            assert g.get_bodies().tobytes() == r.get_bodies().tobytes()
+        b = b[::-1].copy()
+    g.close()
+    r.close()
+
+
+@pytest.mark.parametrize("n", [6800, 6825, 13600, 13625, 27500])
+def test_exports_of_several_pinned_buffers(vxp, n):
+    """Exports of about one, two and four buffers of 512 KB, every field and some, whole
+    and of a range: the values set."""
+    rng = np.random.default_rng(n)
+    b = np.zeros(n, dtype=vxp.abi.BODY_DTYPE)
+    b["id"] = np.arange(1, n + 1)
+    b["body_type"] = vxp.abi.BODY_DYNAMIC
+    b["position"] = rng.uniform(-500, 500, size=(n, 3))
+    b["rotation"] = vxp.scenes.shoemake_quat(rng, n)
+    b["linear_velocity"] = rng.uniform(-1, 1, size=(n, 3))
+    b["angular_velocity"] = rng.uniform(-1, 1, size=(n, 3))
+    b["is_sleeping"] = rng.integers(0, 2, size=n)
+    g = vxp.VoxelPhysicsSystem(max_bodies=n)
+    g.set_bodies(b)  # no collider: a body's box is its position
+    for fields in (None, ["rotation", "sleeping"], ["position", "aabb_max", "angular_velocity"]):
+        for first, k in ((0, n), (1, n - 2)):
+            out = g.export_state(fields, first=first, n=k)
+            for f, v in out.items():
+                want = b[{"aabb_min": "position", "aabb_max": "position", "sleeping": "is_sleeping"}.get(f, f)]
+                assert (np.asarray(v).reshape(k, -1) == want[first : first + k].reshape(k, -1)).all(), (fields, first, f)
+    g.close()
+
+
+@pytest.mark.parametrize("cap", [0, 1, 1023, 1024, 2046, 2047, 2197, 4000])
+def test_collider_read_of_several_pinned_buffers(vxp, cap):
+    """2197 bricks, more than the 1023 that one buffer holds, read with room for
+    none, one, one and two buffers' and all of them."""
+    rng = np.random.default_rng(5)
+    bricks = vxp.scenes.readme_box(104)
+    assert len(bricks) == 2197
+    bricks["voxels"][:, rng.integers(0, 512, size=200)] = 0
+    g = vxp.VoxelPhysicsSystem()
+    g.add_collider(3, 0.1, bricks)
+    whole_info, whole = g.read_collider(3)
+    order = np.lexsort(whole["pos"].T)
+    assert whole[order].tobytes() == bricks[np.lexsort(bricks["pos"].T)].tobytes()
+    info = np.zeros(1, dtype=vxp.abi.COLLIDER_INFO_DTYPE)
+    out = np.zeros(max(cap, 1), dtype=vxp.abi.BRICK_DTYPE)
+    n = ctypes.c_uint32(0)
+    rc = g.lib.vxp_collider_read(g.ctx, 3, vxp.abi.ptr(info), vxp.abi.ptr(out) if cap else None, cap, ctypes.byref(n))
+    assert rc == 0 and n.value == 2197
+    assert info[0].tobytes() == whole_info.tobytes()
+    k = min(cap, 2197)
+    assert out[:k].tobytes() == whole[:k].tobytes()
+    assert not out[k:]["voxels"].any()
     g.close()

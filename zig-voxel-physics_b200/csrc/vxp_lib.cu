@@ -315,42 +315,31 @@ template <class T> struct DBuf {
 // Pinned host memory for what the library copies to and from the device: a
 // copy to pageable memory is staged by the driver piece by piece, with a wait
 // in each call.  The driver pins 2 MB at a time (1.2-2.8 ms) and small buffers
-// share a piece, so none takes more than it needs: with 1 MB at least for each,
-// a new context's first edit took 3.3 ms, now 0.7 (later ones 0.6).  Larger
-// copies than kPinnedMost go to the caller's memory directly.  So does a
-// context's first body table, and its first one read back, of more than
-// kPinnedAtOnce: pinning costs what many such copies save, and a context may
-// need only one.  First vxp_bodies_set of a new context, pinned at once /
-// pageable: 8000 bodies (1.5 MB) 2.3 / 0.40 ms, 15000 (2.8 MB) 4.5 / 1.0; first
-// vxp_bodies_get of 15000 (1.9 MB) 2.8 / 0.20.  (4000 bodies, 0.75 MB, pinned
-// 0.46, pageable copies 0.65.)
-constexpr size_t kPinnedMost = (size_t)32 << 20, kPinnedAtOnce = (size_t)1 << 20;
+// share a piece, so none takes more than it needs (with 1 MB at least for each,
+// a new context's first edit took 3.3 ms, now 0.7, later ones 0.6) and none more
+// than kPinnedMost: what is larger goes through it in pieces, or, where it is
+// one array of the caller's, to that directly.  (Pinned whole, the table of 8000
+// bodies took 2.5 ms in the call that pinned it, that of 15000 4.1, and 3.1 back;
+// through pageable memory 0.45, 0.80 and 0.39, so 0.25, 0.38 and 0.19.  A
+// context's buffers together stay within the first 2 MB.)
+constexpr size_t kPinnedMost = (size_t)512 << 10;
 struct Pinned {
     void* p = nullptr;
     size_t n = 0;
-    bool large_before = false;  // more than kPinnedAtOnce was asked of wait_and_see
     Pinned() = default;
     Pinned(const Pinned&) = delete;
     Pinned& operator=(const Pinned&) = delete;
     ~Pinned() {
         if (p) cudaFreeHost(p);
     }
-    // As get, but nullptr the first time that more than kPinnedAtOnce is asked for.
-    void* wait_and_see(size_t bytes) {
-        if (bytes > kPinnedAtOnce && !large_before) {
-            large_before = true;
-            return nullptr;
-        }
-        return get(bytes);
-    }
-    // At least `bytes`, or nullptr (too large, or no memory).
-    void* get(size_t bytes) {
-        if (bytes > kPinnedMost) return nullptr;
+    // At least `bytes`, or nullptr (more than `most`, or no memory).
+    void* get(size_t bytes, size_t most = kPinnedMost) {
+        if (bytes > most) return nullptr;
         if (bytes > n) {
             if (p) cudaFreeHost(p);
             p = nullptr;
             n = 0;
-            const size_t want = std::min(kPinnedMost, std::max<size_t>(bytes + bytes / 2, (size_t)1 << 15));
+            const size_t want = std::min(most, std::max<size_t>(bytes + bytes / 2, (size_t)1 << 15));
             if (cudaMallocHost(&p, want) != cudaSuccess) {
                 cudaGetLastError();
                 p = nullptr;
@@ -365,10 +354,10 @@ struct Pinned {
 // be queued while the next is filled; a buffer's event says when it is free.
 struct UploadRing {
     static constexpr int kBuffers = 4;
+    static constexpr size_t kMost = (size_t)416 << 10;  // of one buffer
     Pinned buf[kBuffers];
     cudaEvent_t done[kBuffers] = {};
     int turn = 0;
-    bool large_before = false;  // more than kPinnedAtOnce was asked for
     UploadRing() = default;
     UploadRing(const UploadRing&) = delete;
     UploadRing& operator=(const UploadRing&) = delete;
@@ -380,19 +369,18 @@ struct UploadRing {
             }
     }
     void* get(size_t bytes) {
-        if (bytes > kPinnedAtOnce && !large_before) {
-            large_before = true;
-            return nullptr;
-        }
         // a buffer that is free now, the last used first (a new one is pinned
-        // only when the others are busy), else the next in turn once it is
-        for (int k = 0; k < kBuffers; ++k) {
-            const int b = (turn + k) % kBuffers;
+        // only when the others are busy, and of large ones two at most), else
+        // the next in turn once it is
+        const int use = bytes > kMost / 4 ? 2 : kBuffers;
+        turn %= use;
+        for (int k = 0; k < use; ++k) {
+            const int b = (turn + k) % use;
             if (!done[b] || cudaEventQuery(done[b]) == cudaSuccess) {
                 turn = b;
                 break;
             }
-            if (k + 1 == kBuffers) turn = (turn + 1) % kBuffers;
+            if (k + 1 == use) turn = (turn + 1) % use;
         }
         cudaGetLastError();  // (a busy buffer's query)
         if (!done[turn] && cudaEventCreateWithFlags(&done[turn], cudaEventDisableTiming) != cudaSuccess) {
@@ -401,7 +389,7 @@ struct UploadRing {
             return nullptr;
         }
         if (cudaEventSynchronize(done[turn]) != cudaSuccess) return nullptr;
-        return buf[turn].get(bytes);
+        return buf[turn].get(bytes, kMost);
     }
     bool queued(cudaStream_t s) { return cudaEventRecord(done[turn], s) == cudaSuccess; }
 };
@@ -696,22 +684,30 @@ struct ColliderStore {
         const Entry& e = colliders[ci];
         // the record and the bricks asked for, behind the work already queued
         const uint32_t n = e.d.n_bricks, k = bricks ? std::min(cap, n) : 0u;
+        const uint32_t piece = std::min(k, (uint32_t)((kPinnedMost - sizeof(DCollider)) / 512));
         DCollider d;
         std::vector<uint8_t> far;
-        uint8_t* v = static_cast<uint8_t*>(rd.get(sizeof(d) + (size_t)k * 512));
+        uint8_t* v = static_cast<uint8_t*>(rd.get(sizeof(d) + (size_t)piece * 512));
         if (!v) {
-            far.resize(sizeof(d) + (size_t)k * 512);
+            far.resize(sizeof(d) + (size_t)piece * 512);
             v = far.data();
         }
-        if (cudaMemcpyAsync(v, d_col.p + ci, sizeof(d), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            (k && cudaMemcpyAsync(v + sizeof(d), d_vox.p + (size_t)e.d.brick_off * 512, (size_t)k * 512,
-                                  cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
-            cudaStreamSynchronize(s) != cudaSuccess) {
-            err = "collider read: copy failed";
-            return VXP_ERR_CUDA;
+        for (uint32_t b0 = 0; b0 == 0 || b0 < k; b0 += piece) {
+            const uint32_t m = std::min(piece, k - b0);
+            if ((b0 == 0 && cudaMemcpyAsync(v, d_col.p + ci, sizeof(d), cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
+                (m && cudaMemcpyAsync(v + sizeof(d), d_vox.p + ((size_t)e.d.brick_off + b0) * 512, (size_t)m * 512,
+                                      cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
+                cudaStreamSynchronize(s) != cudaSuccess) {
+                err = "collider read: copy failed";
+                return VXP_ERR_CUDA;
+            }
+            for (uint32_t b = 0; b < m; ++b) {
+                for (int q = 0; q < 3; ++q) bricks[b0 + b].pos[q] = e.pos[((size_t)b0 + b) * 3 + q];
+                std::memcpy(bricks[b0 + b].voxels, v + sizeof(d) + (size_t)b * 512, 512);
+            }
+            if (m == 0) break;
         }
         std::memcpy(&d, v, sizeof(d));
-        v += sizeof(d);
         if (info) {
             std::memset(info, 0, sizeof(*info));
             info->voxel_size = d.vs;
@@ -726,12 +722,6 @@ struct ColliderStore {
             info->has_table = d.nb_off != kNoTable ? 1u : 0u;
         }
         if (n_out) *n_out = n;
-        if (k) {
-            for (uint32_t b = 0; b < k; ++b) {
-                for (int q = 0; q < 3; ++q) bricks[b].pos[q] = e.pos[(size_t)b * 3 + q];
-                std::memcpy(bricks[b].voxels, v + (size_t)b * 512, 512);
-            }
-        }
         return VXP_OK;
     }
 
@@ -1395,64 +1385,74 @@ struct WorldBuffers {
             err = "body buffers: device allocation failed";
             return VXP_ERR_OOM;
         }
-        // bodies | properties | (id, index) | collider ids | statics | island state
-        const size_t o_prop = n * sizeof(DBody), o_id = o_prop + n * sizeof(DBodyProp), o_cid = o_id + n * sizeof(uint2),
-                     o_stat = o_cid + n * sizeof(uint32_t), o_isl = o_stat + statics * sizeof(uint32_t),
-                     total = o_isl + IS_N * sizeof(uint32_t);
-        std::vector<DBody> far;  // (aligned as the records are)
-        unsigned char* st = static_cast<unsigned char*>(up.get(total));
-        const bool pinned = st != nullptr;
-        if (!pinned) {
-            far.resize(total / sizeof(DBody) + 1);
-            st = reinterpret_cast<unsigned char*>(far.data());
-        }
-        DBody* db = reinterpret_cast<DBody*>(st);
-        DBodyProp* dp = reinterpret_cast<DBodyProp*>(st + o_prop);
-        uint2* id = reinterpret_cast<uint2*>(st + o_id);
-        uint32_t* cid = reinterpret_cast<uint32_t*>(st + o_cid);
-        uint32_t* stl = reinterpret_cast<uint32_t*>(st + o_stat);
-        uint32_t* isl = reinterpret_cast<uint32_t*>(st + o_isl);
-        static_assert(sizeof(DBody) % 16 == 0 && sizeof(DBodyProp) % 8 == 0, "records follow one another");
         collider_public.resize(n);
         moving_collider.clear();
         measured = 0;
+        // 2048 bodies a buffer: bodies | properties | (id, index) | collider ids |
+        // their statics | island state (in the last)
+        constexpr uint32_t kPer = 2048;
+        constexpr size_t kBody = sizeof(DBody) + sizeof(DBodyProp) + sizeof(uint2) + 2 * sizeof(uint32_t);
+        static_assert(kPer * kBody + IS_N * sizeof(uint32_t) <= UploadRing::kMost, "a buffer holds them");
+        static_assert(sizeof(DBody) % 16 == 0 && sizeof(DBodyProp) % 8 == 0, "records follow one another");
+        std::vector<DBody> far;  // without pinned memory (aligned as the records are)
         uint32_t ns = 0;
-        for (uint32_t i = 0; i < n; ++i) {
-            const vxp_body& s = b[i];
-            DBody& d = db[i];
-            d.p = make_float4(s.position[0], s.position[1], s.position[2], s.inv_mass);
-            d.q = make_float4(s.rotation[0], s.rotation[1], s.rotation[2], s.rotation[3]);
-            d.v = make_float4(s.linear_velocity[0], s.linear_velocity[1], s.linear_velocity[2], 0.f);
-            d.w = make_float4(s.angular_velocity[0], s.angular_velocity[1], s.angular_velocity[2], 0.f);
-            d.i0 = d.i1 = d.i2 = make_float4(0.f, 0.f, 0.f, 0.f);
-            DBodyProp& p = dp[i];
-            for (int k = 0; k < 9; ++k) p.il[k] = s.inv_inertia_local[k];
-            p.friction = s.friction;
-            p.restitution = s.restitution;
-            p.lin_damp = s.linear_damping;
-            p.ang_damp = s.angular_damping;
-            p.sleep_timer = s.sleep_timer;
-            p.id = s.id;
-            p.type = s.body_type;
-            p.collider = cols.index_of(s.collider_id);
-            if (s.body_type != 0u) moving_collider.push_back(p.collider);
-            else stl[ns++] = i;  // never moved by a step; ascending
-            p.sleeping = s.is_sleeping ? 1u : 0u;
-            collider_public[i] = cid[i] = s.collider_id;
-            id[i] = order.by_id.empty() ? make_uint2(s.id, i) : order.by_id[i];
-        }
-        // the next solve rebuilds its islands: their roots are body indices
-        // (IslandManager.markDirty, islands.zig:301-303)
-        for (uint32_t k = 0; k < IS_N; ++k) isl[k] = k == IS_DIRTY ? 1u : 0u;
-        auto put = [&](void* dst, size_t off, size_t bytes) {
-            return bytes == 0 || cudaMemcpyAsync(dst, st + off, bytes, cudaMemcpyHostToDevice, stream) == cudaSuccess;
-        };
-        if (!put(body.p, 0, o_prop) || !put(prop.p, o_prop, o_id - o_prop) || !put(ids.p, o_id, o_cid - o_id) ||
-            !put(pub_cid.p, o_cid, o_stat - o_cid) || !put(stat.p, o_stat, o_isl - o_stat) ||
-            !put(isl_state.p, o_isl, total - o_isl) || (pinned && !up.queued(stream)) ||
-            (!pinned && cudaStreamSynchronize(stream) != cudaSuccess)) {
-            err = "body upload failed";
-            return VXP_ERR_CUDA;
+        for (uint32_t i0 = 0; i0 == 0 || i0 < n; i0 += kPer) {
+            const uint32_t m = std::min(kPer, n - i0), ns0 = ns;
+            const size_t o_prop = m * sizeof(DBody), o_id = o_prop + m * sizeof(DBodyProp), o_cid = o_id + m * sizeof(uint2),
+                         o_stat = o_cid + m * sizeof(uint32_t), o_isl = o_stat + m * sizeof(uint32_t),
+                         total = o_isl + IS_N * sizeof(uint32_t);
+            unsigned char* st = static_cast<unsigned char*>(up.get(total));
+            const bool pinned = st != nullptr;
+            if (!pinned) {
+                far.resize(total / sizeof(DBody) + 1);
+                st = reinterpret_cast<unsigned char*>(far.data());
+            }
+            DBody* db = reinterpret_cast<DBody*>(st);
+            DBodyProp* dp = reinterpret_cast<DBodyProp*>(st + o_prop);
+            uint2* id = reinterpret_cast<uint2*>(st + o_id);
+            uint32_t* cid = reinterpret_cast<uint32_t*>(st + o_cid);
+            uint32_t* stl = reinterpret_cast<uint32_t*>(st + o_stat);
+            uint32_t* isl = reinterpret_cast<uint32_t*>(st + o_isl);
+            for (uint32_t j = 0; j < m; ++j) {
+                const uint32_t i = i0 + j;
+                const vxp_body& s = b[i];
+                DBody& d = db[j];
+                d.p = make_float4(s.position[0], s.position[1], s.position[2], s.inv_mass);
+                d.q = make_float4(s.rotation[0], s.rotation[1], s.rotation[2], s.rotation[3]);
+                d.v = make_float4(s.linear_velocity[0], s.linear_velocity[1], s.linear_velocity[2], 0.f);
+                d.w = make_float4(s.angular_velocity[0], s.angular_velocity[1], s.angular_velocity[2], 0.f);
+                d.i0 = d.i1 = d.i2 = make_float4(0.f, 0.f, 0.f, 0.f);
+                DBodyProp& p = dp[j];
+                for (int k = 0; k < 9; ++k) p.il[k] = s.inv_inertia_local[k];
+                p.friction = s.friction;
+                p.restitution = s.restitution;
+                p.lin_damp = s.linear_damping;
+                p.ang_damp = s.angular_damping;
+                p.sleep_timer = s.sleep_timer;
+                p.id = s.id;
+                p.type = s.body_type;
+                p.collider = cols.index_of(s.collider_id);
+                if (s.body_type != 0u) moving_collider.push_back(p.collider);
+                else stl[ns++ - ns0] = i;  // never moved by a step; ascending
+                p.sleeping = s.is_sleeping ? 1u : 0u;
+                collider_public[i] = cid[j] = s.collider_id;
+                id[j] = order.by_id.empty() ? make_uint2(s.id, i) : order.by_id[i];
+            }
+            // the next solve rebuilds its islands: their roots are body indices
+            // (IslandManager.markDirty, islands.zig:301-303)
+            for (uint32_t k = 0; k < IS_N; ++k) isl[k] = k == IS_DIRTY ? 1u : 0u;
+            auto put = [&](void* dst, size_t off, size_t bytes) {
+                return bytes == 0 || cudaMemcpyAsync(dst, st + off, bytes, cudaMemcpyHostToDevice, stream) == cudaSuccess;
+            };
+            const bool last = n - i0 <= kPer;
+            if (!put(body.p + i0, 0, o_prop) || !put(prop.p + i0, o_prop, o_id - o_prop) ||
+                !put(ids.p + i0, o_id, o_cid - o_id) || !put(pub_cid.p + i0, o_cid, o_stat - o_cid) ||
+                !put(stat.p + ns0, o_stat, (ns - ns0) * sizeof(uint32_t)) ||
+                !put(isl_state.p, o_isl, last ? total - o_isl : 0u) || (pinned && !up.queued(stream)) ||
+                (!pinned && cudaStreamSynchronize(stream) != cudaSuccess)) {
+                err = "body upload failed";
+                return VXP_ERR_CUDA;
+            }
         }
         n_static = statics;
         n_bodies = n;
@@ -1469,7 +1469,7 @@ struct WorldBuffers {
             return VXP_ERR_ARG;
         }
         const size_t bytes = n * sizeof(vxp_body);
-        unsigned char* st = static_cast<unsigned char*>(rd.wait_and_see(bytes + 16));
+        unsigned char* st = static_cast<unsigned char*>(rd.get(bytes + 16));
         if (!st) {
             if (check)
                 if (int rc = take_error(stream, err)) return rc;
@@ -2323,8 +2323,10 @@ static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_
         if (ptr[f]) total += (per[f] * n + 15u) & ~(size_t)15u;
     }
     if (total == 0) return VXP_OK;
-    // the staging buffer comes back in one copy, with the error word (check)
-    unsigned char* back = static_cast<unsigned char*>(rd.wait_and_see(total + 16));
+    // the staging buffer comes back in one copy or a few, with the error word
+    // behind the first (check)
+    const size_t piece = std::min(total, kPinnedMost - 16);  // (a multiple of 16)
+    unsigned char* back = static_cast<unsigned char*>(rd.get(piece + 16));
     if (check && !back)
         if (int rc = w.take_error(stream, err)) return rc;
     if (w.export_stage.reserve(total) != cudaSuccess) {
@@ -2346,17 +2348,23 @@ static int export_world(WorldBuffers& w, const ColliderSet& cs, const vxp_state_
         return VXP_ERR_CUDA;
     }
     if (back) {
-        uint32_t* e = reinterpret_cast<uint32_t*>(back + total);
+        uint32_t* e = reinterpret_cast<uint32_t*>(back + piece);
         *e = 0u;
-        if (cudaMemcpyAsync(back, st, total, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
-            (check && cudaMemcpyAsync(e, w.ctr.p + C_ERROR, sizeof(*e), cudaMemcpyDeviceToHost, stream) != cudaSuccess) ||
-            cudaStreamSynchronize(stream) != cudaSuccess) {
-            err = "export: copy to host failed";
-            return VXP_ERR_CUDA;
+        for (size_t at = 0; at < total; at += piece) {
+            const size_t end = std::min(total, at + piece);
+            if (cudaMemcpyAsync(back, st + at, end - at, cudaMemcpyDeviceToHost, stream) != cudaSuccess ||
+                (check && at == 0 &&
+                 cudaMemcpyAsync(e, w.ctr.p + C_ERROR, sizeof(*e), cudaMemcpyDeviceToHost, stream) != cudaSuccess) ||
+                cudaStreamSynchronize(stream) != cudaSuccess) {
+                err = "export: copy to host failed";
+                return VXP_ERR_CUDA;
+            }
+            if (*e) return w.take_error(stream, err);
+            for (int f = 0; f < 7; ++f) {
+                const size_t lo = std::max(at, off[f]), hi = std::min(end, off[f] + per[f] * n);
+                if (ptr[f] && lo < hi) std::memcpy((unsigned char*)ptr[f] + (lo - off[f]), back + (lo - at), hi - lo);
+            }
         }
-        if (*e) return w.take_error(stream, err);
-        for (int f = 0; f < 7; ++f)
-            if (ptr[f]) std::memcpy(ptr[f], back + off[f], per[f] * n);
         return VXP_OK;
     }
     for (int f = 0; f < 7; ++f) {
