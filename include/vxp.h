@@ -387,7 +387,7 @@ int vxp_last_kernel_ms(vxp_ctx* ctx, float out[2]);
 int vxp_synchronize(vxp_ctx* ctx);
 
 /* -1: choose per step (default: one CTA for a handful of small bodies, one
- * thread-block cluster for up to 160 bodies whose colliders' bounds hold up to
+ * thread-block cluster for up to 256 bodies whose colliders' bounds hold up to
  * a million voxels, else a grid); 0: one CTA steps the world; 1: the world is
  * stepped by a cooperative grid over every SM.  Same results. */
 int vxp_set_launch_mode(vxp_ctx* ctx, int mode);

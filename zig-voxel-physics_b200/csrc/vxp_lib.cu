@@ -1769,15 +1769,20 @@ constexpr unsigned long long kGridWaitNs = 10ull * 1000ull * 1000ull * 1000ull;
 //   27 boxes 438 / 325 / 366    125 boxes 1218 / 520 / 515   216 cubes 1148 / 503 / 507
 //   343 boxes 2222 / 676 / 616  8 of 40^3 voxels (0.5 M) 1039 / 446 / 499
 //   27 of 64^3 voxels (7 M) 9255 / 1514 / 985
+// Between 160 and 512 bodies what they do decides: whole calls, 200 cubes
+// apart - / 128 / 188, in contact - / 634 / 633, 250: 129 / 190 and 720 / 712,
+// 300: 142 / 191 and 785 / 710.  A solve alone (no probing) is the cluster's up
+// to where it was measured: 511 cubes apart 116 / 152, in contact 597 / 595.
 enum class StepLaunch { kBlock, kCluster, kGrid };
 constexpr uint32_t kBlockBodies = 17, kBlockVoxels = 12 * 1024;
-constexpr uint32_t kClusterBodies = 160, kClusterVoxels = 1024 * 1024;
-StepLaunch step_launch(vxp_ctx* ctx) {
+constexpr uint32_t kClusterBodies = 256, kClusterVoxels = 1024 * 1024, kClusterSolveBodies = 511;
+StepLaunch step_launch(vxp_ctx* ctx, uint32_t phases) {
     ctx->w.measure(ctx->cols);
     if (ctx->use_grid >= 0) return ctx->use_grid ? StepLaunch::kGrid : StepLaunch::kBlock;
     const uint32_t n = ctx->w.n_bodies;
     if (n <= kBlockBodies && ctx->w.voxels <= kBlockVoxels) return StepLaunch::kBlock;
     const bool cluster = ctx->solver_flow == VXP_SOLVER_CLUSTER && ctx->cluster_size > 0 && ctx->step_cluster_smem > 0;
+    if (phases == PH_SOLVE && cluster && n <= kClusterSolveBodies) return StepLaunch::kCluster;
     if (n > kClusterBodies || ctx->w.voxels > kClusterVoxels) return StepLaunch::kGrid;
     return cluster ? StepLaunch::kCluster : n <= 64 ? StepLaunch::kBlock : StepLaunch::kGrid;
 }
@@ -1785,7 +1790,7 @@ StepLaunch step_launch(vxp_ctx* ctx) {
 // Runs the step kernel.  device_pairs: the kernel builds the pair list itself.
 int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, float margin) {
     if (int rc = ctx->cols.sync(ctx->stream, ctx->err)) return rc;
-    const StepLaunch how = step_launch(ctx);
+    const StepLaunch how = step_launch(ctx, phases);
     // large colliders: room for the parts their pairs may be cut into, a part
     // per 512 voxels of bounds, and for those parts' candidates
     if (ctx->w.voxels > kClusterVoxels)
