@@ -1889,7 +1889,9 @@ int compute_device_pairs(vxp_ctx* ctx, float margin, uint32_t* n_out) {
         uint32_t* ep = reinterpret_cast<uint32_t*>(ctx->bar.p + 3);
         void* args[] = {(void*)&wd, (void*)&cs, (void*)&bp, (void*)&ep, (void*)&timeout};
         CK(cudaMemsetAsync(ctx->bar.p, 0, 4 * sizeof(GridBar), ctx->stream));
-        CK(cudaLaunchCooperativeKernel((const void*)k_pairs_grid, dim3(ctx->grid_blocks), dim3(kGridThreads), args,
+        // a warp for two rows: the barriers of a few blocks cost less than the whole grid's
+        const uint32_t blocks = std::min(ctx->grid_blocks, (n + 31u) / 32u);
+        CK(cudaLaunchCooperativeKernel((const void*)k_pairs_grid, dim3(blocks), dim3(kGridThreads), args,
                                        grid_smem(wd.cache_cap), ctx->stream));
         CK(cudaMemcpyAsync(ctx->h_count + 2, w.n_pairs_dev.p, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaMemcpyAsync(ctx->h_count + 1, ep, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
