@@ -1772,25 +1772,29 @@ constexpr unsigned long long kGridWaitNs = 10ull * 1000ull * 1000ull * 1000ull;
 // Between 160 and 512 bodies what they do decides: whole calls, 200 cubes
 // apart - / 128 / 188, in contact - / 634 / 633, 250: 129 / 190 and 720 / 712,
 // 300: 142 / 191 and 785 / 710.  A solve alone (no probing) is the cluster's up
-// to where it was measured: 511 cubes apart 116 / 152, in contact 597 / 595.
+// to where it was measured, 511 cubes apart 116 / 152, in contact 597 / 595, and so
+// is a step or a narrow phase on a caller's list of few pairs: 400 cubes, ten of
+// them in contact, 210 / 256 and 83 / 120.
 enum class StepLaunch { kBlock, kCluster, kGrid };
 constexpr uint32_t kBlockBodies = 17, kBlockVoxels = 12 * 1024;
-constexpr uint32_t kClusterBodies = 256, kClusterVoxels = 1024 * 1024, kClusterSolveBodies = 511;
-StepLaunch step_launch(vxp_ctx* ctx, uint32_t phases) {
+constexpr uint32_t kClusterBodies = 256, kClusterVoxels = 1024 * 1024, kClusterLightBodies = 511;
+constexpr uint32_t kFewPairs = 256;
+StepLaunch step_launch(vxp_ctx* ctx, uint32_t phases, bool device_pairs) {
     ctx->w.measure(ctx->cols);
     if (ctx->use_grid >= 0) return ctx->use_grid ? StepLaunch::kGrid : StepLaunch::kBlock;
     const uint32_t n = ctx->w.n_bodies;
     if (n <= kBlockBodies && ctx->w.voxels <= kBlockVoxels) return StepLaunch::kBlock;
     const bool cluster = ctx->solver_flow == VXP_SOLVER_CLUSTER && ctx->cluster_size > 0 && ctx->step_cluster_smem > 0;
-    if (phases == PH_SOLVE && cluster && n <= kClusterSolveBodies) return StepLaunch::kCluster;
-    if (n > kClusterBodies || ctx->w.voxels > kClusterVoxels) return StepLaunch::kGrid;
+    if (phases == PH_SOLVE && cluster && n <= kClusterLightBodies) return StepLaunch::kCluster;
+    const bool few = cluster && !device_pairs && ctx->last_pairs <= kFewPairs;
+    if (n > (few ? kClusterLightBodies : kClusterBodies) || ctx->w.voxels > kClusterVoxels) return StepLaunch::kGrid;
     return cluster ? StepLaunch::kCluster : n <= 64 ? StepLaunch::kBlock : StepLaunch::kGrid;
 }
 
 // Runs the step kernel.  device_pairs: the kernel builds the pair list itself.
 int launch_step(vxp_ctx* ctx, float dt, uint32_t phases, bool device_pairs, float margin) {
     if (int rc = ctx->cols.sync(ctx->stream, ctx->err)) return rc;
-    const StepLaunch how = step_launch(ctx, phases);
+    const StepLaunch how = step_launch(ctx, phases, device_pairs);
     // large colliders: room for the parts their pairs may be cut into, a part
     // per 512 voxels of bounds, and for those parts' candidates
     if (ctx->w.voxels > kClusterVoxels)
