@@ -724,21 +724,24 @@ def test_time_of_worlds_without_contacts(vxp):
         g.set_bodies(b)
         return g
 
-    def median_s(g, what):
-        out = []
+    def fastest_s(worlds, what):  # in turn
+        out = [[] for _ in worlds]
         for _ in range(61):
-            t0 = time.perf_counter()
-            what(g)
-            g.synchronize()
-            out.append(time.perf_counter() - t0)
-        return sorted(out)[30]
+            for g, o in zip(worlds, out):
+                t0 = time.perf_counter()
+                what(g)
+                g.synchronize()
+                o.append(time.perf_counter() - t0)
+        return [min(o) for o in out]
 
     dt = np.float32(1e-5)
     small, step, solve = world(160), world(200), world(400)
-    assert median_s(step, lambda g: g.step(dt)) < 1.25 * median_s(small, lambda g: g.step(dt))
-    solve.narrow_phase(np.zeros(0, dtype=vxp.abi.PAIR_DTYPE))
-    small.narrow_phase(np.zeros(0, dtype=vxp.abi.PAIR_DTYPE))
-    assert median_s(solve, lambda g: g.solve(dt)) < 1.2 * median_s(small, lambda g: g.solve(dt))
+    a, b = fastest_s((small, step), lambda g: g.step(dt))
+    assert b < 1.25 * a
+    for g in (small, solve):
+        g.narrow_phase(np.zeros(0, dtype=vxp.abi.PAIR_DTYPE))
+    a, b = fastest_s((small, solve), lambda g: g.solve(dt))
+    assert b < 1.2 * a
     for g in (small, step, solve):
         g.close()
 
@@ -781,22 +784,33 @@ def test_time_of_steps_on_few_pairs(vxp):
     (0.085 ms; on the grid 0.13)."""
     import time
 
-    def median_s(n):
+    none = np.zeros(0, dtype=vxp.abi.PAIR_DTYPE)
+    worlds, fastest = [], [1.0, 1.0]
+    for n in (250, 400):
         b = np.zeros(n, dtype=vxp.abi.BODY_DTYPE)
         b["id"] = np.arange(1, n + 1)
         b["body_type"] = vxp.abi.BODY_DYNAMIC
         b["inv_mass"] = 1.0
         b["rotation"][:, 3] = 1.0
-        g = vxp.VoxelPhysicsSystem(substeps=2)
-        g.set_bodies(b)
-        none = np.zeros(0, dtype=vxp.abi.PAIR_DTYPE)
-        out = []
-        for _ in range(61):
+        worlds.append(vxp.VoxelPhysicsSystem(substeps=2))
+        worlds[-1].set_bodies(b)
+    for _ in range(61):  # in turn
+        for i, g in enumerate(worlds):
             t0 = time.perf_counter()
             g.step(np.float32(1e-4), none)
             g.synchronize()
-            out.append(time.perf_counter() - t0)
+            fastest[i] = min(fastest[i], time.perf_counter() - t0)
+    assert fastest[1] < 1.25 * fastest[0]
+    for g in worlds:
         g.close()
-        return sorted(out)[30]
 
-    assert median_s(400) < 1.25 * median_s(250)
+
+@pytest.mark.parametrize("mode,boxes,smem", [(0, 3, None), (-1, 3, None), (-1, 4, 4096), (-1, 4, 0), (1, 4, None)])
+def test_without_friction(vxp, mode, boxes, smem):
+    """No friction: bodies, and manifolds with tangent masses of zero, as the
+    oracle's (after worlds with friction, whose rows are left in shared memory)."""
+    def scene():
+        return vxp.scenes.config2(mass_fn=O.mass_fn, n_side=boxes, seed=7)
+
+    lockstep(vxp, scene(), 60, mode=mode, cluster_smem=smem, substeps=4).close()
+    lockstep(vxp, scene(), 90, mode=mode, cluster_smem=smem, substeps=4, enable_friction=0).close()

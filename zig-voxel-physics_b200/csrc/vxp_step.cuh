@@ -4554,6 +4554,10 @@ __device__ bool phase_solve_cluster(G& g, const WorldDev& w, uint32_t M, uint32_
                 cpr(vs, CP_NI, i) = ni[i];
                 cpr(vs, CP_TI0, i) = t0[i];
                 cpr(vs, CP_TI1, i) = t1[i];
+                if (!cf.friction_on) {  // prepare writes no tangent masses then
+                    cpr(vs, CP_TM0, i) = 0.f;
+                    cpr(vs, CP_TM1, i) = 0.f;
+                }
             }
         }
     }
