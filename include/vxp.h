@@ -388,8 +388,13 @@ int vxp_synchronize(vxp_ctx* ctx);
 
 /* -1: choose per step (default: one CTA for a handful of small bodies, one
  * thread-block cluster for up to 256 bodies whose colliders' bounds hold up to
- * a million voxels, else a grid); 0: one CTA steps the world; 1: the world is
- * stepped by a cooperative grid over every SM.  Same results. */
+ * a million voxels, and up to 511 for a solve alone or a caller's list of at
+ * most 256 pairs, else a grid); 0: one CTA steps the world; 1: the world is
+ * stepped by a cooperative grid over every SM.  Same results.  Steps of several
+ * contexts, each from its own thread, overlap on the GPU on one CTA or cluster
+ * each, and not on grids: eight contexts of 345 bodies take 2.2 ms for a frame of
+ * all by default and 1.9 ms in mode 0 (of 218 bodies 0.7 and 1.5, of 1000 2.8 and
+ * 4.2). */
 int vxp_set_launch_mode(vxp_ctx* ctx, int mode);
 
 /* Grid launch tuning: after the narrow phase, the solver runs on
