@@ -321,8 +321,9 @@ template <class T> struct DBuf {
 // one array of the caller's, to that directly.  (Pinned whole, the table of 8000
 // bodies took 2.5 ms in the call that pinned it, that of 15000 4.1, and 3.1 back;
 // through pageable memory 0.45, 0.80 and 0.39, so 0.25, 0.38 and 0.19.  A
-// context's buffers together stay within the first 2 MB.)
-constexpr size_t kPinnedMost = (size_t)512 << 10;
+// context's buffers, one of this and two of an upload's, stay within the first
+// 2 MB.)
+constexpr size_t kPinnedMost = (size_t)1 << 20;
 struct Pinned {
     void* p = nullptr;
     size_t n = 0;
